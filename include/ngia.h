@@ -236,7 +236,9 @@ int ngia_ctx_align_pairs(ngia_ctx *ctx, const uint32_t *d_pairs, uint32_t count,
  * words per lane: (8,3) (8,4) (16,4) (16,6) (32,4) (32,6) (32,8) (32,16) -- whose
  * group_limit admits the band (ls + rs <= group_limit, or a rep of at most G
  * slices); otherwise one pair per thread.  group_limit 0 leaves a class
- * unused; a limit above (G-1)K + G is refused.  Scores never depend on the
+ * unused; a limit above (G-1)K + G is refused.  stream_max 16, the default,
+ * also lets a round hold wider windows (up to 28 words) and whole short reps
+ * one pair per lane where that takes fewer words.  Scores never depend on the
  * plan. */
 #define NGIA_GROUP_CLASSES 8
 typedef struct ngia_plan {

@@ -4,9 +4,6 @@
 #include <vector>
 
 #include "align.cuh"
-#include "align_group.cuh"
-#include "align_group_cta.cuh"
-#include "align_stream.cuh"
 #include "kernels.cuh"
 
 namespace ngia {
@@ -21,15 +18,6 @@ __device__ __forceinline__ uint32_t lcs_any(const uint32_t *rep, const uint32_t 
   if (b.width <= 8) return lcs_window<8>(rep, tar, b, blocks);
   if (b.width <= 16) return lcs_window<16>(rep, tar, b, blocks);
   return lcs_general(rep, tar, b, lines, blocks);
-}
-
-// Adds the warp's computed 32x32 blocks (row words x column blocks) to *work.
-__device__ __forceinline__ void count_work(uint32_t blocks, unsigned long long *work) {
-  // two 16-bit halves, so that a warp's sum cannot overflow
-  const uint32_t lo = __reduce_add_sync(kFull, blocks & 0xFFFFu);
-  const uint32_t hi = __reduce_add_sync(kFull, blocks >> 16);
-  const unsigned long long sum = ((unsigned long long)hi << 16) + lo;
-  if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(work, sum);
 }
 
 __global__ void __launch_bounds__(128)
@@ -68,87 +56,6 @@ align_jobs_dev_count_kernel(const uint32_t *__restrict__ packed,
     const uint32_t lcs = lcs_any(rep, tar, b, lines);
     jobs[3 * j + 2] = identity_score(lcs, lr, lt, t);
   }
-}
-
-// The batched kernels read their class's range of the queue order from
-// device memory (bounds[cls] .. bounds[cls + 1], written by the classifier),
-// so that a round needs no host round trip and can be captured as a graph.
-
-// Batched form, general kernel: one pair per thread, grid-stride over the
-// class's range.
-__global__ void __launch_bounds__(128)
-align_general_kernel(const uint32_t *__restrict__ packed,
-                     const uint64_t *__restrict__ offs, const uint2 *__restrict__ pairs,
-                     const uint32_t *__restrict__ order, const uint32_t *__restrict__ bounds,
-                     int cls, uint32_t *__restrict__ scores, float t, int fma_mode,
-                     unsigned long long *__restrict__ work) {
-  const uint32_t begin = bounds[cls], end = bounds[cls + 1];
-  uint32_t done = 0;
-  for (uint32_t k = begin + blockIdx.x * blockDim.x + threadIdx.x; k < end;
-       k += gridDim.x * blockDim.x) {
-    const uint32_t p = order[k];
-    const uint2 pr = pairs[p];
-    const uint32_t *rep = packed + offs[pr.x];
-    const uint32_t *tar = packed + offs[pr.y];
-    const uint32_t lr = __ldg(rep), lt = __ldg(tar);
-    const Band b = make_band(lr, lt, t, fma_mode);
-    uint32_t lines[kMaxRowBlocks];
-    uint32_t blocks;
-    const uint32_t lcs = lcs_general(rep, tar, b, lines, blocks);
-    done += blocks * ((b.width + 7u) & ~7u);
-    scores[p] = identity_score(lcs, lr, lt, t);
-  }
-  count_work(done, work);
-}
-
-// Batched form, group kernel (align_group.cuh): a persistent grid whose groups
-// of G lanes take pairs of one class from its queue.
-template <int G, int K, int KC>
-__global__ void __launch_bounds__(kGroupThreads)
-align_group_kernel(const uint32_t *__restrict__ packed, const uint32_t *__restrict__ nib,
-                   uint64_t inv, const uint64_t *__restrict__ offs,
-                   const uint2 *__restrict__ pairs, const uint32_t *__restrict__ order,
-                   const uint32_t *__restrict__ bounds, int cls,
-                   unsigned int *__restrict__ cursor, uint32_t *__restrict__ scores, float t,
-                   int fma_mode, unsigned long long *__restrict__ work) {
-  extern __shared__ uint32_t smem[];
-  const uint32_t done = align_group<G, K, KC>(packed, nib, inv, offs, pairs, order,
-                                              bounds[cls], bounds[cls + 1], cursor, scores, t,
-                                              fma_mode, smem);
-  count_work(done, work);
-}
-
-// The widest group classes: one block of W warps per pair
-// (align_group_cta.cuh).
-template <int W, int K, int KC>
-__global__ void __launch_bounds__(32 * W)
-align_group_cta_kernel(const uint32_t *__restrict__ packed, const uint32_t *__restrict__ nib,
-                       uint64_t inv, const uint64_t *__restrict__ offs,
-                       const uint2 *__restrict__ pairs, const uint32_t *__restrict__ order,
-                       const uint32_t *__restrict__ bounds, int cls,
-                       unsigned int *__restrict__ cursor, uint32_t *__restrict__ scores, float t,
-                       int fma_mode, unsigned long long *__restrict__ work) {
-  extern __shared__ uint32_t smem[];
-  const uint32_t done = align_group_cta<W, K, KC>(packed, nib, inv, offs, pairs, order,
-                                                  bounds[cls], bounds[cls + 1], cursor, scores,
-                                                  t, fma_mode, smem);
-  count_work(done, work);
-}
-
-// Batched form, streaming shared-memory table kernel (align_stream.cuh):
-// a persistent grid whose lanes take pairs of one class from its queue.
-template <int W, int K>
-__global__ void __launch_bounds__(kStreamThreads, NGIA_STREAM_MIN_BLOCKS)
-align_stream_kernel(const uint32_t *__restrict__ packed, const uint32_t *__restrict__ nib,
-                    uint64_t inv, const uint64_t *__restrict__ offs,
-                    const uint2 *__restrict__ pairs, const uint32_t *__restrict__ order,
-                    const uint32_t *__restrict__ bounds, int cls,
-                    unsigned int *__restrict__ cursor, uint32_t *__restrict__ scores, float t,
-                    int fma_mode, unsigned long long *__restrict__ work) {
-  extern __shared__ uint32_t smem[];
-  const uint32_t done = align_stream<W, K>(packed, nib, inv, offs, pairs, order, bounds[cls],
-                                           bounds[cls + 1], cursor, scores, t, fma_mode, smem);
-  count_work(done, work);
 }
 
 // Load-time layout kernels: one warp per record, lane k taking the record's
@@ -425,8 +332,6 @@ int launch_dense_layouts(const uint32_t *packed, const uint64_t *offs, uint32_t 
   return NGIA_OK;
 }
 
-// Blocks of a persistent launch: as many as fit on the device at once, and no
-// more than `want`.  Occupancy is looked up once per (kernel, device).
 struct OccEntry {
   const void *func;
   int dev, per_sm, sms;
@@ -434,17 +339,15 @@ struct OccEntry {
 static std::mutex g_occ_mu;
 static std::vector<OccEntry> g_occ;
 
-template <typename F>
-static int persistent_grid(F func, int threads, size_t smem, uint32_t want, uint32_t *grid) {
+int persistent_grid(const void *func, int threads, size_t smem, uint32_t want, uint32_t *grid) {
   int dev = 0;
   NGIA_CUDA(cudaGetDevice(&dev));
-  const void *key = reinterpret_cast<const void *>(func);
   std::lock_guard<std::mutex> lock(g_occ_mu);
   const OccEntry *hit = nullptr;
   for (const OccEntry &e : g_occ)
-    if (e.func == key && e.dev == dev) hit = &e;
+    if (e.func == func && e.dev == dev) hit = &e;
   if (!hit) {
-    OccEntry e{key, dev, 0, 0};
+    OccEntry e{func, dev, 0, 0};
     NGIA_CUDA(cudaDeviceGetAttribute(&e.sms, cudaDevAttrMultiProcessorCount, dev));
     NGIA_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // the most shared memory per SM the L1 split allows: more resident blocks
@@ -460,105 +363,13 @@ static int persistent_grid(F func, int threads, size_t smem, uint32_t want, uint
   return NGIA_OK;
 }
 
-// Launch arguments shared by every class of one batched round.
-struct RoundArgs {
-  const uint32_t *packed, *nib;
-  uint64_t inv;
-  const uint32_t *dplanes;
-  const uint64_t *offs;
-  const uint2 *pairs;
-  const uint32_t *order, *bounds;
-  uint32_t *scores;
-  float t;
-  int fm;
-  unsigned long long *work;
-};
-
-template <int W, int K>
-static int launch_stream_k(const RoundArgs &a, int cls, unsigned int *cursor,
-                           cudaStream_t s) {
-  constexpr size_t smem = stream_smem_bytes(W, K);
-  uint32_t grid = 0;
-  NGIA_TRY(persistent_grid(align_stream_kernel<W, K>, kStreamThreads, smem, kFull, &grid));
-  // K < 16 tables fill from the code planes (records with the same offsets)
-  if (K < 16 && !a.dplanes) return NGIA_ERR_STATE;
-  align_stream_kernel<W, K><<<grid, kStreamThreads, smem, s>>>(
-      K < 16 ? a.dplanes : a.packed, a.nib, a.inv, a.offs, a.pairs, a.order, a.bounds, cls,
-      cursor, a.scores, a.t, a.fm, a.work);
-  NGIA_LAUNCHED();
-  return NGIA_OK;
-}
-
-template <int G, int K, int KC>
-static int launch_group_k(const RoundArgs &a, int cls, unsigned int *cursor, cudaStream_t s) {
-  constexpr size_t smem = group_smem_bytes(K, KC);
-  uint32_t grid = 0;
-  NGIA_TRY(persistent_grid(align_group_kernel<G, K, KC>, kGroupThreads, smem, kFull, &grid));
-  if (KC == 8 && !a.dplanes) return NGIA_ERR_STATE;
-  align_group_kernel<G, K, KC><<<grid, kGroupThreads, smem, s>>>(
-      KC == 8 ? a.dplanes : a.packed, a.nib, a.inv, a.offs, a.pairs, a.order, a.bounds, cls,
-      cursor, a.scores, a.t, a.fm, a.work);
-  NGIA_LAUNCHED();
-  return NGIA_OK;
-}
-
-template <int W, int K, int KC>
-static int launch_group_cta_k(const RoundArgs &a, int cls, unsigned int *cursor,
-                              cudaStream_t s) {
-  constexpr size_t smem = group_cta_smem_bytes<W, K, KC>();
-  uint32_t grid = 0;
-  NGIA_TRY(persistent_grid(align_group_cta_kernel<W, K, KC>, 32 * W, smem, kFull, &grid));
-  if (KC == 8 && !a.dplanes) return NGIA_ERR_STATE;
-  align_group_cta_kernel<W, K, KC><<<grid, 32 * W, smem, s>>>(
-      KC == 8 ? a.dplanes : a.packed, a.nib, a.inv, a.offs, a.pairs, a.order, a.bounds, cls,
-      cursor, a.scores, a.t, a.fm, a.work);
-  NGIA_LAUNCHED();
-  return NGIA_OK;
-}
-
-// A class of (32 lanes, K words) on one block of kCtaWarps warps per pair
-// (32 * kCtaWarps lanes, K / kCtaWarps words): the same rows per ring turn and
-// a wider span, so the class's binning holds (align_group_cta.cuh).
-// Measured on 2,000,000 heavy-tailed protein pairs (autotuned round): one warp
-// per pair 9.28 ms, blocks of two warps 9.69 ms, of four 10.46 ms -- the
-// shorter chains do not pay for the extra issue slots and barriers, so the
-// block-wide form is off by default (NGIA_CTA_WARPS=2 or 4 at build time).
-#ifndef NGIA_CTA_WARPS
-#define NGIA_CTA_WARPS 0  // 0: the classes run on one warp per pair (align_group.cuh)
-#endif
-// the first group class (index within the ladder) run block-wide when
-// NGIA_CTA_WARPS is set: 6 = the two widest, (32,8) and (32,16); 4 adds
-// (32,4) and (32,6).  On the re-laddered classes, same pairs and box: one
-// warp per pair 8.05 ms per round (autotuned), blocks of two warps from
-// (32,4) on 8.52 ms, from (32,6) on 8.65 ms.
-#ifndef NGIA_CTA_FROM
-#define NGIA_CTA_FROM 6
-#endif
-static_assert(NGIA_CTA_FROM >= 4 && NGIA_CTA_FROM <= 7, "block-wide classes are the G = 32 ones");
-constexpr int kCtaWarps = NGIA_CTA_WARPS > 0 ? NGIA_CTA_WARPS : 1;
 template <int K>
-static int launch_group_cta(const RoundArgs &a, int KC, int cls, unsigned int *cursor,
-                            cudaStream_t s) {
-  static_assert(K % kCtaWarps == 0, "slices of K / kCtaWarps words");
-  constexpr int KW = K / kCtaWarps;
-  static_assert((32 * kCtaWarps - 1) * KW + 32 * kCtaWarps >= 31 * K + 32, "span");
-  return KC <= 8 ? launch_group_cta_k<kCtaWarps, KW, 8>(a, cls, cursor, s)
-                 : launch_group_cta_k<kCtaWarps, KW, 16>(a, cls, cursor, s);
-}
+int launch_align_k(int kernel, const RoundArgs &a, uint32_t m, cudaStream_t s);
 
-template <int W>
-static int launch_stream(const RoundArgs &a, int K, int cls, unsigned int *cursor,
-                         cudaStream_t s) {
-  return K == 5   ? launch_stream_k<W, 5>(a, cls, cursor, s)
-         : K == 8 ? launch_stream_k<W, 8>(a, cls, cursor, s)
-                  : launch_stream_k<W, 16>(a, cls, cursor, s);
-}
-
-template <int G, int K>
-static int launch_group(const RoundArgs &a, int KC, int cls, unsigned int *cursor,
-                        cudaStream_t s) {
-  return KC <= 8 ? launch_group_k<G, K, 8>(a, cls, cursor, s)
-                 : launch_group_k<G, K, 16>(a, cls, cursor, s);
+int launch_align(int kernel, const RoundArgs &a, int K, uint32_t m, cudaStream_t s) {
+  return K == 5   ? launch_align_k<5>(kernel, a, m, s)
+         : K == 8 ? launch_align_k<8>(kernel, a, m, s)
+                  : launch_align_k<16>(kernel, a, m, s);
 }
 
 int launch_align_jobs(const uint32_t *packed, const uint64_t *offs, uint32_t *jobs,
@@ -580,60 +391,6 @@ int launch_align_jobs_dev_count(const uint32_t *packed, const uint64_t *offs,
       packed, offs, jobs, d_count, identity_threshold(identity), round_mode());
   NGIA_LAUNCHED();
   return NGIA_OK;
-}
-
-int launch_align_class(int cls, const uint32_t *packed, const uint32_t *nib,
-                       const Alphabet &ab, const uint64_t *offs, const uint2 *pairs,
-                       const uint32_t *order, const uint32_t *bounds, uint32_t *scores,
-                       uint32_t identity, unsigned long long *work, unsigned int *cursor,
-                       cudaStream_t s) {
-  const RoundArgs a{packed, nib, ab.inv, ab.dplanes, offs, pairs, order, bounds, scores,
-                    identity_threshold(identity), round_mode(), work};
-  switch (cls) {
-#define NGIA_STREAM_CASE(C) \
-  case C: return launch_stream<class_width(C)>(a, ab.K, cls, cursor, s);
-    NGIA_STREAM_CASE(0)
-    NGIA_STREAM_CASE(1)
-    NGIA_STREAM_CASE(2)
-    NGIA_STREAM_CASE(3)
-    NGIA_STREAM_CASE(4)
-    NGIA_STREAM_CASE(5)
-    NGIA_STREAM_CASE(6)
-    NGIA_STREAM_CASE(7)
-    NGIA_STREAM_CASE(8)
-    NGIA_STREAM_CASE(9)
-    NGIA_STREAM_CASE(10)
-#undef NGIA_STREAM_CASE
-#define NGIA_GROUP_CASE(C) \
-  case C: return launch_group<group_shape(C).G, group_shape(C).K>(a, ab.K, cls, cursor, s);
-    NGIA_GROUP_CASE(kFirstGroupClass)
-    NGIA_GROUP_CASE(kFirstGroupClass + 1)
-    NGIA_GROUP_CASE(kFirstGroupClass + 2)
-    NGIA_GROUP_CASE(kFirstGroupClass + 3)
-#undef NGIA_GROUP_CASE
-    // the G = 32 classes, block-wide from NGIA_CTA_FROM on when NGIA_CTA_WARPS is set
-#define NGIA_WIDE_CASE(I)                                                                   \
-  case kFirstGroupClass + I:                                                                \
-    static_assert(group_shape(kFirstGroupClass + I).G == 32, "a G = 32 class");             \
-    return NGIA_CTA_WARPS && I >= NGIA_CTA_FROM                                              \
-               ? launch_group_cta<group_shape(kFirstGroupClass + I).K>(a, ab.K, cls, cursor, s) \
-               : launch_group<32, group_shape(kFirstGroupClass + I).K>(a, ab.K, cls, cursor, s);
-    NGIA_WIDE_CASE(4)
-    NGIA_WIDE_CASE(5)
-    NGIA_WIDE_CASE(6)
-    NGIA_WIDE_CASE(7)
-#undef NGIA_WIDE_CASE
-    static_assert(kNumGroupClasses == 8, "the ladder's cases above");
-    case kGeneralClass: {
-      uint32_t grid = 0;
-      NGIA_TRY(persistent_grid(align_general_kernel, 128, 0, kFull, &grid));
-      align_general_kernel<<<grid, 128, 0, s>>>(packed, offs, pairs, order, bounds, cls, scores,
-                                                a.t, a.fm, work);
-      NGIA_LAUNCHED();
-      return NGIA_OK;
-    }
-    default: return NGIA_ERR_ARG;
-  }
 }
 
 }  // namespace ngia

@@ -254,11 +254,11 @@ __device__ inline uint32_t lcs_general(const uint32_t *__restrict__ rep,
   return zeros;
 }
 
-// Width classes of the batched aligner:
-//   0..10  streaming shared-memory table kernel (align_stream.cuh), one pair
-//          per lane, W = 4, 5, ..., 12, 14, 16 words by stream_width (every
-//          width up to 12: a window word above the band costs as much as a
-//          live one, and bands of equal ls + rs - 1 are common)
+// Width classes of the batched aligner.  The plan's ladder (width_class):
+//   0..10  one pair per lane in a sliding window (align_window.cuh), W = 4, 5,
+//          ..., 12, 14, 16 words by stream_width (every width up to 12: a
+//          window word above the band costs as much as a live one, and bands
+//          of equal ls + rs - 1 are common)
 //   11..18 group kernel (align_group.cuh), one pair per group of G lanes with
 //          K words per lane: (8,3) (8,4) (16,4) (16,6) (32,4) (32,6) (32,8)
 //          (32,16).  A column step costs a lane 3 ops per word plus a fixed
@@ -269,12 +269,19 @@ __device__ inline uint32_t lcs_general(const uint32_t *__restrict__ rep,
 //          proteins rather than sixteen lanes of one or two
 //   19     general kernel, one pair per thread (any width)
 //   20     pairs failing the length filter (score 0, not launched)
+// and, with a plan that sends every window of 16 words to the lanes, the
+// further one-pair-per-lane classes that round_class prefers:
+//   21..24 sliding windows of 18, 20, 24, 28 words
+//   25..31 fixed windows (the whole rep) of 8, 10, 12, 14, 16, 20, 24 words
 constexpr int kNumLdsClasses = 11;
 constexpr int kFirstGroupClass = 11;
 constexpr int kNumGroupClasses = 8;
 constexpr int kGeneralClass = kFirstGroupClass + kNumGroupClasses;
 constexpr int kSkipClass = kGeneralClass + 1;
 constexpr int kNumClasses = kSkipClass + 1;
+constexpr int kFirstWideClass = kNumClasses, kNumWideClasses = 4;
+constexpr int kFirstFixedClass = kFirstWideClass + kNumWideClasses, kNumFixedClasses = 7;
+constexpr int kNumRoundClasses = kFirstFixedClass + kNumFixedClasses;
 
 struct GroupShape {
   int G, K;
@@ -293,6 +300,19 @@ __host__ __device__ constexpr GroupShape group_shape(int c) {
 __host__ __device__ constexpr int class_width(int c) {
   return c < 9 ? 4 + c : c == 9 ? 14 : c == 10 ? 16 : 0;
 }
+
+// Window words of the further classes.
+__host__ __device__ constexpr int wide_width(int k) {
+  return k == 0 ? 18 : k == 1 ? 20 : k == 2 ? 24 : 28;
+}
+__host__ __device__ constexpr int fixed_width(int k) {
+  return k < 5 ? 8 + 2 * k : k == 5 ? 20 : 24;
+}
+
+// The widest sliding window for tables of K entries per row word: 28 words of
+// 16 entries would leave a streaming multiprocessor's shared memory to three
+// warps (align_window.cuh).
+__host__ __device__ constexpr uint32_t widest_window(int K) { return K > 8 ? 24u : 28u; }
 
 // Window a streaming kernel needs for a pair: the live rows of block i,
 // [max(i - ls, 0), min(i + rs, nr)), inside [i - ls, i - ls + W).
@@ -346,6 +366,34 @@ __host__ __device__ inline int width_class(const Band &b) {
   return width_class(b, default_plan());
 }
 
+// The class a round runs a pair in.  It is width_class's, except that with
+// stream_max 16 (every window the ladder has) a pair also has the classes
+// above: sliding windows up to `widest` words instead of a group of lanes, and
+// a fixed window where the rep is short enough for a narrower one than the
+// sliding window would be.  Fewest window words wins: the lanes run 3 ALU
+// operations per window word and column, so a pair's time is its words.
+// Align phase without and with these classes: 1,000,003 proteins at identity
+// 50 12.9 -> 9.6 ms, 25,013 nucleotide reads with N at 85 6.4 -> 3.5 ms, 2
+// million heavy-tailed protein pairs at 90 8.7 -> 7.8 ms.
+__host__ __device__ inline int round_class(const Band &b, const ClassPlan &plan,
+                                           uint32_t widest) {
+  const int c = width_class(b, plan);
+  if (c == kSkipClass || plan.stream_max < 16) return c;
+  const uint32_t ws = stream_width(b);
+  int slide = c < kNumLdsClasses ? c : -1;
+  uint32_t words = slide >= 0 ? (uint32_t)class_width(c) : kFull;
+  if (slide < 0 && ws <= widest) {
+    slide = ws <= 18 ? 0 : ws <= 20 ? 1 : ws <= 24 ? 2 : 3;
+    words = (uint32_t)wide_width(slide);
+    slide += kFirstWideClass;
+  }
+  if (b.nr <= 24) {
+    const int f = b.nr <= 8 ? 0 : b.nr <= 16 ? (int)(b.nr - 7) / 2 : b.nr <= 20 ? 5 : 6;
+    if ((uint32_t)fixed_width(f) < words) return kFirstFixedClass + f;
+  }
+  return slide >= 0 ? slide : c;
+}
+
 // Queue order inside a class: longest targets first.  The sort key of a pair
 // is class-major, then 7 - floor(log2 nc) (column blocks in octaves, capped
 // at 7), one 8-bit radix pass.
@@ -363,7 +411,7 @@ __host__ __device__ inline uint32_t class_sort_key(int cls, const Band &b) {
   return ((uint32_t)cls << 3) | (7u - (h < 7u ? h : 7u));
 }
 constexpr int kClassKeyBits = 8;
-static_assert(kNumClasses <= 32, "class sort key: 5 class bits");
+static_assert(kNumRoundClasses <= 32, "class sort key: 5 class bits");
 __host__ __device__ constexpr uint32_t skip_sort_key() { return ((uint32_t)kSkipClass << 3) | 7u; }
 
 }  // namespace ngia

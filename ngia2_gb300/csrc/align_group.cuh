@@ -148,7 +148,7 @@ __device__ __forceinline__ uint32_t group_row_bound(const uint32_t (&V)[K], uint
 // (word x column block) count.
 template <int G, int K, int KC>
 __device__ inline uint32_t align_group(const uint32_t *__restrict__ packed,
-                                       const uint32_t *__restrict__ nib, uint64_t inv,
+                                       const uint32_t *__restrict__ nib,
                                        const uint64_t *__restrict__ offs,
                                        const uint2 *__restrict__ pairs,
                                        const uint32_t *__restrict__ order, uint32_t begin,
@@ -159,7 +159,7 @@ __device__ inline uint32_t align_group(const uint32_t *__restrict__ packed,
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t sub = lane % G;
   const uint32_t src = lane - sub + (sub + G - 1) % G;  // the lane below in the ring
-  const LdsTable<K, KC> tab{smem + (threadIdx.x >> 5) * (KC * K * 32) + lane, inv};
+  const LdsTable<K, KC> tab{smem + lane};
 #pragma unroll 1
   for (uint32_t s = 0; s < (uint32_t)K; ++s) {
     tab.clear(s);

@@ -146,6 +146,17 @@ __host__ __device__ inline uint32_t identity_score(uint32_t lcs, uint32_t lr,
   return hit ? lcs * 100u / den : 0u;
 }
 
+// identity_score(...) > 0, without its division.
+__host__ __device__ inline bool score_positive(uint32_t lcs, uint32_t lr, uint32_t lt, float t) {
+  const uint32_t den = lr + lt - lcs;
+#ifdef __CUDA_ARCH__
+  const bool hit = __uint2float_rn(lcs) > __fmul_rn(__uint2float_rn(den), t);
+#else
+  const bool hit = (float)lcs > (float)den * t;
+#endif
+  return hit && lcs * 100u >= den;
+}
+
 // Early exit.  One column step raises the number of zero bits of the row
 // vector (the running LCS) by at most one, and the score test
 // lcs > (Lr + Lt - lcs) * t is monotone in lcs.  So once
@@ -158,13 +169,13 @@ __host__ __device__ inline bool stream_may_reach(uint32_t lcs_so_far, uint32_t c
   uint32_t ub = lcs_so_far + left;
   const uint32_t cap = lr < lt ? lr : lt;
   if (ub > cap) ub = cap;
-  return identity_score(ub, lr, lt, t) > 0;
+  return score_positive(ub, lr, lt, t);
 }
 
 // The same test for an upper bound of the final LCS itself.
 __host__ __device__ inline bool lcs_may_reach(uint32_t ub, uint32_t lr, uint32_t lt, float t) {
   const uint32_t cap = lr < lt ? lr : lt;
-  return identity_score(ub < cap ? ub : cap, lr, lt, t) > 0;
+  return score_positive(ub < cap ? ub : cap, lr, lt, t);
 }
 
 __host__ __device__ inline bool may_reach_threshold(uint32_t lcs_so_far, uint32_t cols_done,

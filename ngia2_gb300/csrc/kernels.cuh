@@ -66,14 +66,31 @@ struct Alphabet {
   // row block's table entries are one logic op each
   const uint32_t *dplanes = nullptr;
 };
-// One width class of the batched aligner: a persistent launch over
-// order[bounds[cls], bounds[cls + 1]) (device bounds, from classify).  `cursor`
-// (device, zero before the launch) is the class's queue head.
-int launch_align_class(int cls, const uint32_t *packed, const uint32_t *nib,
-                       const Alphabet &ab, const uint64_t *offs, const uint2 *pairs,
-                       const uint32_t *order, const uint32_t *bounds, uint32_t *scores,
-                       uint32_t identity, unsigned long long *work, unsigned int *cursor,
-                       cudaStream_t s);
+// What every class of one batched round reads and writes.
+struct RoundArgs {
+  const uint32_t *rows;   // records whose planes fill the tables (residue or aligner codes)
+  const uint32_t *packed; // records with residue-code planes
+  const uint32_t *nib;    // records as aligner-code nibbles
+  const uint64_t *offs;
+  const uint32_t *lens;
+  const uint2 *pairs;
+  const uint32_t *order, *bounds;
+  unsigned int *cursors;  // pairs taken from each class's queue (zero at launch)
+  uint32_t *scores;
+  float t;
+  int fm;
+  unsigned long long *work;
+};
+
+// Blocks of a persistent launch: as many as fit on the device at once, and no
+// more than `want`.  Occupancy is looked up once per (kernel, device).
+int persistent_grid(const void *func, int threads, size_t smem, uint32_t want, uint32_t *grid);
+// The width classes of one batched round as persistent launches, `kernel` one
+// of 0 .. kAlignKernels - 1 (independent of one another; each takes the pairs
+// of its classes through their cursors, zero before the launch).  m: the
+// round's pairs, an upper bound of any class's.
+constexpr int kAlignKernels = 5;
+int launch_align(int kernel, const RoundArgs &a, int K, uint32_t m, cudaStream_t s);
 // All layouts of records offs[0..n) in one pass under an assumed code map
 // (inv: nibble d = residue code of aligner code d, pipelined loads): nibbles,
 // recoded nibbles and code planes.  *bad = 1 if a residue has a code outside
@@ -122,10 +139,11 @@ int collect_write(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_
                   cudaStream_t s);
 // Width class sort keys of `count` pairs, per-class counts (added to
 // class_count), band cells (added to *cells) and the class bounds of the
-// class-major order (bounds[c] = pairs in classes below c; kNumClasses + 1
-// entries, written after the counts are complete).
+// class-major order (bounds[c] = pairs in classes below c; kNumRoundClasses +
+// 1 entries, written after the counts are complete).  widest: the widest
+// sliding window to use (widest_window).
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
-             const ClassPlan &plan, uint32_t *cls, unsigned int *class_count,
+             const ClassPlan &plan, uint32_t widest, uint32_t *cls, unsigned int *class_count,
              unsigned long long *cells, uint32_t *bounds, cudaStream_t s);
 int bits_for(uint32_t max_value);
 // The part-th of `parts` contiguous ranges [h_cut[0], h_cut[1]) of the pairs,

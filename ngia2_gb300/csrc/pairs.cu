@@ -269,13 +269,13 @@ constexpr uint32_t kClassifyUnroll = 4;
 
 __global__ void __launch_bounds__(256)
 classify_kernel(const uint32_t *__restrict__ lens, const uint2 *__restrict__ pairs,
-                uint64_t count, float t, int fma_mode, ClassPlan plan,
+                uint64_t count, float t, int fma_mode, ClassPlan plan, uint32_t widest,
                 uint32_t *__restrict__ cls,
                 unsigned int *__restrict__ class_count,
                 unsigned long long *__restrict__ cells) {
-  __shared__ unsigned int sc[kNumClasses];
+  __shared__ unsigned int sc[kNumRoundClasses];
   __shared__ unsigned long long scells;
-  if (threadIdx.x < kNumClasses) sc[threadIdx.x] = 0;
+  if (threadIdx.x < kNumRoundClasses) sc[threadIdx.x] = 0;
   if (threadIdx.x == 0) scells = 0;
   __syncthreads();
   unsigned long long my_cells = 0;
@@ -308,7 +308,7 @@ classify_kernel(const uint32_t *__restrict__ lens, const uint2 *__restrict__ pai
           cls[p] = skip_sort_key();
         } else {
           const Band b = make_band(lr[u], lt[u], t, fma_mode);
-          c = (uint32_t)width_class(b, plan);
+          c = (uint32_t)round_class(b, plan, widest);
           cls[p] = class_sort_key((int)c, b);
           my_cells += band_blocks(b);
         }
@@ -319,24 +319,27 @@ classify_kernel(const uint32_t *__restrict__ lens, const uint2 *__restrict__ pai
   }
   atomicAdd(&scells, my_cells);
   __syncthreads();
-  if (threadIdx.x < kNumClasses && sc[threadIdx.x]) atomicAdd(&class_count[threadIdx.x], sc[threadIdx.x]);
+  if (threadIdx.x < kNumRoundClasses && sc[threadIdx.x]) atomicAdd(&class_count[threadIdx.x], sc[threadIdx.x]);
   if (threadIdx.x == 0 && scells) atomicAdd(cells, scells * 1024ull);
 }
 
 __global__ void class_bounds_kernel(const unsigned int *__restrict__ class_count,
                                     uint32_t *__restrict__ bounds) {
-  if (threadIdx.x == 0) {
-    uint32_t run = 0;
-    for (int c = 0; c < kNumClasses; ++c) {
-      bounds[c] = run;
-      run += class_count[c];
-    }
-    bounds[kNumClasses] = run;
+  static_assert(kNumRoundClasses <= 32, "one warp");
+  const uint32_t lane = threadIdx.x;
+  const uint32_t v = lane < kNumRoundClasses ? class_count[lane] : 0u;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, x, o);
+    if (lane >= (uint32_t)o) x += y;
   }
+  if (lane < kNumRoundClasses) bounds[lane] = x - v;
+  if (lane == 31) bounds[kNumRoundClasses] = x;
 }
 
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
-             const ClassPlan &plan, uint32_t *cls, unsigned int *class_count,
+             const ClassPlan &plan, uint32_t widest, uint32_t *cls, unsigned int *class_count,
              unsigned long long *cells, uint32_t *bounds, cudaStream_t s) {
   if (count > 0) {
     int dev = 0, sms = 0;
@@ -344,7 +347,7 @@ int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t 
     NGIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const uint32_t want = ceil_div(count, 256u), cap = (uint32_t)sms * 8;
     classify_kernel<<<want < cap ? want : cap, 256, 0, s>>>(
-        lens, pairs, count, identity_threshold(identity), round_mode(), plan, cls,
+        lens, pairs, count, identity_threshold(identity), round_mode(), plan, widest, cls,
         class_count, cells);
     NGIA_LAUNCHED();
   }

@@ -128,28 +128,35 @@ int Round::enqueue(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t id
   cudaStream_t s = stream;
   Counters *dc = counters();
   NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
-  NGIA_TRY(classify(db.lens, pairs, m, identity, plan, cls_.as<uint32_t>(), dc->class_count,
-                    &dc->cells, dc->bounds, s));
+  NGIA_TRY(classify(db.lens, pairs, m, identity, plan, widest_window(db.ab.K),
+                    cls_.as<uint32_t>(), dc->class_count, &dc->cells, dc->bounds, s));
   NGIA_TRY(radix_sort_pairs(cls_.as<uint32_t>(), nullptr, cls_sorted_.as<uint32_t>(),
                             order_.as<uint32_t>(), m, 1, 0, kClassKeyBits, sort_tmp_.p, s));
   NGIA_CUDA(cudaMemsetAsync(scores, 0, (size_t)(m ? m : 1) * 4, s));
   if (ev_mid) NGIA_CUDA(cudaEventRecord(ev_mid, s));
   if (m == 0) return NGIA_OK;
-  // classes as concurrent branches, widest first (dealt round-robin over the
-  // side streams): the few long pairs' warps leave most of the device to the
-  // other classes instead of running alone at the end
-  int launch_order[kNumClasses - 1];
-  launch_order[0] = kGeneralClass;
-  for (int c = 1; c < kNumClasses - 1; ++c) launch_order[c] = kGeneralClass - c;
+  // the kernels as concurrent branches, widest classes first: the few long
+  // pairs' warps leave most of the device to the others instead of running
+  // alone at the end
+  const RoundArgs args{db.ab.K < 16 ? db.ab.dplanes : db.packed,
+                       db.packed,
+                       db.nib,
+                       db.offs,
+                       db.lens,
+                       pairs,
+                       order_.as<uint32_t>(),
+                       dc->bounds,
+                       dc->cursor,
+                       scores,
+                       identity_threshold(identity),
+                       round_mode(),
+                       &dc->work};
+  if (!args.rows) return NGIA_ERR_STATE;
   NGIA_CUDA(cudaEventRecord(fork_, s));
   for (int k = 0; k < kSide; ++k) NGIA_CUDA(cudaStreamWaitEvent(side_[k], fork_, 0));
-  int k = 0;
-  for (int cl : launch_order) {
-    NGIA_TRY(launch_align_class(cl, db.packed, db.nib, db.ab, db.offs, pairs,
-                                order_.as<uint32_t>(), dc->bounds, scores, identity, &dc->work,
-                                &dc->cursor[cl], side_[k]));
-    k = (k + 1) % kSide;
-  }
+  static_assert(kAlignKernels == kSide + 1, "one branch per kernel");
+  for (int k = 0; k < kAlignKernels; ++k)
+    NGIA_TRY(launch_align(k, args, db.ab.K, m, k < kSide ? side_[k] : s));
   for (int j = 0; j < kSide; ++j) {
     NGIA_CUDA(cudaEventRecord(join_[j], side_[j]));
     NGIA_CUDA(cudaStreamWaitEvent(s, join_[j], 0));

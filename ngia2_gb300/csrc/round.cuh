@@ -33,11 +33,11 @@ struct Counters {  // device-side counters of one graph build or round
   unsigned long long cand_total;
   unsigned long long cells;
   uint64_t unique_total;
-  unsigned int class_count[kNumClasses];
+  unsigned int class_count[kNumRoundClasses];
   uint32_t fast_count;
   unsigned long long work;  // 32x32 blocks the aligners computed
-  unsigned int cursor[kNumClasses];  // pairs taken from each class's queue
-  uint32_t bounds[kNumClasses + 1];  // class ranges of the queue order
+  unsigned int cursor[kNumRoundClasses];  // pairs taken from each class's queue
+  uint32_t bounds[kNumRoundClasses + 1];  // class ranges of the queue order
   unsigned int collect_ticket, collect_error;  // the one-pass candidate collection
 };
 
@@ -79,7 +79,7 @@ class Round {
   // The batched aligner over m device pairs into scores, enqueued on the
   // round's stream with no host round trip: counters zeroed, width classes
   // and their bounds, class-major queue order (longest first), scores
-  // zeroed, one persistent launch per class as concurrent branches.  Events
+  // zeroed, the classes as concurrent persistent launches.  Events
   // ev_start/ev_mid/ev_end (may be null) are recorded around it.
   int enqueue(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t identity,
               uint32_t *scores, cudaEvent_t ev_mid);
