@@ -36,28 +36,6 @@ align_jobs_kernel(const uint32_t *__restrict__ packed,
   jobs[3 * j + 2] = identity_score(lcs, lr, lt, t);
 }
 
-// Same over a job list whose length lives in device memory (graph-capturable
-// per-band rounds of fast mode).  Grid-stride.
-__global__ void __launch_bounds__(128)
-align_jobs_dev_count_kernel(const uint32_t *__restrict__ packed,
-                            const uint64_t *__restrict__ offs,
-                            uint32_t *__restrict__ jobs,
-                            const uint32_t *__restrict__ d_count, float t,
-                            int fma_mode) {
-  const uint32_t count = *d_count;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count;
-       j += gridDim.x * blockDim.x) {
-    const uint32_t *rep = packed + offs[jobs[3 * j]];
-    const uint32_t *tar = packed + offs[jobs[3 * j + 1]];
-    const uint32_t lr = __ldg(rep), lt = __ldg(tar);
-    const Band b = make_band(lr, lt, t, fma_mode);
-    if (!b.pass) continue;
-    uint32_t lines[kMaxRowBlocks];
-    const uint32_t lcs = lcs_any(rep, tar, b, lines);
-    jobs[3 * j + 2] = identity_score(lcs, lr, lt, t);
-  }
-}
-
 // Load-time layout kernels: one warp per record, lane k taking the record's
 // 32-residue blocks k, k + 32, ... (four words each, coalesced across the
 // warp); bit work by shifts and masks, no per-residue loops.
@@ -377,18 +355,6 @@ int launch_align_jobs(const uint32_t *packed, const uint64_t *offs, uint32_t *jo
   if (count == 0) return NGIA_OK;
   align_jobs_kernel<<<ceil_div(count, 128u), 128, 0, s>>>(
       packed, offs, jobs, count, identity_threshold(identity), round_mode());
-  NGIA_LAUNCHED();
-  return NGIA_OK;
-}
-
-int launch_align_jobs_dev_count(const uint32_t *packed, const uint64_t *offs,
-                                uint32_t *jobs, const uint32_t *d_count,
-                                uint32_t max_count, uint32_t identity,
-                                cudaStream_t s) {
-  if (max_count == 0) return NGIA_OK;
-  const uint32_t blocks = ceil_div(max_count, 128u);
-  align_jobs_dev_count_kernel<<<blocks, 128, 0, s>>>(
-      packed, offs, jobs, d_count, identity_threshold(identity), round_mode());
   NGIA_LAUNCHED();
   return NGIA_OK;
 }

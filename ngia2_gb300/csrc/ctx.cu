@@ -153,7 +153,7 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   // buffer holds the worst case, bands x n)
   NGIA_TRY(c->pairs.reserve((size_t)bands * n * 8));
   uint2 *pairs = c->pairs.as<uint2>();
-  NGIA_TRY(collect_scan(rep, lens, n, bands, identity, &dc->collect_ticket,
+  NGIA_TRY(collect_scan(rep, lens, nullptr, n, bands, identity, &dc->collect_ticket,
                         reinterpret_cast<unsigned long long *>(c->uoff.p), &dc->cand_total,
                         &dc->unique_total, &dc->collect_error, pairs, s));
   Counters hc;
@@ -234,17 +234,44 @@ int ctx_fast_cluster(ngia_ctx *c, uint32_t identity, uint32_t bands, uint32_t *h
   if (bands < 1 || bands > c->rep_bands) return NGIA_ERR_ARG;
   cudaStream_t s = c->stream;
   const uint32_t n = c->n;
+  const uint32_t *rep = c->rep.as<uint32_t>();
   NGIA_TRY(c->counters.reserve(sizeof(Counters)));
-  NGIA_TRY(c->jobs.reserve((size_t)n * 12));
-  NGIA_TRY(c->ucount.reserve((size_t)n * 4));  // parent pointers
+  NGIA_TRY(c->uoff.reserve((size_t)n * 8));
+  NGIA_TRY(c->ucount.reserve((size_t)n * 4));  // first bands, then parent pointers
   uint32_t *parent = c->ucount.as<uint32_t>();
   Counters *dc = c->counters.as<Counters>();
   NGIA_CUDA(cudaMemsetAsync(parent, 0xFF, (size_t)n * 4, s));
   NGIA_CUDA(cudaEventRecord(c->ev[0], s));
-  for (uint32_t b = 0; b < bands; ++b)
-    NGIA_TRY(fast_round(c->packed.as<uint32_t>(), c->offs.as<uint64_t>(),
-                        c->rep.as<uint32_t>() + (size_t)b * n, parent, n, identity,
-                        c->jobs.as<uint32_t>(), &dc->fast_count, s));
+  // Runs of bands 0-3, 4-15 and the rest, shorter where bands x n would pass
+  // 2^30 pair slots.  One run would align, for a target with many close
+  // relatives, every distinct rep of 64 bands where the first usually scores;
+  // a run per band costs 64 rounds (20,000 proteins, families of ten close
+  // relatives, identity 90: 16.3 ms one band at a time through the
+  // one-thread-per-pair kernel, 0.6 ms so).
+  const uint32_t most = (1u << 30) / n ? (1u << 30) / n : 1u;
+  for (uint32_t b0 = 0, b1; b0 < bands; b0 = b1) {
+    const uint32_t end = b0 < 4 ? 4u : b0 < 16 ? 16u : (uint32_t)kBands;
+    b1 = std::min(std::min(end, bands), b0 + most);
+    NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
+    NGIA_TRY(c->pairs.reserve((size_t)(b1 - b0) * n * 8));
+    uint2 *pairs = c->pairs.as<uint2>();
+    NGIA_TRY(collect_scan(rep + (size_t)b0 * n, c->lens.as<uint32_t>(), parent, n, b1 - b0,
+                          identity, &dc->collect_ticket,
+                          reinterpret_cast<unsigned long long *>(c->uoff.p), &dc->cand_total,
+                          &dc->unique_total, &dc->collect_error, pairs, s));
+    Counters hc;
+    NGIA_CUDA(cudaMemcpyAsync(&hc, dc, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+    NGIA_CUDA(cudaStreamSynchronize(s));
+    if (hc.collect_error) return NGIA_ERR_CUDA;
+    const uint32_t m = (uint32_t)hc.unique_total;
+    if (m == 0) continue;
+    NGIA_TRY(c->scores.reserve((size_t)m * 4));
+    uint32_t *scores = c->scores.as<uint32_t>();
+    NGIA_TRY(c->round.reserve(m));
+    NGIA_TRY(c->round.enqueue(db_view(c), pairs, m, identity, scores, nullptr));
+    NGIA_TRY(fast_first_band(rep, n, b0, b1, pairs, scores, m, parent, s));
+  }
+  NGIA_TRY(fast_parents(rep, n, parent, s));
   NGIA_CUDA(cudaEventRecord(c->ev[1], s));
   std::vector<uint32_t> par(n);
   NGIA_CUDA(cudaMemcpyAsync(par.data(), parent, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
@@ -626,7 +653,7 @@ void ngia_ctx_destroy(ngia_ctx *c) {
                           &c->offs,     &c->lens,  &c->rep,       &c->sigs,     &c->ucount,
                           &c->uoff,
                           &c->counters, &c->pairs, &c->scores,    &c->sort_tmp, &c->emit_tmp,
-                          &c->edges,    &c->scan_tmp, &c->jobs, &c->sketch_table};
+                          &c->edges,    &c->scan_tmp, &c->sketch_table};
   for (ngia::DevBuf *b : bufs) b->release();
   c->round.destroy();  // shares c->stream, which it leaves alone
   for (int k = 0; k < ngia_ctx::kEvents; ++k)
@@ -719,7 +746,7 @@ int ngia_ctx_test_lookback_timeout(ngia_ctx *c, uint32_t identity, uint32_t band
   NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
   const unsigned int one = 1;  // the first ticket handed out is 1: block 0 never publishes
   NGIA_CUDA(cudaMemcpyAsync(&dc->collect_ticket, &one, sizeof(one), cudaMemcpyHostToDevice, s));
-  NGIA_TRY(collect_scan(c->rep.as<uint32_t>(), c->lens.as<uint32_t>(), n, bands, identity,
+  NGIA_TRY(collect_scan(c->rep.as<uint32_t>(), c->lens.as<uint32_t>(), nullptr, n, bands, identity,
                         &dc->collect_ticket, reinterpret_cast<unsigned long long *>(c->uoff.p),
                         &dc->cand_total, &dc->unique_total, &dc->collect_error,
                         c->pairs.as<uint2>(), s, spin_limit));

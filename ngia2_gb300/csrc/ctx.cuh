@@ -43,7 +43,7 @@ struct ngia_ctx {
   uint64_t table_inv = 0;  // the aligner-code map the sketch tables were built for
   ngia::DevBuf sketch_table;
   // graph build work
-  ngia::DevBuf ucount, uoff, counters, pairs, scores, emit_tmp, edges, scan_tmp, jobs,
+  ngia::DevBuf ucount, uoff, counters, pairs, scores, emit_tmp, edges, scan_tmp,
       sort_tmp;
   uint64_t n_edges = 0;
   // the batched aligner (scratch, side streams, plan, cached graph) on `stream`

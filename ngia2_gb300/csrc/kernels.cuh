@@ -51,10 +51,6 @@ int bucket(const uint32_t *sigs, uint32_t n, uint32_t bands, uint32_t *rep,
 // align.cu
 int launch_align_jobs(const uint32_t *packed, const uint64_t *offs, uint32_t *jobs,
                       uint32_t count, uint32_t identity, cudaStream_t s);
-int launch_align_jobs_dev_count(const uint32_t *packed, const uint64_t *offs,
-                                uint32_t *jobs, const uint32_t *d_count,
-                                uint32_t max_count, uint32_t identity,
-                                cudaStream_t s);
 // Alphabet of the target codes the aligner reads: codes 1..K-1 in use;
 // inv packs, per code d < K, the residue code whose match mask d stands for
 // (identity when the codes were not recoded).
@@ -125,12 +121,14 @@ int launch_pack_layout(const uint8_t *res, const uint64_t *starts, const uint32_
 // Candidate pairs in one pass (see pairs.cu): pairs[] must hold bands * n;
 // *ticket and *unique_total zero before the call, status[] holds
 // ceil(n / 32) words (cleared here); *error set if a look-back gave up after
-// spin_limit polls of a predecessor's status.
+// spin_limit polls of a predecessor's status.  taken: null, or targets whose
+// entry is not 0xFFFFFFFF are left out.
 constexpr uint32_t kLookbackSpins = 1u << 22;
-int collect_scan(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_t bands,
-                 uint32_t identity, unsigned int *ticket, unsigned long long *status,
-                 unsigned long long *cand_total, uint64_t *unique_total, unsigned int *error,
-                 uint2 *pairs, cudaStream_t s, uint32_t spin_limit = kLookbackSpins);
+int collect_scan(const uint32_t *rep, const uint32_t *lens, const uint32_t *taken, uint32_t n,
+                 uint32_t bands, uint32_t identity, unsigned int *ticket,
+                 unsigned long long *status, unsigned long long *cand_total,
+                 uint64_t *unique_total, unsigned int *error, uint2 *pairs, cudaStream_t s,
+                 uint32_t spin_limit = kLookbackSpins);
 int collect_count(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_t bands,
                   uint32_t identity, uint32_t *ucount, unsigned long long *cand_total,
                   cudaStream_t s);
@@ -158,8 +156,12 @@ size_t emit_scratch_bytes(uint32_t count, uint32_t n_nodes);
 int emit_sorted(const uint2 *pairs, const uint32_t *scores, uint32_t count,
                 uint32_t n_nodes, ngia_edge *out, uint64_t *h_m, void *scratch,
                 cudaStream_t s);
-int fast_round(const uint32_t *packed, const uint64_t *offs, const uint32_t *rep_row,
-               uint32_t *parent, uint32_t n, uint32_t identity, uint32_t *jobs,
-               uint32_t *d_count, cudaStream_t s);
+// Fast mode's bands [b0, b1): first_band[target] = min of itself and the first
+// of those bands that names the rep of a pair scoring > 0.
+int fast_first_band(const uint32_t *rep, uint32_t n, uint32_t b0, uint32_t b1,
+                    const uint2 *pairs, const uint32_t *scores, uint32_t m,
+                    uint32_t *first_band, cudaStream_t s);
+// first_band[i] (0xFFFFFFFF: none) -> parent[i], in place.
+int fast_parents(const uint32_t *rep, uint32_t n, uint32_t *parent, cudaStream_t s);
 
 }  // namespace ngia

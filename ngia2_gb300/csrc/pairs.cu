@@ -106,14 +106,15 @@ collect_kernel(const uint32_t *__restrict__ rep, const uint32_t *__restrict__ le
 // length gathers read once.  status[] (zero before the launch): per block,
 // bits 62-63 = 0 not ready / 1 its own count / 2 the prefix through it, bits
 // 0-61 the value.  A look-back that waits too long sets *error and the block
-// writes nothing.
+// writes nothing.  taken (may be null): targets whose entry is not kFull have
+// no pairs (fast mode's assigned targets).
 constexpr unsigned long long kStAgg = 1ull << 62, kStIncl = 2ull << 62;
 constexpr unsigned long long kStValue = (1ull << 62) - 1;
 
 __global__ void __launch_bounds__(kPairThreads)
 collect_scan_kernel(const uint32_t *__restrict__ rep, const uint32_t *__restrict__ lens,
-                    uint32_t n, uint32_t bands, float t, unsigned int *__restrict__ ticket,
-                    unsigned long long *__restrict__ status,
+                    const uint32_t *__restrict__ taken, uint32_t n, uint32_t bands, float t,
+                    unsigned int *__restrict__ ticket, unsigned long long *__restrict__ status,
                     unsigned long long *__restrict__ cand_total,
                     uint64_t *__restrict__ unique_total, unsigned int *__restrict__ error,
                     uint2 *__restrict__ pairs, uint32_t spin_limit) {
@@ -143,7 +144,7 @@ collect_scan_kernel(const uint32_t *__restrict__ rep, const uint32_t *__restrict
   for (uint32_t k = 0; k < kPer; ++k) {
     const uint32_t c = warp + k * (kPairThreads / 32), i = i0 + c;
     uint32_t u = 0;
-    if (i < n) {
+    if (i < n && (!taken || __ldg(taken + i) == kFull)) {  // warp-uniform
       ts[k] = scan_target(tile, c, i, lens, bands, t, vals[warp]);
       cand_sum += ts[k].cand;
       u = __popc(ts[k].first0) + __popc(ts[k].first1);
@@ -227,14 +228,15 @@ collect_scan_kernel(const uint32_t *__restrict__ rep, const uint32_t *__restrict
   if (lane == 0 && cand_sum) atomicAdd(cand_total, (unsigned long long)cand_sum);
 }
 
-int collect_scan(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_t bands,
-                 uint32_t identity, unsigned int *ticket, unsigned long long *status,
-                 unsigned long long *cand_total, uint64_t *unique_total, unsigned int *error,
-                 uint2 *pairs, cudaStream_t s, uint32_t spin_limit) {
+int collect_scan(const uint32_t *rep, const uint32_t *lens, const uint32_t *taken, uint32_t n,
+                 uint32_t bands, uint32_t identity, unsigned int *ticket,
+                 unsigned long long *status, unsigned long long *cand_total,
+                 uint64_t *unique_total, unsigned int *error, uint2 *pairs, cudaStream_t s,
+                 uint32_t spin_limit) {
   if (n == 0) return NGIA_OK;
   const uint32_t nblocks = ceil_div(n, kTargetsPerBlock);
   NGIA_CUDA(cudaMemsetAsync(status, 0, (size_t)nblocks * 8, s));
-  collect_scan_kernel<<<nblocks, kPairThreads, 0, s>>>(rep, lens, n, bands,
+  collect_scan_kernel<<<nblocks, kPairThreads, 0, s>>>(rep, lens, taken, n, bands,
                                                        identity_threshold(identity), ticket,
                                                        status, cand_total, unique_total, error,
                                                        pairs, spin_limit);
@@ -614,52 +616,49 @@ int emit_sorted(const uint2 *pairs, const uint32_t *scores, uint32_t count,
 }
 
 // ---- fast mode ------------------------------------------------------------------------
-// Jobs of one band (src/fastClustering.hpp:256-258): rep[i] != i and i not
-// yet assigned.  The order of jobs inside a band does not affect the result
-// (each target appears once per band), so they are appended with one atomic
-// per warp.
+// In band order a target is assigned to the rep of the first band whose pair
+// scores > 0 (src/fastClustering.hpp:256-258, 330-334).  Nothing but the
+// target's own earlier bands decides it, so the bands need not run one after
+// another: a run of bands [b0, b1) is collected for the targets still
+// unassigned, its distinct pairs are aligned in one batched round, and each
+// pair that scored lowers its target's first band to the first one of the run
+// that names its rep.
 __global__ void __launch_bounds__(256)
-fast_jobs_kernel(const uint32_t *__restrict__ rep_row, const uint32_t *__restrict__ parent,
-                 uint32_t n, uint32_t *__restrict__ jobs, uint32_t *__restrict__ d_count) {
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t r = i < n ? rep_row[i] : 0u;
-    const bool job = i < n && r != i && parent[i] == kFull;
-    const uint32_t bal = __ballot_sync(kFull, job);
-    uint32_t slot = 0;
-    if (lane == 0 && bal) slot = atomicAdd(d_count, (uint32_t)__popc(bal));
-    slot = __shfl_sync(kFull, slot, 0) + __popc(bal & ((1u << lane) - 1u));
-    if (job) {
-      jobs[3 * (size_t)slot] = r;
-      jobs[3 * (size_t)slot + 1] = i;
-      jobs[3 * (size_t)slot + 2] = 0;
-    }
+fast_first_band_kernel(const uint32_t *__restrict__ rep, uint32_t n, uint32_t b0, uint32_t b1,
+                       const uint2 *__restrict__ pairs, const uint32_t *__restrict__ scores,
+                       uint32_t m, uint32_t *__restrict__ first_band) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m;
+       p += gridDim.x * blockDim.x) {
+    if (scores[p] == 0) continue;
+    const uint2 pr = pairs[p];
+    uint32_t b = b0;
+    while (b + 1 < b1 && __ldg(rep + (size_t)b * n + pr.y) != pr.x) ++b;
+    atomicMin(first_band + pr.y, b);
   }
 }
 
-// A hit assigns the target to its rep (src/fastClustering.hpp:330-334).
+// first_band[i] -> the rep that band names (kFull: unassigned)
 __global__ void __launch_bounds__(256)
-fast_assign_kernel(const uint32_t *__restrict__ jobs, const uint32_t *__restrict__ d_count,
-                   uint32_t *__restrict__ parent) {
-  const uint32_t count = *d_count;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count;
-       j += gridDim.x * blockDim.x)
-    if (jobs[3 * (size_t)j + 2] > 0) parent[jobs[3 * (size_t)j + 1]] = jobs[3 * (size_t)j];
+fast_parent_kernel(const uint32_t *__restrict__ rep, uint32_t n, uint32_t *__restrict__ parent) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t b = parent[i];
+  if (b != kFull) parent[i] = rep[(size_t)b * n + i];
 }
 
-int fast_round(const uint32_t *packed, const uint64_t *offs, const uint32_t *rep_row,
-               uint32_t *parent, uint32_t n, uint32_t identity, uint32_t *jobs,
-               uint32_t *d_count, cudaStream_t s) {
-  int dev = 0, sms = 0;
-  NGIA_CUDA(cudaGetDevice(&dev));
-  NGIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  NGIA_CUDA(cudaMemsetAsync(d_count, 0, sizeof(uint32_t), s));
-  const uint32_t want = ceil_div(n, 256u), cap = (uint32_t)sms * 8;
-  fast_jobs_kernel<<<want < cap ? want : cap, 256, 0, s>>>(rep_row, parent, n, jobs, d_count);
+int fast_first_band(const uint32_t *rep, uint32_t n, uint32_t b0, uint32_t b1,
+                    const uint2 *pairs, const uint32_t *scores, uint32_t m,
+                    uint32_t *first_band, cudaStream_t s) {
+  if (m == 0) return NGIA_OK;
+  const uint32_t want = ceil_div(m, 256u);
+  fast_first_band_kernel<<<want < 65536u ? want : 65536u, 256, 0, s>>>(rep, n, b0, b1, pairs,
+                                                                        scores, m, first_band);
   NGIA_LAUNCHED();
-  NGIA_TRY(launch_align_jobs_dev_count(packed, offs, jobs, d_count, n, identity, s));
-  fast_assign_kernel<<<want < cap ? want : cap, 256, 0, s>>>(jobs, d_count, parent);
+  return NGIA_OK;
+}
+
+int fast_parents(const uint32_t *rep, uint32_t n, uint32_t *parent, cudaStream_t s) {
+  fast_parent_kernel<<<ceil_div(n, 256u), 256, 0, s>>>(rep, n, parent);
   NGIA_LAUNCHED();
   return NGIA_OK;
 }

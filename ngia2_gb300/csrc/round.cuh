@@ -34,7 +34,6 @@ struct Counters {  // device-side counters of one graph build or round
   unsigned long long cells;
   uint64_t unique_total;
   unsigned int class_count[kNumRoundClasses];
-  uint32_t fast_count;
   unsigned long long work;  // 32x32 blocks the aligners computed
   unsigned int cursor[kNumRoundClasses];  // pairs taken from each class's queue
   uint32_t bounds[kNumRoundClasses + 1];  // class ranges of the queue order
