@@ -119,7 +119,7 @@ int ctx_sketch_bucket(ngia_ctx *c, uint32_t bands, ngia_stats *st, bool sketch_d
     else {
       NGIA_TRY(ctx_ready_layouts(c));  // a pieced load leaves the nibbles out
       NGIA_TRY(launch_sketch_nibbles(c->nib.as<uint32_t>(), c->offs.as<uint64_t>(), c->n,
-                                     c->sigs.as<uint32_t>(), s));
+                                     c->sigs.as<uint32_t>(), c->n, kBands, s));
     }
     NGIA_CUDA(cudaEventRecord(c->ev[9], s));
   }

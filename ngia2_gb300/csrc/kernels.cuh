@@ -9,8 +9,9 @@ namespace ngia {
 // sketch.cu
 int launch_sketch(const uint32_t *packed, const uint64_t *offs, uint32_t n,
                   uint32_t *sigs, cudaStream_t s);
+// Bands 0 .. bands - 1 only, band b of record i at sigs[b * stride + i].
 int launch_sketch_nibbles(const uint32_t *nib, const uint64_t *offs, uint32_t n,
-                          uint32_t *sigs, cudaStream_t s);
+                          uint32_t *sigs, size_t stride, uint32_t bands, cudaStream_t s);
 // Databases of at most four residue codes (none of them 0): an 8-mer is one of
 // kSketchTableEntries values.  build_sketch_table fills sketch_table_bytes()
 // of device memory from the aligner codes' inverse map (part of the band

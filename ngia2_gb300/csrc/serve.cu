@@ -209,7 +209,8 @@ static int run_request(Server *s, Slot *sl, Request *r) {
   if (s->recode_map)
     NGIA_TRY(launch_dense_layouts(packed, offs, q, s->recode_map, s->dense.as<uint32_t>(),
                                   s->dplanes.as<uint32_t>(), st));
-  NGIA_TRY(launch_sketch_nibbles(s->nib.as<uint32_t>(), offs, q, sl->sigs.as<uint32_t>(), st));
+  NGIA_TRY(launch_sketch_nibbles(s->nib.as<uint32_t>(), offs, q, sl->sigs.as<uint32_t>(), q,
+                                 kBands, st));
   const uint32_t slots = q * (uint32_t)kBands;
   lookup_kernel<<<ceil_div(slots, 256u), 256, 0, st>>>(s->keys.as<uint32_t>(),
                                                        s->vals.as<uint32_t>(), s->n,

@@ -134,15 +134,84 @@ sketch_kernel(const uint32_t *__restrict__ words, const uint64_t *__restrict__ o
   }
 }
 
+// Bands [NB * blockIdx.y, ...) below `bands` only, signatures at sigs[band *
+// stride + i]: one warp per record and run of NB bands, the band seeds in
+// registers.
+template <typename Source, int NB>
+__global__ void __launch_bounds__(256)
+sketch_bands_kernel(const uint32_t *__restrict__ words, const uint64_t *__restrict__ offs,
+                    uint32_t n, uint32_t *__restrict__ sigs, size_t stride, uint32_t bands) {
+  static_assert(NB <= 32, "one lane per band writes");
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t band0 = blockIdx.y * NB;
+  uint32_t fold[NB];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) fold[k] = band_seed_fold(band0 + (uint32_t)k);
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const uint32_t *rec = words + offs[i];
+    const uint32_t len = __ldg(rec);
+    const uint32_t first = len >= 8 ? 7u : (len > 0 ? len - 1 : 0u);
+    const uint32_t per = (len - first + 31u) >> 5;
+    const uint32_t pb = first + lane * per;
+    const uint32_t pe = min(pb + per, len);
+    uint32_t mn[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) mn[k] = kFull;
+    if (pb < pe) {
+      Source src = Source::make(rec);
+      src.start(pb);
+      for (uint32_t p = pb; p < pe; ++p) {
+        const uint32_t kmer = src.at(p);
+        const uint32_t y = kmer ^ (kmer >> 16);
+#pragma unroll
+        for (int k = 0; k < NB; ++k) mn[k] = min(mn[k], band_hash_tail(y ^ fold[k]));
+      }
+    }
+    uint32_t mine = kFull;
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      const uint32_t r = __reduce_min_sync(kFull, mn[k]);
+      if ((uint32_t)k == lane) mine = r;
+    }
+    if (lane < (uint32_t)NB && band0 + lane < bands) sigs[(band0 + lane) * stride + i] = mine;
+  }
+}
+
+template <typename Source, int NB>
+static int launch_bands(const uint32_t *words, const uint64_t *offs, uint32_t n, uint32_t *sigs,
+                        size_t stride, uint32_t bands, uint32_t cap, cudaStream_t s) {
+  const uint32_t want = ceil_div(n, 8u);  // 8 warps per block
+  sketch_bands_kernel<Source, NB><<<dim3(want < cap ? want : cap, ceil_div(bands, (uint32_t)NB)),
+                                    256, 0, s>>>(words, offs, n, sigs, stride, bands);
+  NGIA_LAUNCHED();
+  return NGIA_OK;
+}
+
 template <typename Source>
 static int launch(const uint32_t *words, const uint64_t *offs, uint32_t n, uint32_t *sigs,
-                  cudaStream_t s) {
+                  size_t stride, uint32_t bands, cudaStream_t s) {
   if (n == 0) return NGIA_OK;
   int dev = 0, sms = 0;
   NGIA_CUDA(cudaGetDevice(&dev));
   NGIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const uint32_t want = ceil_div(n, 8u);  // 8 warps per block
   const uint32_t cap = (uint32_t)sms * 16u;
+  // Fewer bands than the file's 64 are hashed as such (400,009 proteins, 3
+  // bands: 0.23 ms where 64 take 4.8).  All 64 of few records are split over
+  // warps: a warp that hashes 64 bands of a record of 340 takes 8,300
+  // instructions by itself, and fewer records than the device holds warps (16
+  // per multiprocessor with 64 minima each) leave it waiting for that.  64, 16
+  // and 8 bands a warp, proteins: 200 records 35, 13.6, 12.6 us; 600: 35, 20.8,
+  // 20.6; 2,400: 62, 49, 54; 4,800: 82, 87, 92 (every run of bands rolls the
+  // k-mers again).
+  if (bands <= 4) return launch_bands<Source, 4>(words, offs, n, sigs, stride, bands, cap, s);
+  if (bands <= 8 || n <= (uint32_t)sms * 2u)
+    return launch_bands<Source, 8>(words, offs, n, sigs, stride, bands, cap, s);
+  if (bands <= 32 || n <= (uint32_t)sms * 16u)
+    return launch_bands<Source, 16>(words, offs, n, sigs, stride, bands, cap, s);
+  if (bands < (uint32_t)kBands || stride != n)
+    return launch_bands<Source, 32>(words, offs, n, sigs, stride, bands, cap, s);
+  const uint32_t want = ceil_div(n, 8u);  // 8 warps per block
   sketch_kernel<Source><<<want < cap ? want : cap, 256, 0, s>>>(words, offs, n, sigs);
   NGIA_LAUNCHED();
   return NGIA_OK;
@@ -150,12 +219,12 @@ static int launch(const uint32_t *words, const uint64_t *offs, uint32_t n, uint3
 
 int launch_sketch(const uint32_t *packed, const uint64_t *offs, uint32_t n, uint32_t *sigs,
                   cudaStream_t s) {
-  return launch<PlaneKmers>(packed, offs, n, sigs, s);
+  return launch<PlaneKmers>(packed, offs, n, sigs, n, kBands, s);
 }
 
 int launch_sketch_nibbles(const uint32_t *nib, const uint64_t *offs, uint32_t n,
-                          uint32_t *sigs, cudaStream_t s) {
-  return launch<NibbleKmers>(nib, offs, n, sigs, s);
+                          uint32_t *sigs, size_t stride, uint32_t bands, cudaStream_t s) {
+  return launch<NibbleKmers>(nib, offs, n, sigs, stride, bands, s);
 }
 
 // ---- databases of at most four residue codes: tables of all 8-mers -------------

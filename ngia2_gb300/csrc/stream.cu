@@ -209,7 +209,7 @@ __global__ void accumulate_kernel(const Counters *__restrict__ rc,
 
 struct StreamState {
   DevBuf region_packed, region_nib, region_dplanes, r_offs, r_lens;
-  DevBuf offs, lens, sigs, sig_tmp, rep, scratch, ucount, uoff, counters, pairs, scores,
+  DevBuf offs, lens, sigs, rep, scratch, ucount, uoff, counters, pairs, scores,
       keys, keys_sorted, order, block_pairs, block_scores, chunk_first, presence, emit_tmp,
       edges;
   Round round;
@@ -217,7 +217,7 @@ struct StreamState {
   cudaStream_t s = nullptr;
   void destroy() {
     DevBuf *bufs[] = {&region_packed, &region_nib, &region_dplanes, &r_offs, &r_lens,
-                      &offs,          &lens,       &sigs,         &sig_tmp, &rep,
+                      &offs,          &lens,       &sigs,         &rep,
                       &scratch,       &ucount,     &uoff,         &counters, &pairs,
                       &scores,        &keys,       &keys_sorted,  &order,   &block_pairs,
                       &block_scores,  &chunk_first, &presence,    &emit_tmp, &edges};
@@ -269,7 +269,6 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
   NGIA_TRY(S.offs.reserve((size_t)n * 8));
   NGIA_TRY(S.lens.reserve((size_t)n * 4));
   NGIA_TRY(S.sigs.reserve((size_t)bands * n * 4));
-  NGIA_TRY(S.sig_tmp.reserve((size_t)kBands * max_recs * 4));
   NGIA_TRY(S.presence.reserve((size_t)C * 4 + 32));  // one word per chunk, then totals
   unsigned long long *acc =
       reinterpret_cast<unsigned long long *>(S.presence.as<uint32_t>() + ((C + 1) & ~1u));
@@ -317,11 +316,8 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
   for (uint32_t k = 0; k < C; ++k) {
     const int slot = (int)(k & 1u);
     NGIA_TRY(load_chunk(k, slot, 0, S.presence.as<uint32_t>() + k));
-    NGIA_TRY(launch_sketch_nibbles(rn, roffs, chunks[k].count, S.sig_tmp.as<uint32_t>(), s));
-    NGIA_CUDA(cudaMemcpy2DAsync(S.sigs.as<uint32_t>() + chunks[k].first, (size_t)n * 4,
-                                S.sig_tmp.p, (size_t)chunks[k].count * 4,
-                                (size_t)chunks[k].count * 4, bands, cudaMemcpyDeviceToDevice,
-                                s));
+    NGIA_TRY(launch_sketch_nibbles(rn, roffs, chunks[k].count,
+                                   S.sigs.as<uint32_t>() + chunks[k].first, n, bands, s));
     NGIA_TRY(S.stager.slot_free(slot, s));
   }
   {  // residue codes present in any chunk
