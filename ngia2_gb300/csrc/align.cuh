@@ -387,7 +387,7 @@ __host__ __device__ inline int round_class(const Band &b, const ClassPlan &plan,
     words = (uint32_t)wide_width(slide);
     slide += kFirstWideClass;
   }
-  if (b.nr <= 24) {
+  if (b.nr <= (widest < 24u ? widest : 24u)) {
     const int f = b.nr <= 8 ? 0 : b.nr <= 16 ? (int)(b.nr - 7) / 2 : b.nr <= 20 ? 5 : 6;
     if ((uint32_t)fixed_width(f) < words) return kFirstFixedClass + f;
   }

@@ -183,8 +183,12 @@ __device__ inline uint32_t align_group(const uint32_t *__restrict__ packed,
   uint32_t done = 0, wstep = 0;
 
   for (;;) {
-    // groups without a pair take the next ones (one atomic per warp)
-    const uint32_t need = __ballot_sync(kFull, !active && !drained) & group_leaders<G>();
+    // groups without a pair take the next ones (one atomic per warp), at every
+    // fourth step so that each pair meets the exit checks at its own fourth
+    // steps, whatever pairs the warp's other groups hold
+    uint32_t need = __ballot_sync(kFull, !active && !drained) & group_leaders<G>();
+    if (!__any_sync(kFull, active)) wstep = 0;
+    if (wstep & 3u) need = 0;
     if (need) {
       const uint32_t leader = __ffs(need) - 1;
       uint32_t first = 0;
@@ -303,7 +307,8 @@ __device__ inline uint32_t align_group(const uint32_t *__restrict__ packed,
     // bound of the final LCS every fourth step, and the end of the pair
     ++wstep;
     const bool last = active && tau + 1 >= tau_end;
-    const bool check = (wstep & 3u) == 0 || __any_sync(kFull, last);
+    const bool fourth = (wstep & 3u) == 0;
+    const bool check = fourth || __any_sync(kFull, last);
     uint32_t S = 0, qhi1 = 0, ub = 0;
     if (check) {
       uint32_t live = 0;
@@ -322,7 +327,7 @@ __device__ inline uint32_t align_group(const uint32_t *__restrict__ packed,
       uint32_t score = 0;
       if (fin) {
         score = identity_score(S, lr, lt, t);
-      } else if (check && qhi1) {
+      } else if (fourth && qhi1) {
         fin = !lcs_may_reach(ub, lr, lt, t);
       }
       if (fin) {

@@ -70,18 +70,21 @@ align_wide_kernel(const __grid_constant__ RoundArgs a) {
 
 // The group classes of at most eight words per lane, widest first.
 template <int KC>
+__device__ __forceinline__ uint32_t group_classes(const RoundArgs &a, uint32_t *smem) {
+  uint32_t done = group_class<kFirstGroupClass + 6, KC>(a, smem);
+  done += group_class<kFirstGroupClass + 5, KC>(a, smem);
+  done += group_class<kFirstGroupClass + 4, KC>(a, smem);
+  done += group_class<kFirstGroupClass + 3, KC>(a, smem);
+  done += group_class<kFirstGroupClass + 2, KC>(a, smem);
+  done += group_class<kFirstGroupClass + 1, KC>(a, smem);
+  return done + group_class<kFirstGroupClass, KC>(a, smem);
+}
+
+template <int KC>
 __global__ void __launch_bounds__(kGroupThreads)
 align_group_kernel(const __grid_constant__ RoundArgs a) {
   extern __shared__ uint32_t smem[];
-  uint32_t *mine = smem + (threadIdx.x >> 5) * (KC * 8 * 32);
-  uint32_t done = group_class<kFirstGroupClass + 6, KC>(a, mine);
-  done += group_class<kFirstGroupClass + 5, KC>(a, mine);
-  done += group_class<kFirstGroupClass + 4, KC>(a, mine);
-  done += group_class<kFirstGroupClass + 3, KC>(a, mine);
-  done += group_class<kFirstGroupClass + 2, KC>(a, mine);
-  done += group_class<kFirstGroupClass + 1, KC>(a, mine);
-  done += group_class<kFirstGroupClass, KC>(a, mine);
-  count_work(done, a.work);
+  count_work(group_classes<KC>(a, smem + (threadIdx.x >> 5) * (KC * 8 * 32)), a.work);
 }
 
 // The one-pair-per-lane classes in three kernels by width (tier 0: windows of

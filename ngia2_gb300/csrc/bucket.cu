@@ -22,6 +22,7 @@
 // average; the loop is bounded by the bucket's start.
 #include <mutex>
 
+#include "block_sort.cuh"
 #include "kernels.cuh"
 
 namespace ngia {
@@ -162,6 +163,24 @@ rep_resolve_far_kernel(const uint32_t *__restrict__ sk, const uint32_t *__restri
   }
 }
 
+// Few records: one block per band sorts the band's (signature, index) keys in
+// shared memory; a record's rep is its neighbour below when the signatures are
+// equal.  The partition below is a dozen launches of a few microseconds each.
+__global__ void __launch_bounds__(1024)
+bucket_small_kernel(const uint32_t *__restrict__ sigs, uint32_t n, uint32_t *__restrict__ rep) {
+  __shared__ uint64_t keys[kSmallBucket];
+  const uint32_t *sig = sigs + (size_t)blockIdx.x * n;
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) keys[i] = (uint64_t)sig[i] << 32 | i;
+  __syncthreads();
+  block_sort(keys, n);
+  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
+    const uint64_t key = keys[k];
+    const uint64_t below = k ? keys[k - 1] : ~key;
+    const uint32_t i = (uint32_t)key;
+    rep[(size_t)blockIdx.x * n + i] = (below >> 32) == (key >> 32) ? (uint32_t)below : i;
+  }
+}
+
 size_t bucket_scratch_bytes(uint32_t n, uint32_t bands) {
   return 2 * (size_t)n * bands * sizeof(uint32_t) + radix_sort_scratch_bytes(n, bands);
 }
@@ -169,6 +188,13 @@ size_t bucket_scratch_bytes(uint32_t n, uint32_t bands) {
 int bucket(const uint32_t *sigs, uint32_t n, uint32_t bands, uint32_t *rep,
            void *scratch, cudaStream_t s) {
   if (n == 0 || bands == 0) return NGIA_OK;
+  if (n <= kSmallBucket) {
+    // 64 bands of 600 records: 11 us, the partition 33 us; of 4,000: 43 and 50
+    // us; at 4,500 the partition takes 39 us
+    bucket_small_kernel<<<bands, n <= 512 ? 256 : 1024, 0, s>>>(sigs, n, rep);
+    NGIA_LAUNCHED();
+    return NGIA_OK;
+  }
   const size_t total = (size_t)n * bands;
   uint32_t *sk = static_cast<uint32_t *>(scratch);
   uint32_t *sv = sk + total;
@@ -205,6 +231,7 @@ extern "C" int ngia_bucket(const uint32_t *d_sigs, uint32_t n, uint32_t bands,
   if (n == 0) return NGIA_OK;
   if (!d_sigs || !d_rep) return NGIA_ERR_ARG;
   cudaStream_t s = ngia::as_stream(stream);
+  if (n <= ngia::kSmallBucket) return ngia::bucket(d_sigs, n, bands, d_rep, nullptr, s);
   void *scratch = nullptr;
   const size_t bytes = ngia::bucket_scratch_bytes(n, bands);
   cudaError_t e = cudaMallocAsync(&scratch, bytes, s);

@@ -44,7 +44,7 @@ DbView db_view(const ngia_ctx *c) {
 // scratch move, or n or bands change).
 static int bucket_graph(ngia_ctx *c, uint32_t bands) {
   cudaStream_t s = c->stream;
-  if (!c->round.use_graphs)
+  if (!c->round.use_graphs || c->n <= kSmallBucket)
     return bucket(c->sigs.as<uint32_t>(), c->n, bands, c->rep.as<uint32_t>(), c->sort_tmp.p, s);
   const uint64_t key_n = ((uint64_t)c->n << 8) | bands;
   const uint64_t gen = g_alloc_gen.load();
@@ -156,7 +156,12 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   NGIA_TRY(collect_scan(rep, lens, nullptr, n, bands, identity, &dc->collect_ticket,
                         reinterpret_cast<unsigned long long *>(c->uoff.p), &dc->cand_total,
                         &dc->unique_total, &dc->collect_error, pairs, s));
-  Counters hc;
+  if (!c->h_counters) {
+    void *p = nullptr;
+    NGIA_CUDA(cudaHostAlloc(&p, sizeof(*c->h_counters), cudaHostAllocDefault));
+    c->h_counters = static_cast<ngia_ctx::HostCounters *>(p);
+  }
+  Counters &hc = c->h_counters->pairs;
   NGIA_CUDA(cudaMemcpyAsync(&hc, dc, sizeof(Counters), cudaMemcpyDeviceToHost, s));
   NGIA_CUDA(cudaStreamSynchronize(s));
   if (hc.collect_error) return NGIA_ERR_CUDA;  // a look-back gave up (never seen)
@@ -182,17 +187,29 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   NGIA_TRY(c->round.enqueue(db_view(c), pairs, m, identity, scores, c->ev[1]));
   NGIA_CUDA(cudaEventRecord(c->ev[2], s));
   // 4. emit: compact hits, sort by (rep, tar)
-  NGIA_TRY(c->emit_tmp.reserve(emit_scratch_bytes(m, n)));
   NGIA_TRY(c->edges.reserve((size_t)(m ? m : 1) * sizeof(ngia_edge)));
   uint64_t ne = 0;
-  NGIA_TRY(emit_sorted(pairs, scores, m, n, c->edges.as<ngia_edge>(), &ne, c->emit_tmp.p, s));
-  NGIA_CUDA(cudaEventRecord(c->ev[3], s));
-  NGIA_CUDA(cudaEventSynchronize(c->ev[3]));
+  const bool small = m > 0 && m <= kSmallEmit;
+  if (small) {
+    uint64_t *d_m = &dc->unique_total;  // read above, free now
+    NGIA_TRY(emit_small(pairs, scores, m, c->edges.as<ngia_edge>(), d_m, s));
+    NGIA_CUDA(cudaEventRecord(c->ev[3], s));
+    NGIA_CUDA(cudaMemcpyAsync(&c->h_counters->edges, d_m, sizeof(uint64_t),
+                              cudaMemcpyDeviceToHost, s));
+  } else {
+    NGIA_TRY(c->emit_tmp.reserve(emit_scratch_bytes(m, n)));
+    NGIA_TRY(emit_sorted(pairs, scores, m, n, c->edges.as<ngia_edge>(), &ne, c->emit_tmp.p, s));
+    NGIA_CUDA(cudaEventRecord(c->ev[3], s));
+  }
+  Counters &rc = c->h_counters->round;
+  if (st)
+    NGIA_CUDA(cudaMemcpyAsync(&rc, c->round.counters(), sizeof(Counters), cudaMemcpyDeviceToHost,
+                              s));
+  NGIA_CUDA(cudaStreamSynchronize(s));
+  if (small) ne = c->h_counters->edges;
   c->n_edges = ne;
   if (h_n_edges) *h_n_edges = ne;
   if (st) {
-    Counters rc;
-    NGIA_CUDA(cudaMemcpy(&rc, c->round.counters(), sizeof(Counters), cudaMemcpyDeviceToHost));
     st->candidate_pairs = hc.cand_total;
     st->unique_pairs = m;
     st->aligned_cells = rc.cells;
@@ -660,6 +677,8 @@ void ngia_ctx_destroy(ngia_ctx *c) {
     if (c->ev[k]) cudaEventDestroy(c->ev[k]);
   if (c->h_flag) cudaFreeHost(c->h_flag);
   c->h_flag = nullptr;
+  if (c->h_counters) cudaFreeHost(c->h_counters);
+  c->h_counters = nullptr;
   if (c->bucket_exec) cudaGraphExecDestroy(c->bucket_exec);
   c->bucket_exec = nullptr;
   if (c->side) cudaStreamDestroy(c->side);

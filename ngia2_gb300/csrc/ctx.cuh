@@ -11,6 +11,11 @@ struct ngia_ctx {
   // 8-10 sketch and bucket timing
   static constexpr int kEvents = 11;
   cudaEvent_t ev[kEvents] = {};
+  // pinned: a graph build's counters (candidates, round) and edge count
+  struct HostCounters {
+    ngia::Counters pairs, round;
+    uint64_t edges;
+  } *h_counters = nullptr;
   uint32_t *h_flag = nullptr;  // pinned: a pipelined load's check, read after the step
   cudaStream_t side = nullptr;  // work that runs beside the main stream's (sketch)
   // pipelined loads (ngia_ctx_run_host): chunks of the records copied on `copy`

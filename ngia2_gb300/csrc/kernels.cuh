@@ -45,6 +45,8 @@ int exclusive_scan_u64(const uint32_t *in, uint64_t *out, uint32_t n,
                        uint64_t *d_total, void *scratch, cudaStream_t s);
 
 // bucket.cu
+// Up to kSmallBucket records a band is sorted by one block, without scratch.
+constexpr uint32_t kSmallBucket = 4096;
 size_t bucket_scratch_bytes(uint32_t n, uint32_t bands);
 int bucket(const uint32_t *sigs, uint32_t n, uint32_t bands, uint32_t *rep,
            void *scratch, cudaStream_t s);
@@ -144,6 +146,14 @@ int collect_write(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
              const ClassPlan &plan, uint32_t widest, uint32_t *cls, unsigned int *class_count,
              unsigned long long *cells, uint32_t *bounds, cudaStream_t s);
+// The whole binning of a round of at most kSmallRound pairs in one launch: the
+// queue order, the class bounds and band cells, cursors and computed blocks
+// zeroed, scores zeroed.
+constexpr uint32_t kSmallRound = 8192;
+int bin_small(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
+              const ClassPlan &plan, uint32_t widest, uint32_t *order, uint32_t *bounds,
+              unsigned int *cursors, unsigned long long *cells, unsigned long long *work,
+              uint32_t *scores, cudaStream_t s);
 int bits_for(uint32_t max_value);
 // The part-th of `parts` contiguous ranges [h_cut[0], h_cut[1]) of the pairs,
 // cut so that each holds about 1/parts of their band blocks (the first pair
@@ -157,6 +167,11 @@ size_t emit_scratch_bytes(uint32_t count, uint32_t n_nodes);
 int emit_sorted(const uint2 *pairs, const uint32_t *scores, uint32_t count,
                 uint32_t n_nodes, ngia_edge *out, uint64_t *h_m, void *scratch,
                 cudaStream_t s);
+// The same for at most kSmallEmit pairs in one launch and without a wait: the
+// edge count lands in *d_m.
+constexpr uint32_t kSmallEmit = 4096;
+int emit_small(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
+               uint64_t *d_m, cudaStream_t s);
 // Fast mode's bands [b0, b1): first_band[target] = min of itself and the first
 // of those bands that names the rep of a pair scoring > 0.
 int fast_first_band(const uint32_t *rep, uint32_t n, uint32_t b0, uint32_t b1,

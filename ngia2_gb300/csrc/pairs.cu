@@ -14,6 +14,7 @@
 // and l+32; equal reps are found with match_any, and the first band of every
 // distinct rep keeps it.  Pairs come out grouped by target in index order.
 #include "align.cuh"
+#include "block_sort.cuh"
 #include "kernels.cuh"
 
 namespace ngia {
@@ -266,6 +267,14 @@ int collect_write(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_
   return NGIA_OK;
 }
 
+// The warp's sum (64-bit shared-memory atomics are compare-and-swap loops: a
+// thread each costs a block more than its pairs' arithmetic).
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  return v;
+}
+
 // ---- width classes ------------------------------------------------------------------
 constexpr uint32_t kClassifyUnroll = 4;
 
@@ -319,7 +328,8 @@ classify_kernel(const uint32_t *__restrict__ lens, const uint2 *__restrict__ pai
       if (c != kFull && (peers & lt_mask) == 0) atomicAdd(&sc[c], (unsigned int)__popc(peers));
     }
   }
-  atomicAdd(&scells, my_cells);
+  my_cells = warp_sum(my_cells);
+  if ((threadIdx.x & 31u) == 0 && my_cells) atomicAdd(&scells, my_cells);
   __syncthreads();
   if (threadIdx.x < kNumRoundClasses && sc[threadIdx.x]) atomicAdd(&class_count[threadIdx.x], sc[threadIdx.x]);
   if (threadIdx.x == 0 && scells) atomicAdd(cells, scells * 1024ull);
@@ -354,6 +364,93 @@ int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t 
     NGIA_LAUNCHED();
   }
   class_bounds_kernel<<<1, 32, 0, s>>>(class_count, bounds);
+  NGIA_LAUNCHED();
+  return NGIA_OK;
+}
+
+// Small rounds: one block bins the pairs.  The general path is eight launches
+// (counters and scores cleared, keys, one radix pass, bounds), each a few
+// microseconds whatever the count; here the keys stay in shared memory, their
+// histogram and its scan give every class and octave its run of the queue, and
+// pairs take their places in it by atomics (the order inside a key is free).
+__global__ void __launch_bounds__(1024)
+bin_small_kernel(const uint32_t *__restrict__ lens, const uint2 *__restrict__ pairs,
+                 uint32_t count, float t, int fma_mode, ClassPlan plan, uint32_t widest,
+                 uint32_t *__restrict__ order, uint32_t *__restrict__ bounds,
+                 unsigned int *__restrict__ cursors, unsigned long long *__restrict__ cells,
+                 unsigned long long *__restrict__ work, uint32_t *__restrict__ scores) {
+  __shared__ uint8_t keys[kSmallRound];
+  __shared__ uint32_t hist[256], wsum[8];
+  __shared__ unsigned long long scells;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  if (tid < 256) hist[tid] = 0;
+  if (tid == 0) scells = 0;
+  __syncthreads();
+  unsigned long long my_cells = 0;
+  for (uint32_t p0 = 0; p0 < count; p0 += 1024) {  // block-uniform
+    const uint32_t p = p0 + tid;
+    uint32_t key = kFull;
+    if (p < count) {
+      const uint2 pr = pairs[p];
+      key = skip_sort_key();
+      if (pr.x != kFull) {  // (an empty pair slot is never aligned)
+        const Band b = make_band(__ldg(lens + pr.x), __ldg(lens + pr.y), t, fma_mode);
+        key = class_sort_key(round_class(b, plan, widest), b);
+        my_cells += band_blocks(b);
+      }
+      keys[p] = (uint8_t)key;
+      scores[p] = 0;
+    }
+    const uint32_t peers = __match_any_sync(kFull, key);
+    if (key != kFull && (peers & lt_mask) == 0) atomicAdd(&hist[key], (uint32_t)__popc(peers));
+  }
+  my_cells = warp_sum(my_cells);
+  if (lane == 0 && my_cells) atomicAdd(&scells, my_cells);
+  __syncthreads();
+  uint32_t v = 0, x = 0;
+  if (tid < 256) {
+    x = v = hist[tid];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) wsum[tid >> 5] = x;
+  }
+  __syncthreads();
+  if (tid < 256) {
+    for (uint32_t w = 0; w < tid >> 5; ++w) x += wsum[w];
+    hist[tid] = x - v;
+    if ((tid & 7u) == 0 && tid / 8 <= (uint32_t)kNumRoundClasses) bounds[tid / 8] = x - v;
+    if (tid == 255 && kNumRoundClasses == 32) bounds[32] = x;
+  }
+  if (tid < kNumRoundClasses) cursors[tid] = 0;
+  if (tid == 0) {
+    *cells = scells * 1024ull;
+    *work = 0;
+  }
+  __syncthreads();
+  for (uint32_t p0 = 0; p0 < count; p0 += 1024) {
+    const uint32_t p = p0 + tid;
+    const uint32_t key = p < count ? keys[p] : kFull;
+    const uint32_t peers = __match_any_sync(kFull, key);
+    const uint32_t leader = __ffs(peers) - 1;
+    uint32_t first = 0;
+    if (lane == leader && key != kFull) first = atomicAdd(&hist[key], (uint32_t)__popc(peers));
+    first = __shfl_sync(kFull, first, leader);
+    if (key != kFull) order[first + __popc(peers & lt_mask)] = p;
+  }
+}
+
+int bin_small(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
+              const ClassPlan &plan, uint32_t widest, uint32_t *order, uint32_t *bounds,
+              unsigned int *cursors, unsigned long long *cells, unsigned long long *work,
+              uint32_t *scores, cudaStream_t s) {
+  if (count > kSmallRound) return NGIA_ERR_ARG;
+  bin_small_kernel<<<1, 1024, 0, s>>>(lens, pairs, count, identity_threshold(identity),
+                                      round_mode(), plan, widest, order, bounds, cursors, cells,
+                                      work, scores);
   NGIA_LAUNCHED();
   return NGIA_OK;
 }
@@ -611,6 +708,42 @@ int emit_sorted(const uint2 *pairs, const uint32_t *scores, uint32_t count,
                             bits > 0 ? bits : 8, sort_scratch, s));
   gather_edges_kernel<<<ceil_div((uint32_t)m, 256u), 256, 0, s>>>(srep, sidx, etar, escore,
                                                                   (uint32_t)m, out);
+  NGIA_LAUNCHED();
+  return NGIA_OK;
+}
+
+// Few pairs: one block gathers the hits as (rep, pair) keys, sorts them in
+// shared memory (a pair's place is its target's, so the order is (rep, tar)) and
+// writes the edges.  The general path is three compaction launches, a wait for
+// the count and three launches per radix pass of the rep.
+__global__ void __launch_bounds__(1024)
+emit_small_kernel(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ scores,
+                  uint32_t count, ngia_edge *__restrict__ out, uint64_t *__restrict__ d_m) {
+  __shared__ uint64_t keys[kSmallEmit];
+  __shared__ uint32_t hits;
+  const uint32_t tid = threadIdx.x;
+  if (tid == 0) hits = 0;
+  __syncthreads();
+  for (uint32_t p = tid; p < count; p += 1024)
+    if (scores[p] > 0) keys[atomicAdd(&hits, 1u)] = (uint64_t)pairs[p].x << 32 | p;
+  __syncthreads();
+  const uint32_t m = hits;
+  block_sort(keys, m);
+  for (uint32_t k = tid; k < m; k += 1024) {
+    const uint32_t p = (uint32_t)keys[k];
+    ngia_edge ed;
+    ed.rep = (int32_t)(keys[k] >> 32);
+    ed.tar = (int32_t)pairs[p].y;
+    ed.weight = __fdiv_rn(__uint2float_rn(scores[p]), 100.0f);
+    out[k] = ed;
+  }
+  if (tid == 0) *d_m = m;
+}
+
+int emit_small(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
+               uint64_t *d_m, cudaStream_t s) {
+  if (count > kSmallEmit) return NGIA_ERR_ARG;
+  emit_small_kernel<<<1, 1024, 0, s>>>(pairs, scores, count, out, d_m);
   NGIA_LAUNCHED();
   return NGIA_OK;
 }

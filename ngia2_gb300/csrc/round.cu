@@ -127,17 +127,6 @@ int Round::enqueue(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t id
                    uint32_t *scores, cudaEvent_t ev_mid) {
   cudaStream_t s = stream;
   Counters *dc = counters();
-  NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
-  NGIA_TRY(classify(db.lens, pairs, m, identity, plan, widest_window(db.ab.K),
-                    cls_.as<uint32_t>(), dc->class_count, &dc->cells, dc->bounds, s));
-  NGIA_TRY(radix_sort_pairs(cls_.as<uint32_t>(), nullptr, cls_sorted_.as<uint32_t>(),
-                            order_.as<uint32_t>(), m, 1, 0, kClassKeyBits, sort_tmp_.p, s));
-  NGIA_CUDA(cudaMemsetAsync(scores, 0, (size_t)(m ? m : 1) * 4, s));
-  if (ev_mid) NGIA_CUDA(cudaEventRecord(ev_mid, s));
-  if (m == 0) return NGIA_OK;
-  // the kernels as concurrent branches, widest classes first: the few long
-  // pairs' warps leave most of the device to the others instead of running
-  // alone at the end
   const RoundArgs args{db.ab.K < 16 ? db.ab.dplanes : db.packed,
                        db.packed,
                        db.nib,
@@ -152,6 +141,28 @@ int Round::enqueue(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t id
                        round_mode(),
                        &dc->work};
   if (!args.rows) return NGIA_ERR_STATE;
+  if (m > 0 && m <= kSmallRound) {
+    // no window over 16 words: few pairs leave the device mostly idle, and a
+    // wide pair's columns end sooner on a group of lanes (align, proteins at
+    // identity 50, windows up to 24 / 16 / 12 words: 409 pairs 92 / 61 / 57 us,
+    // 1,176: 96 / 65 / 62, 2,957: 98 / 94 / 96, 7,800: 119 / 113 / 123)
+    NGIA_TRY(bin_small(db.lens, pairs, m, identity, plan, 16u,
+                       order_.as<uint32_t>(), dc->bounds, dc->cursor, &dc->cells, &dc->work,
+                       scores, s));
+    if (ev_mid) NGIA_CUDA(cudaEventRecord(ev_mid, s));
+  } else {
+    NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
+    NGIA_TRY(classify(db.lens, pairs, m, identity, plan, widest_window(db.ab.K),
+                      cls_.as<uint32_t>(), dc->class_count, &dc->cells, dc->bounds, s));
+    NGIA_TRY(radix_sort_pairs(cls_.as<uint32_t>(), nullptr, cls_sorted_.as<uint32_t>(),
+                              order_.as<uint32_t>(), m, 1, 0, kClassKeyBits, sort_tmp_.p, s));
+    NGIA_CUDA(cudaMemsetAsync(scores, 0, (size_t)(m ? m : 1) * 4, s));
+    if (ev_mid) NGIA_CUDA(cudaEventRecord(ev_mid, s));
+    if (m == 0) return NGIA_OK;
+  }
+  // the kernels as concurrent branches, widest classes first: the few long
+  // pairs' warps leave most of the device to the others instead of running
+  // alone at the end
   NGIA_CUDA(cudaEventRecord(fork_, s));
   for (int k = 0; k < kSide; ++k) NGIA_CUDA(cudaStreamWaitEvent(side_[k], fork_, 0));
   static_assert(kAlignKernels == kSide + 1, "one branch per kernel");

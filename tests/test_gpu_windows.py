@@ -111,7 +111,9 @@ def test_windows_match_oracle(cuda, built, alphabet, identity):
     assert (want > 0).any() and (want == 0).any()
     with ng.Context() as ctx:
         ctx.load(packed, offs, lens)
-        got, _ = ctx.align_pairs(pairs, identity)
-    bad = np.flatnonzero(got != want)
-    assert len(bad) == 0, [(int(lens[pairs[i, 0]]), int(lens[pairs[i, 1]]), int(got[i]),
-                            int(want[i])) for i in bad[:8]]
+        for repeat in (1, 7):  # a round of few pairs, and of more than 8,192
+            many = np.tile(pairs, (repeat, 1))
+            got, _ = ctx.align_pairs(many, identity)
+            bad = np.flatnonzero(got != np.tile(want, repeat))
+            assert len(bad) == 0, [(int(lens[many[i, 0]]), int(lens[many[i, 1]]), int(got[i]),
+                                    int(want[i % len(want)])) for i in bad[:8]]
