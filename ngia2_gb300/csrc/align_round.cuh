@@ -57,34 +57,34 @@ __device__ __forceinline__ uint32_t group_class(const RoundArgs &a, uint32_t *sm
                                      a.bounds[C + 1], a.cursors + C, a.scores, a.t, a.fm, smem);
 }
 
-// The widest bands: (32,16) and the general class.
+// The classes of 32 lanes, widest first, and the general class: few and long
+// pairs, at most seven warps of them per multiprocessor, so that a pair of
+// 30,000 residues does not share its scheduler with three others and end the
+// round alone (2 million heavy-tailed pairs after the seed filter: 6.3 ms in
+// one kernel with the classes of 8 and 16 lanes at 14 warps, 4.7 ms here).
 template <int KC>
-__global__ void __launch_bounds__(kGroupThreads)
+__global__ void __launch_bounds__(32)
 align_wide_kernel(const __grid_constant__ RoundArgs a) {
   extern __shared__ uint32_t smem[];
-  uint32_t *mine = smem + (threadIdx.x >> 5) * (KC * 16 * 32);
   uint32_t done = align_general(a, kGeneralClass);
-  done += group_class<kFirstGroupClass + 7, KC>(a, mine);
+  done += group_class<kFirstGroupClass + 7, KC>(a, smem);
+  done += group_class<kFirstGroupClass + 6, KC>(a, smem);
+  done += group_class<kFirstGroupClass + 5, KC>(a, smem);
+  done += group_class<kFirstGroupClass + 4, KC>(a, smem);
   count_work(done, a.work);
 }
 
-// The group classes of at most eight words per lane, widest first.
-template <int KC>
-__device__ __forceinline__ uint32_t group_classes(const RoundArgs &a, uint32_t *smem) {
-  uint32_t done = group_class<kFirstGroupClass + 6, KC>(a, smem);
-  done += group_class<kFirstGroupClass + 5, KC>(a, smem);
-  done += group_class<kFirstGroupClass + 4, KC>(a, smem);
-  done += group_class<kFirstGroupClass + 3, KC>(a, smem);
-  done += group_class<kFirstGroupClass + 2, KC>(a, smem);
-  done += group_class<kFirstGroupClass + 1, KC>(a, smem);
-  return done + group_class<kFirstGroupClass, KC>(a, smem);
-}
-
+// The classes of 16 and 8 lanes, widest first.
 template <int KC>
 __global__ void __launch_bounds__(kGroupThreads)
 align_group_kernel(const __grid_constant__ RoundArgs a) {
   extern __shared__ uint32_t smem[];
-  count_work(group_classes<KC>(a, smem + (threadIdx.x >> 5) * (KC * 8 * 32)), a.work);
+  uint32_t *mine = smem + (threadIdx.x >> 5) * (KC * 6 * 32);
+  uint32_t done = group_class<kFirstGroupClass + 3, KC>(a, mine);
+  done += group_class<kFirstGroupClass + 2, KC>(a, mine);
+  done += group_class<kFirstGroupClass + 1, KC>(a, mine);
+  done += group_class<kFirstGroupClass, KC>(a, mine);
+  count_work(done, a.work);
 }
 
 // The one-pair-per-lane classes in three kernels by width (tier 0: windows of
@@ -190,10 +190,9 @@ int launch_align_k(int kernel, const RoundArgs &a, uint32_t m, cudaStream_t s) {
   constexpr auto slots = [](int tier) { return (size_t)K * window_slots(K, tier) * 32 * 4; };
   switch (kernel) {
     case 0:
-      return launch_round(align_wide_kernel<KC>, kGroupThreads, group_smem_bytes(16, KC), warps,
-                          a, s);
+      return launch_round(align_wide_kernel<KC>, 32, (size_t)KC * 16 * 32 * 4, m, a, s);
     case 1:
-      return launch_round(align_group_kernel<KC>, kGroupThreads, group_smem_bytes(8, KC), warps,
+      return launch_round(align_group_kernel<KC>, kGroupThreads, group_smem_bytes(6, KC), warps,
                           a, s);
     case 2: return launch_round(align_window_kernel<K, 2>, 32, slots(2), lanes, a, s);
     case 3: return launch_round(align_window_kernel<K, 1>, 32, slots(1), lanes, a, s);

@@ -139,13 +139,21 @@ int collect_write(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_
                   uint32_t identity, const uint64_t *offsets, uint2 *pairs,
                   cudaStream_t s);
 // Width class sort keys of `count` pairs, per-class counts (added to
-// class_count), band cells (added to *cells) and the class bounds of the
-// class-major order (bounds[c] = pairs in classes below c; kNumRoundClasses +
-// 1 entries, written after the counts are complete).  widest: the widest
-// sliding window to use (widest_window).
+// class_count) and band cells (added to *cells).  widest: the widest sliding
+// window to use (widest_window).
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
              const ClassPlan &plan, uint32_t widest, uint32_t *cls, unsigned int *class_count,
-             unsigned long long *cells, uint32_t *bounds, cudaStream_t s);
+             unsigned long long *cells, cudaStream_t s);
+// bounds[c] = pairs in classes below c (kNumRoundClasses + 1 entries).
+int class_bounds(const unsigned int *class_count, uint32_t *bounds, cudaStream_t s);
+// seed_filter.cu
+// Moves the pairs whose score is certainly 0, by the words their sequences
+// share, from their class (cls, class_count) to the skip class; between
+// classify and class_bounds.  K: the alphabet's table entries; *cursor zero
+// before the call.
+int seed_filter(const uint32_t *nib, int K, const uint64_t *offs, const uint32_t *lens,
+                const uint2 *pairs, uint32_t m, uint32_t identity, uint32_t *cls,
+                unsigned int *class_count, unsigned int *cursor, cudaStream_t s);
 // The whole binning of a round of at most kSmallRound pairs in one launch: the
 // queue order, the class bounds and band cells, cursors and computed blocks
 // zeroed, scores zeroed.

@@ -352,7 +352,7 @@ __global__ void class_bounds_kernel(const unsigned int *__restrict__ class_count
 
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
              const ClassPlan &plan, uint32_t widest, uint32_t *cls, unsigned int *class_count,
-             unsigned long long *cells, uint32_t *bounds, cudaStream_t s) {
+             unsigned long long *cells, cudaStream_t s) {
   if (count > 0) {
     int dev = 0, sms = 0;
     NGIA_CUDA(cudaGetDevice(&dev));
@@ -363,6 +363,10 @@ int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t 
         class_count, cells);
     NGIA_LAUNCHED();
   }
+  return NGIA_OK;
+}
+
+int class_bounds(const unsigned int *class_count, uint32_t *bounds, cudaStream_t s) {
   class_bounds_kernel<<<1, 32, 0, s>>>(class_count, bounds);
   NGIA_LAUNCHED();
   return NGIA_OK;

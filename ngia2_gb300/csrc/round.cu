@@ -153,7 +153,10 @@ int Round::enqueue(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t id
   } else {
     NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
     NGIA_TRY(classify(db.lens, pairs, m, identity, plan, widest_window(db.ab.K),
-                      cls_.as<uint32_t>(), dc->class_count, &dc->cells, dc->bounds, s));
+                      cls_.as<uint32_t>(), dc->class_count, &dc->cells, s));
+    NGIA_TRY(seed_filter(db.nib, db.ab.K, db.offs, db.lens, pairs, m, identity,
+                         cls_.as<uint32_t>(), dc->class_count, &dc->seed_cursor, s));
+    NGIA_TRY(class_bounds(dc->class_count, dc->bounds, s));
     NGIA_TRY(radix_sort_pairs(cls_.as<uint32_t>(), nullptr, cls_sorted_.as<uint32_t>(),
                               order_.as<uint32_t>(), m, 1, 0, kClassKeyBits, sort_tmp_.p, s));
     NGIA_CUDA(cudaMemsetAsync(scores, 0, (size_t)(m ? m : 1) * 4, s));
