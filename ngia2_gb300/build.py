@@ -22,7 +22,7 @@ LIBDIR = PKG / "lib"
 OBJDIR = ROOT / "_build" / "ngia"
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["align_k16.cu", "align_k8.cu", "align_k5.cu", "sketch.cu", "sort.cu", "bucket.cu",
+CU_SOURCES = ["align_k16.cu", "align_k8.cu", "align_k5.cu", "align_jobs.cu", "sketch.cu", "sort.cu", "bucket.cu",
               "align.cu", "pairs.cu", "edges.cu", "ctx.cu", "round.cu", "serve.cu", "stream.cu",
               "seed_filter.cu", "pack.cu", "probe.cu"]
 CPP_SOURCES = ["packed_io.cpp", "leiden.cpp", "cluster.cpp", "device_session.cpp"]

@@ -1,69 +1,17 @@
-// align.cu -- alignment kernels: the drop-in job-triple kernel and the
-// length-binned batched kernels.
+// align.cu -- the load-time layouts of the aligner's records, and the batched
+// round's launches.
 #include <mutex>
 #include <vector>
 
 #include "align.cuh"
+#include "align_lds.cuh"
 #include "kernels.cuh"
 
 namespace ngia {
 
-// One thread per job, in job order: the drop-in for the reference's
-// one-launch-per-band kernel_dynamic<<<ceil(count/64), 64>>> (launch at
-// src/buildGraph.hpp:323).  The window width is picked per pair at run time.
-__device__ __forceinline__ uint32_t lcs_any(const uint32_t *rep, const uint32_t *tar,
-                                            const Band &b, uint32_t *lines) {
-  uint32_t blocks;
-  if (b.width <= 4) return lcs_window<4>(rep, tar, b, blocks);
-  if (b.width <= 8) return lcs_window<8>(rep, tar, b, blocks);
-  if (b.width <= 16) return lcs_window<16>(rep, tar, b, blocks);
-  return lcs_general(rep, tar, b, lines, blocks);
-}
-
-__global__ void __launch_bounds__(128)
-align_jobs_kernel(const uint32_t *__restrict__ packed,
-                  const uint64_t *__restrict__ offs, uint32_t *__restrict__ jobs,
-                  uint32_t count, float t, int fma_mode) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= count) return;
-  const uint32_t *rep = packed + offs[jobs[3 * j]];
-  const uint32_t *tar = packed + offs[jobs[3 * j + 1]];
-  const uint32_t lr = __ldg(rep), lt = __ldg(tar);
-  const Band b = make_band(lr, lt, t, fma_mode);
-  if (!b.pass) return;  // the reference leaves the score word as it was
-  uint32_t lines[kMaxRowBlocks];
-  const uint32_t lcs = lcs_any(rep, tar, b, lines);
-  jobs[3 * j + 2] = identity_score(lcs, lr, lt, t);
-}
-
 // Load-time layout kernels: one warp per record, lane k taking the record's
 // 32-residue blocks k, k + 32, ... (four words each, coalesced across the
 // warp); bit work by shifts and masks, no per-residue loops.
-
-// bits 0..7 of b to bits 0, 4, ..., 28
-__device__ __forceinline__ uint32_t spread8(uint32_t b) {
-  b = (b | (b << 12)) & 0x000F000Fu;
-  b = (b | (b << 6)) & 0x03030303u;
-  return (b | (b << 3)) & 0x11111111u;
-}
-
-// Four plane words of a block (bit r of plane e = bit e of the code of
-// residue r) -> its four nibble words (word q: residues 8q..8q+7, the first in
-// the high nibble).
-__device__ __forceinline__ void planes_to_nibbles(const uint32_t (&pl)[4], int np,
-                                                  uint32_t (&out)[4]) {
-  uint32_t rv[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) rv[e] = e < np ? __brev(pl[e]) : 0u;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    uint32_t w = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (e < np) w |= spread8((rv[e] >> (24 - 8 * q)) & 0xFFu) << e;
-    out[q] = w;
-  }
-}
 
 // mask of the residues of a block whose code is c, from its four planes
 __device__ __forceinline__ uint32_t code_mask(const uint32_t (&pl)[4], uint32_t c) {
@@ -350,23 +298,4 @@ int launch_align(int kernel, const RoundArgs &a, int K, uint32_t m, cudaStream_t
                   : launch_align_k<16>(kernel, a, m, s);
 }
 
-int launch_align_jobs(const uint32_t *packed, const uint64_t *offs, uint32_t *jobs,
-                      uint32_t count, uint32_t identity, cudaStream_t s) {
-  if (count == 0) return NGIA_OK;
-  align_jobs_kernel<<<ceil_div(count, 128u), 128, 0, s>>>(
-      packed, offs, jobs, count, identity_threshold(identity), round_mode());
-  NGIA_LAUNCHED();
-  return NGIA_OK;
-}
-
 }  // namespace ngia
-
-extern "C" int ngia_align_pairs(const uint32_t *d_packed, const uint64_t *d_rec_offsets,
-                                uint32_t *d_jobs, uint32_t count, uint32_t identity,
-                                void *stream) {
-  if (identity < 1 || identity > 99) return NGIA_ERR_ARG;
-  if (count == 0) return NGIA_OK;
-  if (!d_packed || !d_rec_offsets || !d_jobs) return NGIA_ERR_ARG;
-  return ngia::launch_align_jobs(d_packed, d_rec_offsets, d_jobs, count, identity,
-                                 ngia::as_stream(stream));
-}

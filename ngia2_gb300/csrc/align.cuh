@@ -15,16 +15,14 @@
 // word at once, which is the same set of dependencies evaluated in another
 // order, and the word-to-word carry is the hardware carry flag.
 //
-// Window form (lcs_window<W>).  Live row blocks [J0(I), J1(I)) never exceed
-// min(ls + rs, nr) words and both ends advance by at most one block per
-// column block, so the live rows sit in a register window V[0..W) based at
-// J0: when J0 advances, V[0] retires into the LCS sum and the window shifts
-// down; a row block entering at J1 gets its four bit planes loaded.  Window
-// slots above J1 hold all-ones with zero planes: zero planes mean code 0,
-// which matches nothing, so those words stay all-ones and only pass the carry
-// through -- exactly the "not yet visited" state of the reference.
+// The live row blocks are at most min(ls + rs, nr) words and both ends advance
+// by at most one block per column block.  A row block above them is all ones
+// with empty masks -- the "not yet visited" state of the reference -- and only
+// passes a carry; one below is frozen.  The batched and drop-in kernels hold
+// them in registers (align_window.cuh) or over a group of lanes
+// (align_group.cuh); the general form below holds any number in local memory.
 //
-// Match masks are computed from the bit planes with no lookup table:
+// The general form computes match masks from the bit planes:
 //   u = (P0 & T0) | (~P0 & B);  u &= ~(Pe ^ Te) for e = 1..3;  t = V & u
 // where Te = all-ones if bit e of the column code is set, B = ~T0 & (T1|T2|T3)
 // (so a zero column code gives u = 0).  Since t = V & M is a subset of V,
@@ -35,42 +33,6 @@
 #include "common.cuh"
 
 namespace ngia {
-
-// One chunk of C words of a multi-word add (carry in when CIN, carry out when
-// COUT), dispatched to the PTX chains.
-template <int C, bool CIN, bool COUT>
-__device__ __forceinline__ void add_chunk(uint32_t *s, const uint32_t *a, const uint32_t *b,
-                                          uint32_t cin, uint32_t &cout) {
-#define NGIA_CHUNK(N)                                              \
-  if constexpr (C == N) {                                          \
-    if constexpr (CIN && COUT) add_chain##N##_cc(s, a, b, cin, cout); \
-    else if constexpr (CIN) add_chain##N##_cn(s, a, b, cin);       \
-    else if constexpr (COUT) add_chain##N##_zc(s, a, b, cout);     \
-    else add_chain##N##_zn(s, a, b);                               \
-  }
-  NGIA_CHUNK(2)
-  NGIA_CHUNK(4)
-  NGIA_CHUNK(8)
-#undef NGIA_CHUNK
-}
-
-// s[0..W) = a + b as one W-word number (carry in = cin != 0 when CIN; W even
-// when CIN or W > 16).
-template <int W, bool CIN>
-__device__ __forceinline__ void add_words(uint32_t *s, const uint32_t *a,
-                                          const uint32_t *b, uint32_t cin) {
-  constexpr int C = W >= 8 ? 8 : (W >= 4 ? 4 : 2);
-  uint32_t c = 0;
-  if constexpr (!CIN && W <= 16) {
-    add_run<W>(s, a, b);
-  } else if constexpr (W == C) {
-    static_assert(W % 2 == 0, "window width must be even");
-    add_chunk<C, CIN, false>(s, a, b, cin, c);
-  } else {
-    add_chunk<C, CIN, true>(s, a, b, cin, c);
-    add_words<W - C, true>(s + C, a + C, b + C, c);
-  }
-}
 
 // Column-code masks of a target block, one column per step.  The four planes
 // are bit-reversed once per block so that column k's bits sit in bit 31 after
@@ -112,82 +74,6 @@ __device__ __forceinline__ uint32_t match_and(uint32_t v, uint32_t p0, uint32_t 
   u &= ~(p2 ^ c.T2);
   u &= ~(p3 ^ c.T3);
   return v & u;
-}
-
-template <int W>
-__device__ __forceinline__ void window_step(uint32_t (&V)[W], const uint32_t (&P0)[W],
-                                            const uint32_t (&P1)[W],
-                                            const uint32_t (&P2)[W],
-                                            const uint32_t (&P3)[W],
-                                            const ColMask &c) {
-  uint32_t t[W], s[W];
-#pragma unroll
-  for (int m = 0; m < W; ++m) t[m] = match_and(V[m], P0[m], P1[m], P2[m], P3[m], c);
-  add_words<W, false>(s, V, t, 0);
-#pragma unroll
-  for (int m = 0; m < W; ++m) V[m] = s[m] | (V[m] ^ t[m]);
-}
-
-// LCS of the banded computation, window form; requires b.width <= W.
-template <int W>
-// `blocks` receives the column blocks processed (fewer than b.nc after an
-// early exit).
-__device__ inline uint32_t lcs_window(const uint32_t *__restrict__ rep,
-                                      const uint32_t *__restrict__ tar, const Band &b,
-                                      uint32_t &blocks) {
-  uint32_t V[W], P0[W], P1[W], P2[W], P3[W];
-#pragma unroll
-  for (int m = 0; m < W; ++m) {
-    V[m] = kFull;
-    P0[m] = P1[m] = P2[m] = P3[m] = 0;
-  }
-  uint32_t lcs = 0, act = 0;  // act = row blocks loaded so far
-  for (uint32_t i = 0; i < b.nc; ++i) {
-    if (i > b.ls) {  // J0 advances: retire the bottom row block
-      lcs += __popc(~V[0]);
-#pragma unroll
-      for (int m = 0; m < W - 1; ++m) {
-        V[m] = V[m + 1];
-        P0[m] = P0[m + 1];
-        P1[m] = P1[m + 1];
-        P2[m] = P2[m + 1];
-        P3[m] = P3[m + 1];
-      }
-      V[W - 1] = kFull;
-      P0[W - 1] = P1[W - 1] = P2[W - 1] = P3[W - 1] = 0;
-    }
-    const uint32_t j0 = i > b.ls ? i - b.ls : 0;
-    const uint32_t j1 = (i + b.rs < b.nr) ? i + b.rs : b.nr;
-    for (; act < j1; ++act) {  // row blocks entering the band
-      const uint32_t *rb = rep + 1 + 4 * act;
-      const uint32_t q0 = __ldg(rb), q1 = __ldg(rb + 1), q2 = __ldg(rb + 2),
-                     q3 = __ldg(rb + 3);
-      const uint32_t slot = act - j0;
-#pragma unroll
-      for (int m = 0; m < W; ++m) {
-        if ((uint32_t)m == slot) {
-          P0[m] = q0;
-          P1[m] = q1;
-          P2[m] = q2;
-          P3[m] = q3;
-        }
-      }
-    }
-    ColumnPlanes col(tar + 1 + 4 * i);
-#pragma unroll 4
-    for (int k = 0; k < 32; ++k) window_step<W>(V, P0, P1, P2, P3, col.next());
-    uint32_t z = lcs;
-#pragma unroll
-    for (int m = 0; m < W; ++m) z += __popc(~V[m]);
-    if (!may_reach_threshold(z, 32 * (i + 1), b)) {  // score 0 already certain
-      blocks = i + 1;
-      return 0;
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < W; ++m) lcs += __popc(~V[m]);
-  blocks = b.nc;
-  return lcs;
 }
 
 // General form for any band width: per column block the live rows are
@@ -309,10 +195,16 @@ __host__ __device__ constexpr int fixed_width(int k) {
   return k < 5 ? 8 + 2 * k : k == 5 ? 20 : 24;
 }
 
-// The widest sliding window for tables of K entries per row word: 28 words of
-// 16 entries would leave a streaming multiprocessor's shared memory to three
-// warps (align_window.cuh).
-__host__ __device__ constexpr uint32_t widest_window(int K) { return K > 8 ? 24u : 28u; }
+constexpr uint32_t kWidestWindow = 28;
+
+// The widest sliding window for tables of K entries per row word: a 28-word
+// window of 16-entry tables would leave a multiprocessor's shared memory to
+// three warps, which is no faster than the groups (1,000,003 proteins at
+// identity 50, align: 9.24 ms with, 9.26 without it; 2 million heavy-tailed
+// pairs: 6.7 and 6.0).
+__host__ __device__ constexpr uint32_t widest_window(int K) {
+  return K > 8 ? 24u : kWidestWindow;
+}
 
 // Window a streaming kernel needs for a pair: the live rows of block i,
 // [max(i - ls, 0), min(i + rs, nr)), inside [i - ls, i - ls + W).
@@ -396,7 +288,7 @@ __host__ __device__ inline int round_class(const Band &b, const ClassPlan &plan,
 
 // Queue order inside a class: longest targets first.  The sort key of a pair
 // is class-major, then 7 - floor(log2 nc) (column blocks in octaves, capped
-// at 7), one 8-bit radix pass.
+// at 7), in eight bits.
 __host__ __device__ inline uint32_t class_sort_key(int cls, const Band &b) {
   uint32_t h = 0;
   if (b.nc > 1) {
@@ -410,7 +302,7 @@ __host__ __device__ inline uint32_t class_sort_key(int cls, const Band &b) {
   h >>= 1;
   return ((uint32_t)cls << 3) | (7u - (h < 7u ? h : 7u));
 }
-constexpr int kClassKeyBits = 8;
+constexpr uint32_t kQueueKeys = 256;
 static_assert(kNumRoundClasses <= 32, "class sort key: 5 class bits");
 __host__ __device__ constexpr uint32_t skip_sort_key() { return ((uint32_t)kSkipClass << 3) | 7u; }
 

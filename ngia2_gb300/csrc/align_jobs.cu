@@ -1,0 +1,125 @@
+// align_jobs.cu -- the drop-in job-triple kernel: the reference's
+// one-launch-per-band kernel_dynamic<<<ceil(count/64), 64>>> (launch at
+// src/buildGraph.hpp:323), on the packed records alone and without scratch.
+//
+// A warp takes 32 jobs in job order, one pair per lane, in the windows of the
+// batched aligner (align_window.cuh): the lanes whose pairs fit 4, 8, 12, 16
+// and 24 words (the whole rep, or the sliding band) run together, the rest
+// through the general form.  Match masks come from tables in shared memory, as
+// there; the target's codes are made from its bit planes, block by block.
+//
+// What bounds it at the reference's launch sizes (a band's few thousand jobs):
+// the longest pair of a warp, a serial chain of 32 columns a block.  With the
+// masks computed from the bit planes in every column, 12 ALU operations a word
+// instead of 3, 6,000 jobs of 20,000 proteins at identity 90 took 107 us, with
+// the tables 75 us.
+#include "align_window.cuh"
+#include "kernels.cuh"
+
+namespace ngia {
+
+constexpr int kJobSlots = 27;  // table slots: 24 words and room to slide
+
+// The lanes of the warp with `run` align their pairs; returns the score.
+template <int W, bool kSlide>
+__device__ __forceinline__ void job_window(bool run, const uint32_t *rep, const uint32_t *tar,
+                                           const Band &b, uint32_t *col, uint32_t &score) {
+  if (!__any_sync(kFull, run)) return;
+  const LdsTable<kJobSlots, 16> tab{col};
+  uint32_t V[W];
+#pragma unroll
+  for (int m = 0; m < W; ++m) V[m] = kFull;
+  WindowPair sp{};
+  if (run) {
+    sp.rep = rep;
+    sp.tar = tar + 1;
+    sp.lr = b.lr;
+    sp.lt = b.lt;
+    sp.nc = b.nc;
+    sp.nr = b.nr;
+    sp.rs = b.rs;
+    sp.ls = b.ls;
+    sp.pf_row = kFull;
+    sp.cur = load4(sp.tar);
+    sp.active = true;
+    if constexpr (kSlide) window_start(V, sp);
+  }
+  uint32_t base = 0;
+  while (__any_sync(kFull, sp.active)) {
+    if constexpr (kSlide) window_advance<W>(tab, base);
+    int32_t total = 0, ub = 0;
+    window_block<W, kJobSlots, 16, kSlide, true>(V, sp, tab, base, total, ub);
+    if (sp.active) {
+      const bool last = sp.i >= sp.nc;
+      if (last || !lcs_may_reach((uint32_t)ub, sp.lr, sp.lt, b.t)) {
+        score = last ? identity_score((uint32_t)total, sp.lr, sp.lt, b.t) : 0u;
+        sp.active = false;
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(32)
+align_jobs_kernel(const uint32_t *__restrict__ packed, const uint64_t *__restrict__ offs,
+                  uint32_t *__restrict__ jobs, uint32_t count, float t, int fma_mode) {
+  extern __shared__ uint32_t smem[];
+  uint32_t *col = smem + threadIdx.x;
+#pragma unroll 1
+  for (int s = 0; s < kJobSlots; ++s) col[s * 32] = 0u;  // code 0 matches nothing
+  const uint32_t j = blockIdx.x * 32u + threadIdx.x;
+  const uint32_t *rep = packed, *tar = packed;
+  Band b{};
+  if (j < count) {
+    rep = packed + offs[jobs[3 * (size_t)j]];
+    tar = packed + offs[jobs[3 * (size_t)j + 1]];
+    b = make_band(__ldg(rep), __ldg(tar), t, fma_mode);
+  }
+  const bool mine = j < count && b.pass;  // else the reference leaves the score word as it was
+  const bool empty = b.nc == 0;
+  // the narrower of the sliding window and the whole rep
+  const uint32_t ws = stream_width(b);
+  const bool fixed = b.nr < ws;
+  const uint32_t words = mine && !empty ? (fixed ? b.nr : ws) : 0u;
+  uint32_t score = 0;
+  job_window<4, true>(!fixed && words - 1u < 4u, rep, tar, b, col, score);
+  job_window<8, true>(!fixed && words - 5u < 4u, rep, tar, b, col, score);
+  job_window<12, true>(!fixed && words - 9u < 4u, rep, tar, b, col, score);
+  job_window<16, true>(!fixed && words - 13u < 4u, rep, tar, b, col, score);
+  job_window<24, true>(!fixed && words - 17u < 8u, rep, tar, b, col, score);
+  job_window<8, false>(fixed && words - 1u < 8u, rep, tar, b, col, score);
+  job_window<16, false>(fixed && words - 9u < 8u, rep, tar, b, col, score);
+  job_window<24, false>(fixed && words - 17u < 8u, rep, tar, b, col, score);
+  if (mine && !empty && words > 24) {
+    uint32_t lines[kMaxRowBlocks];
+    uint32_t blocks;
+    score = identity_score(lcs_general(rep, tar, b, lines, blocks), b.lr, b.lt, t);
+  } else if (mine && empty) {
+    score = identity_score(0u, b.lr, b.lt, t);
+  }
+  if (mine) jobs[3 * (size_t)j + 2] = score;
+}
+
+int launch_align_jobs(const uint32_t *packed, const uint64_t *offs, uint32_t *jobs,
+                      uint32_t count, uint32_t identity, cudaStream_t s) {
+  if (count == 0) return NGIA_OK;
+  constexpr size_t smem = (size_t)kJobSlots * 16 * 32 * 4;
+  const void *func = reinterpret_cast<const void *>(align_jobs_kernel);
+  uint32_t grid = 0;  // (sets the kernel's shared memory)
+  NGIA_TRY(persistent_grid(func, 32, smem, kFull, &grid));
+  align_jobs_kernel<<<ceil_div(count, 32u), 32, smem, s>>>(
+      packed, offs, jobs, count, identity_threshold(identity), round_mode());
+  NGIA_LAUNCHED();
+  return NGIA_OK;
+}
+
+}  // namespace ngia
+
+extern "C" int ngia_align_pairs(const uint32_t *d_packed, const uint64_t *d_rec_offsets,
+                                uint32_t *d_jobs, uint32_t count, uint32_t identity,
+                                void *stream) {
+  if (identity < 1 || identity > 99) return NGIA_ERR_ARG;
+  if (count == 0) return NGIA_OK;
+  if (!d_packed || !d_rec_offsets || !d_jobs) return NGIA_ERR_ARG;
+  return ngia::launch_align_jobs(d_packed, d_rec_offsets, d_jobs, count, identity,
+                                 ngia::as_stream(stream));
+}

@@ -58,4 +58,36 @@ __device__ __forceinline__ uint4 load4(const uint32_t *p) {
   return make_uint4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
 }
 
+// bits 0..7 of b to bits 0, 4, ..., 28
+__device__ __forceinline__ uint32_t spread8(uint32_t b) {
+  b = (b | (b << 12)) & 0x000F000Fu;
+  b = (b | (b << 6)) & 0x03030303u;
+  return (b | (b << 3)) & 0x11111111u;
+}
+
+// Four plane words of a block (bit r of plane e = bit e of the code of
+// residue r) -> its four nibble words (word q: residues 8q..8q+7, the first in
+// the high nibble).
+__device__ __forceinline__ void planes_to_nibbles(const uint32_t (&pl)[4], int np,
+                                                  uint32_t (&out)[4]) {
+  uint32_t rv[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) rv[e] = e < np ? __brev(pl[e]) : 0u;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t w = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (e < np) w |= spread8((rv[e] >> (24 - 8 * q)) & 0xFFu) << e;
+    out[q] = w;
+  }
+}
+
+__device__ __forceinline__ uint4 planes_to_nibbles(const uint4 &pl) {
+  const uint32_t in[4] = {pl.x, pl.y, pl.z, pl.w};
+  uint32_t out[4];
+  planes_to_nibbles(in, 4, out);
+  return make_uint4(out[0], out[1], out[2], out[3]);
+}
+
 }  // namespace ngia

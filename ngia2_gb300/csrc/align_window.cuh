@@ -101,10 +101,10 @@ __device__ __forceinline__ void window_columns(uint32_t (&V)[W], const uint32_t 
   }
 }
 
-// One class of the round on this warp: takes pairs from order[bounds[cls],
-// bounds[cls + 1]) until the queue is empty.  col: the lane's column of the
-// warp's table of NS slots, whose code-0 row holds zeros.  Returns the lane's
-// column blocks x W.
+// One column block of the warp's pairs (the tables already at `base`): slide,
+// let the next rows enter, 32 column steps, then for a lane with a pair
+//   total = the LCS so far, ub = an upper bound of the pair's final LCS.
+// kPlanes: the target's words are bit planes, made into codes here.
 //
 // The early exit (see align.cuh): the banded LCS is the best monotone path
 // through the matrix counting matches in band cells only (rows below the band
@@ -113,6 +113,112 @@ __device__ __forceinline__ void window_columns(uint32_t (&V)[W], const uint32_t 
 // most  L(j) + min(columns left, Lr - j)  with L(j) the zeros of rows 0..j
 // now; taken at word granularity (zeros through a word's end, rows above its
 // start) and over the retired rows.
+template <int W, int NS, int K, bool kSlide, bool kPlanes>
+__device__ __forceinline__ void window_block(uint32_t (&V)[W], WindowPair &sp,
+                                             const LdsTable<NS, K> &tab, uint32_t base,
+                                             int32_t &total, int32_t &ub) {
+  const uint32_t lv = kSlide ? W - min(sp.rs, sp.nr) : 0u;
+  uint32_t j1 = 0;
+  uint4 nxt = sp.cur, pfn = sp.pf;
+  uint32_t pfn_row = sp.pf_row;
+  if (sp.active) {
+    if constexpr (kSlide) {
+      // the word sliding out is row i - lv - 1; past the rep's end it holds
+      // nothing to count
+      if ((int32_t)(sp.i - lv - 1) < (int32_t)sp.nr) sp.lcs += __popc(~V[0]);
+#pragma unroll
+      for (int m = 0; m + 1 < W; ++m) V[m] = V[m + 1];
+      V[W - 1] = kFull;
+    }
+    // the next block's code words and entering row (J1 moves up at most one
+    // row per block), loaded now so that their latency hides behind this block
+    const bool more = sp.i + 1 < sp.nc;
+    if (more) nxt = load4(sp.tar + 4 * (sp.i + 1));
+    j1 = sp.i + sp.rs < sp.nr ? sp.i + sp.rs : sp.nr;
+    const uint32_t j1n = sp.i + 1 + sp.rs < sp.nr ? sp.i + 1 + sp.rs : sp.nr;
+    if (more && j1n > j1) {
+      pfn_row = j1n - 1;
+      pfn = load4(sp.rep + 1 + 4 * pfn_row);
+    }
+    // slot of row r: base + (r - (i - lv)) sliding, r fixed
+    const uint32_t slot0 = kSlide ? base + lv - sp.i : 0u;
+    if (sp.i > sp.ls && sp.i - sp.ls <= sp.nr && (!kSlide || lv > sp.ls))
+      tab.clear(slot0 + sp.i - sp.ls - 1);  // the row leaving the band
+    if constexpr (!kSlide) {
+#pragma unroll
+      for (int m = 0; m < W; ++m)
+        if ((uint32_t)m >= sp.act) V[m] = kFull;
+    }
+    while (sp.act < j1) {
+      if (sp.act == sp.pf_row) {
+        tab.fill(slot0 + sp.act, sp.pf);
+        ++sp.act;
+      } else {  // a pair's first block: four rows' loads together
+        uint4 r[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+          if (sp.act + k < j1) r[k] = load4(sp.rep + 1 + 4 * (sp.act + k));
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+          if (sp.act + k < j1) tab.fill(slot0 + sp.act + k, r[k]);
+        sp.act = min(sp.act + 4, j1);
+      }
+    }
+  }
+  // the whole warp together (a lane without a pair steps on what its words
+  // and masks hold, which its next start replaces)
+  __syncwarp();
+  window_columns<W, NS>(V, tab.base + base * 32, kPlanes ? planes_to_nibbles(sp.cur) : sp.cur);
+  if (sp.active) {
+    ++sp.i;
+    const int32_t cols = 32 * (int32_t)sp.i;
+    const int32_t left = (int32_t)sp.lt > cols ? (int32_t)sp.lt - cols : 0;
+    // rows above the first row of word 0
+    const int32_t above0 =
+        (int32_t)sp.lr - (kSlide ? 32 * ((int32_t)sp.i - 1 - (int32_t)lv) : 0);
+    total = kSlide ? sp.lcs : 0;
+    ub = max(total, 0) + min(left, (int32_t)sp.lr);
+#pragma unroll
+    for (int m = 0; m < W; ++m) {
+      const int32_t above = above0 - 32 * m;
+      if (kSlide ? above > 0 : (uint32_t)m < j1) {
+        total += __popc(~V[m]);
+        ub = max(ub, total + min(left, above));
+      }
+    }
+    sp.cur = nxt;
+    sp.pf = pfn;
+    sp.pf_row = pfn_row;
+  }
+}
+
+// Advances the tables of a sliding window by one slot.
+template <int W, int NS, int K>
+__device__ __forceinline__ void window_advance(const LdsTable<NS, K> &tab, uint32_t &base) {
+  if (base + W == NS) {
+#pragma unroll 1
+    for (uint32_t s = 0; s + 1 < (uint32_t)W; ++s) tab.move(s, base + 1 + s);
+    base = 0;
+  } else {
+    ++base;
+  }
+}
+
+// A sliding window's words before a pair's first block (and its slide): rows
+// below 0 are zeros, taken off the count.
+template <int W>
+__device__ __forceinline__ void window_start(uint32_t (&V)[W], WindowPair &sp) {
+  const uint32_t lv = W - min(sp.rs, sp.nr);
+  sp.lcs = -32 * (int32_t)(lv + 1);
+#pragma unroll
+  for (int m = 0; m < W; ++m) V[m] = (uint32_t)m <= lv ? 0u : kFull;
+}
+
+// One class of the round on this warp: takes pairs from order[bounds[cls],
+// bounds[cls + 1]) until the queue is empty.  col: the lane's column of the
+// warp's table of NS slots, whose code-0 row holds zeros.  Returns the lane's
+// column blocks x W.
+//
 // Lanes start new pairs only every kStartEvery-th step (or when no lane has
 // one).  A start costs the warp the new rows' loads and table writes whatever
 // the lanes that start, so with 16-entry tables fewer, fuller starts are worth
@@ -192,12 +298,7 @@ __device__ __forceinline__ uint32_t align_window(const RoundArgs &a, int cls, ui
           sp.act = 0;
           sp.pf_row = kFull;
           sp.active = true;
-          if constexpr (kSlide) {  // rows below 0, as before the step's slide
-            const uint32_t lv = W - min(sp.rs, sp.nr);
-            sp.lcs = -32 * (int32_t)(lv + 1);
-#pragma unroll
-            for (int m = 0; m < W; ++m) V[m] = (uint32_t)m <= lv ? 0u : kFull;
-          }
+          if constexpr (kSlide) window_start(V, sp);
         }
       }
       a_used += take;
@@ -209,88 +310,12 @@ __device__ __forceinline__ uint32_t align_window(const RoundArgs &a, int cls, ui
       if (queue_empty) break;
       continue;
     }
-    if constexpr (kSlide) {  // every lane, with or without a pair
-      if (base + W == NS) {
-#pragma unroll 1
-        for (uint32_t s = 0; s + 1 < (uint32_t)W; ++s) tab.move(s, base + 1 + s);
-        base = 0;
-      } else {
-        ++base;
-      }
-    }
-    const uint32_t lv = kSlide ? W - min(sp.rs, sp.nr) : 0u;
-    uint32_t j1 = 0;
-    uint4 nxt = sp.cur, pfn = sp.pf;
-    uint32_t pfn_row = sp.pf_row;
+    // every lane, with or without a pair
+    if constexpr (kSlide) window_advance<W>(tab, base);
+    int32_t total = 0, ub = 0;
+    window_block<W, NS, K, kSlide, false>(V, sp, tab, base, total, ub);
     if (sp.active) {
-      if constexpr (kSlide) {
-        // the word sliding out is row i - lv - 1; past the rep's end it holds
-        // nothing to count
-        if ((int32_t)(sp.i - lv - 1) < (int32_t)sp.nr) sp.lcs += __popc(~V[0]);
-#pragma unroll
-        for (int m = 0; m + 1 < W; ++m) V[m] = V[m + 1];
-        V[W - 1] = kFull;
-      }
-      // the next block's code words and entering row (J1 moves up at most one
-      // row per block), loaded now so that their latency hides behind this block
-      const bool more = sp.i + 1 < sp.nc;
-      if (more) nxt = load4(sp.tar + 4 * (sp.i + 1));
-      j1 = sp.i + sp.rs < sp.nr ? sp.i + sp.rs : sp.nr;
-      const uint32_t j1n = sp.i + 1 + sp.rs < sp.nr ? sp.i + 1 + sp.rs : sp.nr;
-      if (more && j1n > j1) {
-        pfn_row = j1n - 1;
-        pfn = load4(sp.rep + 1 + 4 * pfn_row);
-      }
-      // slot of row r: base + (r - (i - lv)) sliding, r fixed
-      const uint32_t slot0 = kSlide ? base + lv - sp.i : 0u;
-      if (sp.i > sp.ls && sp.i - sp.ls <= sp.nr && (!kSlide || lv > sp.ls))
-        tab.clear(slot0 + sp.i - sp.ls - 1);  // the row leaving the band
-      if constexpr (!kSlide) {
-#pragma unroll
-        for (int m = 0; m < W; ++m)
-          if ((uint32_t)m >= sp.act) V[m] = kFull;
-      }
-      while (sp.act < j1) {
-        if (sp.act == sp.pf_row) {
-          tab.fill(slot0 + sp.act, sp.pf);
-          ++sp.act;
-        } else {  // a pair's first block: four rows' loads together
-          uint4 r[4];
-#pragma unroll
-          for (uint32_t k = 0; k < 4; ++k)
-            if (sp.act + k < j1) r[k] = load4(sp.rep + 1 + 4 * (sp.act + k));
-#pragma unroll
-          for (uint32_t k = 0; k < 4; ++k)
-            if (sp.act + k < j1) tab.fill(slot0 + sp.act + k, r[k]);
-          sp.act = min(sp.act + 4, j1);
-        }
-      }
-    }
-    // the whole warp together (a lane without a pair steps on what its words
-    // and masks hold, which its next start replaces)
-    __syncwarp();
-    window_columns<W, NS>(V, col + base * 32, sp.cur);
-    if (sp.active) {
-      ++sp.i;
       done += W;
-      const int32_t cols = 32 * (int32_t)sp.i;
-      const int32_t left = (int32_t)sp.lt > cols ? (int32_t)sp.lt - cols : 0;
-      // rows above the first row of word 0
-      const int32_t above0 =
-          (int32_t)sp.lr - (kSlide ? 32 * ((int32_t)sp.i - 1 - (int32_t)lv) : 0);
-      int32_t total = kSlide ? sp.lcs : 0;
-      int32_t ub = max(total, 0) + min(left, (int32_t)sp.lr);
-#pragma unroll
-      for (int m = 0; m < W; ++m) {
-        const int32_t above = above0 - 32 * m;
-        if (kSlide ? above > 0 : (uint32_t)m < j1) {
-          total += __popc(~V[m]);
-          ub = max(ub, total + min(left, above));
-        }
-      }
-      sp.cur = nxt;
-      sp.pf = pfn;
-      sp.pf_row = pfn_row;
       const bool last = sp.i >= sp.nc;
       if (last || !lcs_may_reach((uint32_t)ub, sp.lr, sp.lt, a.t)) {
         a.scores[sp.p] = last ? identity_score((uint32_t)total, sp.lr, sp.lt, a.t) : 0u;

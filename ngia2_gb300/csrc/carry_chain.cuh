@@ -14,129 +14,6 @@
 
 namespace ngia {
 
-__device__ __forceinline__ void add_chain2_zn(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  asm("add.cc.u32 %0, %2, %4;\n\t"
-      "addc.u32 %1, %3, %5;\n\t"
-      : "=r"(s[0]), "=r"(s[1])
-      : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]));
-}
-
-__device__ __forceinline__ void add_chain2_zc(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t &cout) {
-  asm("add.cc.u32 %0, %3, %5;\n\t"
-      "addc.cc.u32 %1, %4, %6;\n\t"
-      "addc.u32 %2, 0, 0;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(cout)
-      : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]));
-}
-
-__device__ __forceinline__ void add_chain2_cn(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t cin) {
-  asm("{\n\t.reg .u32 t;\n\t"
-      "add.cc.u32 t, %6, 0xFFFFFFFF;\n\t"
-      "addc.cc.u32 %0, %2, %4;\n\t"
-      "addc.u32 %1, %3, %5;\n\t"
-      "}"
-      : "=r"(s[0]), "=r"(s[1])
-      : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]), "r"(cin));
-}
-
-__device__ __forceinline__ void add_chain2_cc(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t cin, uint32_t &cout) {
-  asm("{\n\t.reg .u32 t;\n\t"
-      "add.cc.u32 t, %7, 0xFFFFFFFF;\n\t"
-      "addc.cc.u32 %0, %3, %5;\n\t"
-      "addc.cc.u32 %1, %4, %6;\n\t"
-      "addc.u32 %2, 0, 0;\n\t"
-      "}"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(cout)
-      : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]), "r"(cin));
-}
-
-__device__ __forceinline__ void add_chain4_zn(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  asm("add.cc.u32 %0, %4, %8;\n\t"
-      "addc.cc.u32 %1, %5, %9;\n\t"
-      "addc.cc.u32 %2, %6, %10;\n\t"
-      "addc.u32 %3, %7, %11;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
-}
-
-__device__ __forceinline__ void add_chain4_zc(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t &cout) {
-  asm("add.cc.u32 %0, %5, %9;\n\t"
-      "addc.cc.u32 %1, %6, %10;\n\t"
-      "addc.cc.u32 %2, %7, %11;\n\t"
-      "addc.cc.u32 %3, %8, %12;\n\t"
-      "addc.u32 %4, 0, 0;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(cout)
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
-}
-
-__device__ __forceinline__ void add_chain4_cn(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t cin) {
-  asm("{\n\t.reg .u32 t;\n\t"
-      "add.cc.u32 t, %12, 0xFFFFFFFF;\n\t"
-      "addc.cc.u32 %0, %4, %8;\n\t"
-      "addc.cc.u32 %1, %5, %9;\n\t"
-      "addc.cc.u32 %2, %6, %10;\n\t"
-      "addc.u32 %3, %7, %11;\n\t"
-      "}"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(cin));
-}
-
-__device__ __forceinline__ void add_chain4_cc(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t cin, uint32_t &cout) {
-  asm("{\n\t.reg .u32 t;\n\t"
-      "add.cc.u32 t, %13, 0xFFFFFFFF;\n\t"
-      "addc.cc.u32 %0, %5, %9;\n\t"
-      "addc.cc.u32 %1, %6, %10;\n\t"
-      "addc.cc.u32 %2, %7, %11;\n\t"
-      "addc.cc.u32 %3, %8, %12;\n\t"
-      "addc.u32 %4, 0, 0;\n\t"
-      "}"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(cout)
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(cin));
-}
-
-__device__ __forceinline__ void add_chain8_zn(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  asm("add.cc.u32 %0, %8, %16;\n\t"
-      "addc.cc.u32 %1, %9, %17;\n\t"
-      "addc.cc.u32 %2, %10, %18;\n\t"
-      "addc.cc.u32 %3, %11, %19;\n\t"
-      "addc.cc.u32 %4, %12, %20;\n\t"
-      "addc.cc.u32 %5, %13, %21;\n\t"
-      "addc.cc.u32 %6, %14, %22;\n\t"
-      "addc.u32 %7, %15, %23;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]));
-}
-
-__device__ __forceinline__ void add_chain8_zc(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t &cout) {
-  asm("add.cc.u32 %0, %9, %17;\n\t"
-      "addc.cc.u32 %1, %10, %18;\n\t"
-      "addc.cc.u32 %2, %11, %19;\n\t"
-      "addc.cc.u32 %3, %12, %20;\n\t"
-      "addc.cc.u32 %4, %13, %21;\n\t"
-      "addc.cc.u32 %5, %14, %22;\n\t"
-      "addc.cc.u32 %6, %15, %23;\n\t"
-      "addc.cc.u32 %7, %16, %24;\n\t"
-      "addc.u32 %8, 0, 0;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(cout)
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]));
-}
-
-__device__ __forceinline__ void add_chain8_cn(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t cin) {
-  asm("{\n\t.reg .u32 t;\n\t"
-      "add.cc.u32 t, %24, 0xFFFFFFFF;\n\t"
-      "addc.cc.u32 %0, %8, %16;\n\t"
-      "addc.cc.u32 %1, %9, %17;\n\t"
-      "addc.cc.u32 %2, %10, %18;\n\t"
-      "addc.cc.u32 %3, %11, %19;\n\t"
-      "addc.cc.u32 %4, %12, %20;\n\t"
-      "addc.cc.u32 %5, %13, %21;\n\t"
-      "addc.cc.u32 %6, %14, %22;\n\t"
-      "addc.u32 %7, %15, %23;\n\t"
-      "}"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(cin));
-}
-
 __device__ __forceinline__ void add_chain8_cc(uint32_t *s, const uint32_t *a, const uint32_t *b, uint32_t cin, uint32_t &cout) {
   asm("{\n\t.reg .u32 t;\n\t"
       "add.cc.u32 t, %25, 0xFFFFFFFF;\n\t"
@@ -289,31 +166,10 @@ __device__ __forceinline__ void add_words_pp(uint32_t *s, const uint32_t *a, con
 }
 
 
-// ---- one chain of any length 1..16, no carry in or out -------------------------
+// ---- one chain of a window's words, no carry in or out -------------------------
 // add_run<N>(s, a, b): s[0..N) = a[0..N) + b[0..N) as one N-word number, the
 // carry rippling through the flag across the whole run (no carry value
-// materialised between words).  Written out for each N.
-__device__ __forceinline__ void add_run1(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  asm(
-      "add.u32 %0, %1, %2;\n\t"
-      : "=r"(s[0])
-      : "r"(a[0]), "r"(b[0]));
-}
-__device__ __forceinline__ void add_run2(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  asm(
-      "add.cc.u32 %0, %2, %4;\n\t"
-      "addc.u32 %1, %3, %5;\n\t"
-      : "=r"(s[0]), "=r"(s[1])
-      : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]));
-}
-__device__ __forceinline__ void add_run3(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  asm(
-      "add.cc.u32 %0, %3, %6;\n\t"
-      "addc.cc.u32 %1, %4, %7;\n\t"
-      "addc.u32 %2, %5, %8;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(b[0]), "r"(b[1]), "r"(b[2]));
-}
+// materialised between words).  Written out for each window width.
 __device__ __forceinline__ void add_run4(uint32_t *s, const uint32_t *a, const uint32_t *b) {
   asm(
       "add.cc.u32 %0, %4, %8;\n\t"
@@ -431,24 +287,6 @@ __device__ __forceinline__ void add_run12(uint32_t *s, const uint32_t *a, const 
       : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(s[8]), "=r"(s[9]), "=r"(s[10]), "=r"(s[11])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]));
 }
-__device__ __forceinline__ void add_run13(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  asm(
-      "add.cc.u32 %0, %13, %26;\n\t"
-      "addc.cc.u32 %1, %14, %27;\n\t"
-      "addc.cc.u32 %2, %15, %28;\n\t"
-      "addc.cc.u32 %3, %16, %29;\n\t"
-      "addc.cc.u32 %4, %17, %30;\n\t"
-      "addc.cc.u32 %5, %18, %31;\n\t"
-      "addc.cc.u32 %6, %19, %32;\n\t"
-      "addc.cc.u32 %7, %20, %33;\n\t"
-      "addc.cc.u32 %8, %21, %34;\n\t"
-      "addc.cc.u32 %9, %22, %35;\n\t"
-      "addc.cc.u32 %10, %23, %36;\n\t"
-      "addc.cc.u32 %11, %24, %37;\n\t"
-      "addc.u32 %12, %25, %38;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(s[8]), "=r"(s[9]), "=r"(s[10]), "=r"(s[11]), "=r"(s[12])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(a[12]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]), "r"(b[12]));
-}
 __device__ __forceinline__ void add_run14(uint32_t *s, const uint32_t *a, const uint32_t *b) {
   asm(
       "add.cc.u32 %0, %14, %28;\n\t"
@@ -467,26 +305,6 @@ __device__ __forceinline__ void add_run14(uint32_t *s, const uint32_t *a, const 
       "addc.u32 %13, %27, %41;\n\t"
       : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(s[8]), "=r"(s[9]), "=r"(s[10]), "=r"(s[11]), "=r"(s[12]), "=r"(s[13])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(a[12]), "r"(a[13]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]), "r"(b[12]), "r"(b[13]));
-}
-__device__ __forceinline__ void add_run15(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  asm(
-      "add.cc.u32 %0, %15, %30;\n\t"
-      "addc.cc.u32 %1, %16, %31;\n\t"
-      "addc.cc.u32 %2, %17, %32;\n\t"
-      "addc.cc.u32 %3, %18, %33;\n\t"
-      "addc.cc.u32 %4, %19, %34;\n\t"
-      "addc.cc.u32 %5, %20, %35;\n\t"
-      "addc.cc.u32 %6, %21, %36;\n\t"
-      "addc.cc.u32 %7, %22, %37;\n\t"
-      "addc.cc.u32 %8, %23, %38;\n\t"
-      "addc.cc.u32 %9, %24, %39;\n\t"
-      "addc.cc.u32 %10, %25, %40;\n\t"
-      "addc.cc.u32 %11, %26, %41;\n\t"
-      "addc.cc.u32 %12, %27, %42;\n\t"
-      "addc.cc.u32 %13, %28, %43;\n\t"
-      "addc.u32 %14, %29, %44;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(s[8]), "=r"(s[9]), "=r"(s[10]), "=r"(s[11]), "=r"(s[12]), "=r"(s[13]), "=r"(s[14])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]), "r"(a[10]), "r"(a[11]), "r"(a[12]), "r"(a[13]), "r"(a[14]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]), "r"(b[12]), "r"(b[13]), "r"(b[14]));
 }
 __device__ __forceinline__ void add_run16(uint32_t *s, const uint32_t *a, const uint32_t *b) {
   asm(
@@ -649,12 +467,11 @@ __device__ __forceinline__ void add_run28(uint32_t *s, const uint32_t *a, const 
 }
 template <int N>
 __device__ __forceinline__ void add_run(uint32_t *s, const uint32_t *a, const uint32_t *b) {
-  static_assert((N >= 1 && N <= 16) || N == 18 || N == 20 || N == 24 || N == 28, "run length");
+  static_assert(N >= 4 && N <= 28, "run length");
 #define NGIA_RUN(K) \
   if constexpr (N == K) add_run##K(s, a, b);
-  NGIA_RUN(1) NGIA_RUN(2) NGIA_RUN(3) NGIA_RUN(4) NGIA_RUN(5) NGIA_RUN(6) NGIA_RUN(7)
-  NGIA_RUN(8) NGIA_RUN(9) NGIA_RUN(10) NGIA_RUN(11) NGIA_RUN(12) NGIA_RUN(13) NGIA_RUN(14)
-  NGIA_RUN(15) NGIA_RUN(16) NGIA_RUN(18) NGIA_RUN(20) NGIA_RUN(24) NGIA_RUN(28)
+  NGIA_RUN(4) NGIA_RUN(5) NGIA_RUN(6) NGIA_RUN(7) NGIA_RUN(8) NGIA_RUN(9) NGIA_RUN(10)
+  NGIA_RUN(11) NGIA_RUN(12) NGIA_RUN(14) NGIA_RUN(16) NGIA_RUN(18) NGIA_RUN(20) NGIA_RUN(24) NGIA_RUN(28)
 #undef NGIA_RUN
 }
 

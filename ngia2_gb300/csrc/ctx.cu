@@ -189,24 +189,37 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   // 4. emit: compact hits, sort by (rep, tar)
   NGIA_TRY(c->edges.reserve((size_t)(m ? m : 1) * sizeof(ngia_edge)));
   uint64_t ne = 0;
-  const bool small = m > 0 && m <= kSmallEmit;
-  if (small) {
+  // few pairs, or few of them that scored (at high identities a few hundred of
+  // millions), are emitted without a wait for their count; the general path
+  // follows where there turn out to be more
+  Counters &rc = c->h_counters->round;
+  if (m > 0) {
     uint64_t *d_m = &dc->unique_total;  // read above, free now
-    NGIA_TRY(emit_small(pairs, scores, m, c->edges.as<ngia_edge>(), d_m, s));
+    if (m <= kSmallEmit) {
+      NGIA_TRY(emit_small(pairs, scores, m, c->edges.as<ngia_edge>(), d_m, s));
+    } else {
+      NGIA_TRY(c->emit_tmp.reserve(kSmallEmit * sizeof(uint32_t)));
+      NGIA_CUDA(cudaMemsetAsync(d_m, 0, sizeof(uint64_t), s));
+      NGIA_TRY(emit_few(pairs, scores, m, c->edges.as<ngia_edge>(), c->emit_tmp.as<uint32_t>(),
+                        d_m, s));
+    }
     NGIA_CUDA(cudaEventRecord(c->ev[3], s));
     NGIA_CUDA(cudaMemcpyAsync(&c->h_counters->edges, d_m, sizeof(uint64_t),
                               cudaMemcpyDeviceToHost, s));
   } else {
-    NGIA_TRY(c->emit_tmp.reserve(emit_scratch_bytes(m, n)));
-    NGIA_TRY(emit_sorted(pairs, scores, m, n, c->edges.as<ngia_edge>(), &ne, c->emit_tmp.p, s));
     NGIA_CUDA(cudaEventRecord(c->ev[3], s));
   }
-  Counters &rc = c->h_counters->round;
   if (st)
     NGIA_CUDA(cudaMemcpyAsync(&rc, c->round.counters(), sizeof(Counters), cudaMemcpyDeviceToHost,
                               s));
   NGIA_CUDA(cudaStreamSynchronize(s));
-  if (small) ne = c->h_counters->edges;
+  if (m > 0) ne = c->h_counters->edges;
+  if (ne > kSmallEmit) {
+    NGIA_TRY(c->emit_tmp.reserve(emit_scratch_bytes(m, n)));
+    NGIA_TRY(emit_sorted(pairs, scores, m, n, c->edges.as<ngia_edge>(), &ne, c->emit_tmp.p, s));
+    NGIA_CUDA(cudaEventRecord(c->ev[3], s));
+    NGIA_CUDA(cudaEventSynchronize(c->ev[3]));
+  }
   c->n_edges = ne;
   if (h_n_edges) *h_n_edges = ne;
   if (st) {

@@ -89,6 +89,10 @@ int persistent_grid(const void *func, int threads, size_t smem, uint32_t want, u
 // of its classes through their cursors, zero before the launch).  m: the
 // round's pairs, an upper bound of any class's.
 constexpr int kAlignKernels = 5;
+// Whether a round of windows of at most `widest` words can have pairs for it.
+constexpr bool align_kernel_used(int kernel, uint32_t widest) {
+  return kernel != 2 || widest > 16;
+}
 int launch_align(int kernel, const RoundArgs &a, int K, uint32_t m, cudaStream_t s);
 // All layouts of records offs[0..n) in one pass under an assumed code map
 // (inv: nibble d = residue code of aligner code d, pipelined loads): nibbles,
@@ -138,22 +142,24 @@ int collect_count(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_
 int collect_write(const uint32_t *rep, const uint32_t *lens, uint32_t n, uint32_t bands,
                   uint32_t identity, const uint64_t *offsets, uint2 *pairs,
                   cudaStream_t s);
-// Width class sort keys of `count` pairs, per-class counts (added to
-// class_count) and band cells (added to *cells).  widest: the widest sliding
-// window to use (widest_window).
+// Queue keys of `count` pairs (class_sort_key), their counts (added to
+// key_count, the skip class left out), band cells (added to *cells) and scores
+// zeroed.  widest: the widest sliding window to use.
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
-             const ClassPlan &plan, uint32_t widest, uint32_t *cls, unsigned int *class_count,
-             unsigned long long *cells, cudaStream_t s);
-// bounds[c] = pairs in classes below c (kNumRoundClasses + 1 entries).
-int class_bounds(const unsigned int *class_count, uint32_t *bounds, cudaStream_t s);
+             const ClassPlan &plan, uint32_t widest, uint8_t *keys, unsigned int *key_count,
+             unsigned long long *cells, uint32_t *scores, cudaStream_t s);
+// The queue from the keys and their counts: bounds[c] = pairs in classes below c
+// (kNumRoundClasses + 1 entries), order[] the pairs by key.  key_count is used up.
+int place_pairs(const uint8_t *keys, uint32_t count, unsigned int *key_count, uint32_t *bounds,
+                uint32_t *order, cudaStream_t s);
 // seed_filter.cu
 // Moves the pairs whose score is certainly 0, by the words their sequences
-// share, from their class (cls, class_count) to the skip class; between
-// classify and class_bounds.  K: the alphabet's table entries; *cursor zero
+// share, from their class (keys, key_count) to the skip class; between
+// classify and place_pairs.  K: the alphabet's table entries; *cursor zero
 // before the call.
 int seed_filter(const uint32_t *nib, int K, const uint64_t *offs, const uint32_t *lens,
-                const uint2 *pairs, uint32_t m, uint32_t identity, uint32_t *cls,
-                unsigned int *class_count, unsigned int *cursor, cudaStream_t s);
+                const uint2 *pairs, uint32_t m, uint32_t identity, uint8_t *keys,
+                unsigned int *key_count, unsigned int *cursor, cudaStream_t s);
 // The whole binning of a round of at most kSmallRound pairs in one launch: the
 // queue order, the class bounds and band cells, cursors and computed blocks
 // zeroed, scores zeroed.
@@ -180,6 +186,11 @@ int emit_sorted(const uint2 *pairs, const uint32_t *scores, uint32_t count,
 constexpr uint32_t kSmallEmit = 4096;
 int emit_small(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
                uint64_t *d_m, cudaStream_t s);
+// The same for any number of pairs as long as at most kSmallEmit of them scored
+// (more: *d_m is some larger number and nothing was written).  hits: kSmallEmit words; *d_m zero
+// before the call.
+int emit_few(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
+             uint32_t *hits, uint64_t *d_m, cudaStream_t s);
 // Fast mode's bands [b0, b1): first_band[target] = min of itself and the first
 // of those bands that names the rep of a pair scoring > 0.
 int fast_first_band(const uint32_t *rep, uint32_t n, uint32_t b0, uint32_t b1,

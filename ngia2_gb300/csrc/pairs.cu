@@ -276,23 +276,26 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 }
 
 // ---- width classes ------------------------------------------------------------------
+// A pair's queue key (class_sort_key: its class, then its columns in octaves)
+// in a byte, the keys' histogram, and each pair's place in the queue by its
+// key's run.  The order inside a run is free, so two passes of atomics place
+// the pairs where a radix sort took three launches and moved the keys too.
 constexpr uint32_t kClassifyUnroll = 4;
 
 __global__ void __launch_bounds__(256)
 classify_kernel(const uint32_t *__restrict__ lens, const uint2 *__restrict__ pairs,
-                uint64_t count, float t, int fma_mode, ClassPlan plan, uint32_t widest,
-                uint32_t *__restrict__ cls,
-                unsigned int *__restrict__ class_count,
-                unsigned long long *__restrict__ cells) {
-  __shared__ unsigned int sc[kNumRoundClasses];
+                uint32_t count, float t, int fma_mode, ClassPlan plan, uint32_t widest,
+                uint8_t *__restrict__ keys, unsigned int *__restrict__ key_count,
+                unsigned long long *__restrict__ cells, uint32_t *__restrict__ scores) {
+  __shared__ unsigned int sc[kQueueKeys];
   __shared__ unsigned long long scells;
-  if (threadIdx.x < kNumRoundClasses) sc[threadIdx.x] = 0;
+  sc[threadIdx.x] = 0;
   if (threadIdx.x == 0) scells = 0;
   __syncthreads();
   unsigned long long my_cells = 0;
   const uint32_t lt_mask = (1u << (threadIdx.x & 31u)) - 1u;
   // block-uniform trips of kClassifyUnroll pairs per thread (their loads in
-  // flight together), so that the class counts can be summed per warp
+  // flight together), so that the key counts can be summed per warp
   constexpr uint32_t U = kClassifyUnroll;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t p0 = (uint64_t)blockIdx.x * blockDim.x; p0 < count; p0 += U * stride) {
@@ -312,62 +315,109 @@ classify_kernel(const uint32_t *__restrict__ lens, const uint2 *__restrict__ pai
 #pragma unroll
     for (uint32_t u = 0; u < U; ++u) {
       const uint64_t p = p0 + u * stride + threadIdx.x;
-      uint32_t c = kFull;
+      uint32_t key = kFull;
       if (p < count) {
-        if (pr[u].x == kFull) {  // an empty pair slot (serving): never aligned
-          c = kSkipClass;
-          cls[p] = skip_sort_key();
-        } else {
+        key = skip_sort_key();  // (an empty pair slot is never aligned)
+        if (pr[u].x != kFull) {
           const Band b = make_band(lr[u], lt[u], t, fma_mode);
-          c = (uint32_t)round_class(b, plan, widest);
-          cls[p] = class_sort_key((int)c, b);
+          key = class_sort_key(round_class(b, plan, widest), b);
           my_cells += band_blocks(b);
         }
+        keys[p] = (uint8_t)key;
+        scores[p] = 0;
       }
-      const uint32_t peers = __match_any_sync(kFull, c);
-      if (c != kFull && (peers & lt_mask) == 0) atomicAdd(&sc[c], (unsigned int)__popc(peers));
+      const uint32_t peers = __match_any_sync(kFull, key);
+      if (key < kQueueKeys && (peers & lt_mask) == 0)
+        atomicAdd(&sc[key], (unsigned int)__popc(peers));
     }
   }
   my_cells = warp_sum(my_cells);
   if ((threadIdx.x & 31u) == 0 && my_cells) atomicAdd(&scells, my_cells);
   __syncthreads();
-  if (threadIdx.x < kNumRoundClasses && sc[threadIdx.x]) atomicAdd(&class_count[threadIdx.x], sc[threadIdx.x]);
+  if (sc[threadIdx.x] && threadIdx.x >> 3 != (uint32_t)kSkipClass)
+    atomicAdd(&key_count[threadIdx.x], sc[threadIdx.x]);
   if (threadIdx.x == 0 && scells) atomicAdd(cells, scells * 1024ull);
 }
 
-__global__ void class_bounds_kernel(const unsigned int *__restrict__ class_count,
-                                    uint32_t *__restrict__ bounds) {
-  static_assert(kNumRoundClasses <= 32, "one warp");
-  const uint32_t lane = threadIdx.x;
-  const uint32_t v = lane < kNumRoundClasses ? class_count[lane] : 0u;
+// key_count -> each key's first place; the classes' bounds.
+__global__ void __launch_bounds__(kQueueKeys)
+class_bounds_kernel(unsigned int *__restrict__ key_count, uint32_t *__restrict__ bounds) {
+  __shared__ uint32_t wsum[kQueueKeys / 32];
+  const uint32_t k = threadIdx.x, lane = k & 31u, v = key_count[k];
   uint32_t x = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_up_sync(kFull, x, o);
     if (lane >= (uint32_t)o) x += y;
   }
-  if (lane < kNumRoundClasses) bounds[lane] = x - v;
-  if (lane == 31) bounds[kNumRoundClasses] = x;
+  if (lane == 31) wsum[k >> 5] = x;
+  __syncthreads();
+  for (uint32_t w = 0; w < k >> 5; ++w) x += wsum[w];
+  key_count[k] = x - v;
+  static_assert(kQueueKeys == 8 * kNumRoundClasses, "eight octaves a class");
+  if ((k & 7u) == 0) bounds[k >> 3] = x - v;
+  if (k == kQueueKeys - 1) bounds[kNumRoundClasses] = x;
+}
+
+// Places the pairs by their keys: a block takes its keys' shares of their runs
+// with one atomic per key, its threads their places in those.
+constexpr uint32_t kPlacePairs = 16;  // per thread
+
+__global__ void __launch_bounds__(256)
+place_kernel(const uint8_t *__restrict__ keys, uint32_t count,
+             unsigned int *__restrict__ key_next, uint32_t *__restrict__ order) {
+  __shared__ unsigned int at[kQueueKeys];
+  at[threadIdx.x] = 0;
+  __syncthreads();
+  const uint32_t base = blockIdx.x * (256u * kPlacePairs);
+  const uint32_t lt_mask = (1u << (threadIdx.x & 31u)) - 1u;
+  uint32_t key[kPlacePairs];
+#pragma unroll
+  for (uint32_t j = 0; j < kPlacePairs; ++j) {
+    const uint32_t p = base + j * 256u + threadIdx.x;
+    key[j] = p < count ? keys[p] : skip_sort_key();
+  }
+  uint32_t place[kPlacePairs];  // within the block's share of the key
+#pragma unroll
+  for (uint32_t j = 0; j < kPlacePairs; ++j) {
+    const uint32_t peers = __match_any_sync(kFull, key[j]);
+    const uint32_t leader = __ffs(peers) - 1;
+    uint32_t first = 0;
+    if ((threadIdx.x & 31u) == leader) first = atomicAdd(&at[key[j]], (unsigned)__popc(peers));
+    place[j] = __shfl_sync(kFull, first, leader) + __popc(peers & lt_mask);
+  }
+  __syncthreads();
+  const unsigned int mine = at[threadIdx.x];
+  if (mine && threadIdx.x >> 3 != (uint32_t)kSkipClass)
+    at[threadIdx.x] = atomicAdd(&key_next[threadIdx.x], mine);
+  __syncthreads();
+#pragma unroll
+  for (uint32_t j = 0; j < kPlacePairs; ++j)
+    if (key[j] >> 3 != (uint32_t)kSkipClass)
+      order[at[key[j]] + place[j]] = base + j * 256u + threadIdx.x;
 }
 
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
-             const ClassPlan &plan, uint32_t widest, uint32_t *cls, unsigned int *class_count,
-             unsigned long long *cells, cudaStream_t s) {
-  if (count > 0) {
-    int dev = 0, sms = 0;
-    NGIA_CUDA(cudaGetDevice(&dev));
-    NGIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const uint32_t want = ceil_div(count, 256u), cap = (uint32_t)sms * 8;
-    classify_kernel<<<want < cap ? want : cap, 256, 0, s>>>(
-        lens, pairs, count, identity_threshold(identity), round_mode(), plan, widest, cls,
-        class_count, cells);
-    NGIA_LAUNCHED();
-  }
+             const ClassPlan &plan, uint32_t widest, uint8_t *keys, unsigned int *key_count,
+             unsigned long long *cells, uint32_t *scores, cudaStream_t s) {
+  if (count == 0) return NGIA_OK;
+  int dev = 0, sms = 0;
+  NGIA_CUDA(cudaGetDevice(&dev));
+  NGIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const uint32_t want = ceil_div(count, 256u), cap = (uint32_t)sms * 8;
+  classify_kernel<<<want < cap ? want : cap, 256, 0, s>>>(
+      lens, pairs, count, identity_threshold(identity), round_mode(), plan, widest, keys,
+      key_count, cells, scores);
+  NGIA_LAUNCHED();
   return NGIA_OK;
 }
 
-int class_bounds(const unsigned int *class_count, uint32_t *bounds, cudaStream_t s) {
-  class_bounds_kernel<<<1, 32, 0, s>>>(class_count, bounds);
+int place_pairs(const uint8_t *keys, uint32_t count, unsigned int *key_count, uint32_t *bounds,
+                uint32_t *order, cudaStream_t s) {
+  class_bounds_kernel<<<1, kQueueKeys, 0, s>>>(key_count, bounds);
+  NGIA_LAUNCHED();
+  if (count == 0) return NGIA_OK;
+  place_kernel<<<ceil_div(count, 256u * kPlacePairs), 256, 0, s>>>(keys, count, key_count, order);
   NGIA_LAUNCHED();
   return NGIA_OK;
 }
@@ -742,6 +792,60 @@ emit_small_kernel(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ 
     out[k] = ed;
   }
   if (tid == 0) *d_m = m;
+}
+
+// Any number of pairs, few of which scored: their indices are appended (warp by
+// warp, until there are too many) to a list of kSmallEmit, which one block sorts
+// as above.
+__global__ void __launch_bounds__(256)
+append_hits_kernel(const uint32_t *__restrict__ scores, uint32_t count,
+                   uint32_t *__restrict__ hits, unsigned long long *__restrict__ d_m) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t p0 = blockIdx.x * 256u; p0 < count; p0 += gridDim.x * 256u) {  // block-uniform
+    const uint32_t p = p0 + threadIdx.x;
+    const bool hit = p < count && scores[p] > 0;
+    const uint32_t all = __ballot_sync(kFull, hit);
+    if (all == 0) continue;
+    unsigned long long first = 0;
+    if (lane == 0) first = atomicAdd(d_m, (unsigned long long)__popc(all));
+    first = __shfl_sync(kFull, first, 0);
+    if (first > kSmallEmit) return;  // too many: the general path takes over
+    first += __popc(all & ((1u << lane) - 1u));
+    if (hit && first < kSmallEmit) hits[first] = p;
+  }
+}
+
+__global__ void __launch_bounds__(1024)
+emit_hits_kernel(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ scores,
+                 const uint32_t *__restrict__ hits, ngia_edge *__restrict__ out,
+                 const uint64_t *__restrict__ d_m) {
+  __shared__ uint64_t keys[kSmallEmit];
+  const uint64_t all = *d_m;
+  if (all > kSmallEmit) return;
+  const uint32_t m = (uint32_t)all;
+  for (uint32_t k = threadIdx.x; k < m; k += 1024)
+    keys[k] = (uint64_t)pairs[hits[k]].x << 32 | hits[k];
+  __syncthreads();
+  block_sort(keys, m);
+  for (uint32_t k = threadIdx.x; k < m; k += 1024) {
+    const uint32_t p = (uint32_t)keys[k];
+    ngia_edge ed;
+    ed.rep = (int32_t)(keys[k] >> 32);
+    ed.tar = (int32_t)pairs[p].y;
+    ed.weight = __fdiv_rn(__uint2float_rn(scores[p]), 100.0f);
+    out[k] = ed;
+  }
+}
+
+int emit_few(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
+             uint32_t *hits, uint64_t *d_m, cudaStream_t s) {
+  const uint32_t want = ceil_div(count, 256u * 8u), cap = 152u * 8u;
+  append_hits_kernel<<<want < cap ? want : cap, 256, 0, s>>>(
+      scores, count, hits, reinterpret_cast<unsigned long long *>(d_m));
+  NGIA_LAUNCHED();
+  emit_hits_kernel<<<1, 1024, 0, s>>>(pairs, scores, hits, out, d_m);
+  NGIA_LAUNCHED();
+  return NGIA_OK;
 }
 
 int emit_small(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,

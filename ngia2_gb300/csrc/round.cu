@@ -71,8 +71,13 @@ int Round::init(cudaStream_t s) {
     e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
     own_stream_ = e == cudaSuccess;
   }
+  // earlier kernels at higher priorities, so that ready at one time they get the
+  // device in that order
+  int least = 0, greatest = 0;
+  if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
   for (int k = 0; k < kSide && e == cudaSuccess; ++k) {
-    e = cudaStreamCreateWithFlags(&side_[k], cudaStreamNonBlocking);
+    e = cudaStreamCreateWithPriority(&side_[k], cudaStreamNonBlocking,
+                                     greatest + k < least ? greatest + k : least);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join_[k], cudaEventDisableTiming);
   }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming);
@@ -104,10 +109,8 @@ void Round::destroy() {
   if (exec_) cudaGraphExecDestroy(exec_);
   exec_ = nullptr;
   counters_.release();
-  cls_.release();
-  cls_sorted_.release();
+  keys_.release();
   order_.release();
-  sort_tmp_.release();
   if (own_stream_ && stream) cudaStreamDestroy(stream);
   stream = nullptr;
   own_stream_ = false;
@@ -116,10 +119,8 @@ void Round::destroy() {
 int Round::reserve(uint32_t m) {
   const size_t n = m ? m : 1;
   NGIA_TRY(counters_.reserve(sizeof(Counters)));
-  NGIA_TRY(cls_.reserve(n * 4));
-  NGIA_TRY(cls_sorted_.reserve(n * 4));
+  NGIA_TRY(keys_.reserve(n));
   NGIA_TRY(order_.reserve(n * 4));
-  NGIA_TRY(sort_tmp_.reserve(radix_sort_scratch_bytes((uint32_t)n, 1)));
   return NGIA_OK;
 }
 
@@ -141,40 +142,38 @@ int Round::enqueue(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t id
                        round_mode(),
                        &dc->work};
   if (!args.rows) return NGIA_ERR_STATE;
-  if (m > 0 && m <= kSmallRound) {
-    // no window over 16 words: few pairs leave the device mostly idle, and a
-    // wide pair's columns end sooner on a group of lanes (align, proteins at
-    // identity 50, windows up to 24 / 16 / 12 words: 409 pairs 92 / 61 / 57 us,
-    // 1,176: 96 / 65 / 62, 2,957: 98 / 94 / 96, 7,800: 119 / 113 / 123)
-    NGIA_TRY(bin_small(db.lens, pairs, m, identity, plan, 16u,
-                       order_.as<uint32_t>(), dc->bounds, dc->cursor, &dc->cells, &dc->work,
-                       scores, s));
-    if (ev_mid) NGIA_CUDA(cudaEventRecord(ev_mid, s));
+  // no window over 16 words in a round of few pairs: they leave the device mostly
+  // idle, and a wide pair's columns end sooner on a group of lanes (align,
+  // proteins at identity 50, windows up to 24 / 16 / 12 words: 409 pairs 92 / 61
+  // / 57 us, 1,176: 96 / 65 / 62, 2,957: 98 / 94 / 96, 7,800: 119 / 113 / 123)
+  const bool small = m > 0 && m <= kSmallRound;
+  const uint32_t widest = small ? 16u : widest_window(db.ab.K);
+  if (small) {
+    NGIA_TRY(bin_small(db.lens, pairs, m, identity, plan, widest, order_.as<uint32_t>(),
+                       dc->bounds, dc->cursor, &dc->cells, &dc->work, scores, s));
   } else {
     NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
-    NGIA_TRY(classify(db.lens, pairs, m, identity, plan, widest_window(db.ab.K),
-                      cls_.as<uint32_t>(), dc->class_count, &dc->cells, s));
+    NGIA_TRY(classify(db.lens, pairs, m, identity, plan, widest, keys_.as<uint8_t>(),
+                      dc->key_count, &dc->cells, scores, s));
     NGIA_TRY(seed_filter(db.nib, db.ab.K, db.offs, db.lens, pairs, m, identity,
-                         cls_.as<uint32_t>(), dc->class_count, &dc->seed_cursor, s));
-    NGIA_TRY(class_bounds(dc->class_count, dc->bounds, s));
-    NGIA_TRY(radix_sort_pairs(cls_.as<uint32_t>(), nullptr, cls_sorted_.as<uint32_t>(),
-                              order_.as<uint32_t>(), m, 1, 0, kClassKeyBits, sort_tmp_.p, s));
-    NGIA_CUDA(cudaMemsetAsync(scores, 0, (size_t)(m ? m : 1) * 4, s));
-    if (ev_mid) NGIA_CUDA(cudaEventRecord(ev_mid, s));
-    if (m == 0) return NGIA_OK;
+                         keys_.as<uint8_t>(), dc->key_count, &dc->seed_cursor, s));
+    NGIA_TRY(place_pairs(keys_.as<uint8_t>(), m, dc->key_count, dc->bounds,
+                         order_.as<uint32_t>(), s));
   }
+  if (ev_mid) NGIA_CUDA(cudaEventRecord(ev_mid, s));
+  if (m == 0) return NGIA_OK;
   // the kernels as concurrent branches, widest classes first: the few long
   // pairs' warps leave most of the device to the others instead of running
   // alone at the end
   NGIA_CUDA(cudaEventRecord(fork_, s));
-  for (int k = 0; k < kSide; ++k) NGIA_CUDA(cudaStreamWaitEvent(side_[k], fork_, 0));
-  static_assert(kAlignKernels == kSide + 1, "one branch per kernel");
-  for (int k = 0; k < kAlignKernels; ++k)
-    NGIA_TRY(launch_align(k, args, db.ab.K, m, k < kSide ? side_[k] : s));
-  for (int j = 0; j < kSide; ++j) {
-    NGIA_CUDA(cudaEventRecord(join_[j], side_[j]));
-    NGIA_CUDA(cudaStreamWaitEvent(s, join_[j], 0));
+  for (int k = 0; k < kAlignKernels; ++k) {
+    if (!align_kernel_used(k, widest)) continue;
+    NGIA_CUDA(cudaStreamWaitEvent(side_[k], fork_, 0));
+    NGIA_TRY(launch_align(k, args, db.ab.K, m, side_[k]));
+    NGIA_CUDA(cudaEventRecord(join_[k], side_[k]));
   }
+  for (int k = 0; k < kAlignKernels; ++k)
+    if (align_kernel_used(k, widest)) NGIA_CUDA(cudaStreamWaitEvent(s, join_[k], 0));
   return NGIA_OK;
 }
 

@@ -33,7 +33,7 @@ struct Counters {  // device-side counters of one graph build or round
   unsigned long long cand_total;
   unsigned long long cells;
   uint64_t unique_total;
-  unsigned int class_count[kNumRoundClasses];
+  unsigned int key_count[kQueueKeys];  // pairs per queue key, then each key's next place
   unsigned long long work;  // 32x32 blocks the aligners computed
   unsigned int cursor[kNumRoundClasses];  // pairs taken from each class's queue
   uint32_t bounds[kNumRoundClasses + 1];  // class ranges of the queue order
@@ -64,7 +64,7 @@ struct RoundStats {
 
 class Round {
  public:
-  static constexpr int kSide = 4;
+  static constexpr int kSide = kAlignKernels;  // a stream per kernel
   cudaStream_t stream = nullptr;
   ClassPlan plan = default_plan();
   uint64_t plan_gen = 0;
@@ -92,7 +92,7 @@ class Round {
              uint32_t *scores);
 
  private:
-  DevBuf counters_, cls_, cls_sorted_, order_, sort_tmp_;
+  DevBuf counters_, keys_, order_;
   cudaStream_t side_[kSide] = {};
   cudaEvent_t join_[kSide] = {}, fork_ = nullptr, ev_[3] = {};
   bool own_stream_ = false;

@@ -160,15 +160,15 @@ template <int Q>
 __global__ void __launch_bounds__(kSeedWarps * 32)
 seed_filter_kernel(const uint32_t *__restrict__ nib, const uint64_t *__restrict__ offs,
                    const uint32_t *__restrict__ lens, const uint2 *__restrict__ pairs,
-                   uint32_t m, float t, int fma_mode, uint32_t *__restrict__ cls,
-                   unsigned int *__restrict__ class_count, unsigned int *__restrict__ cursor,
+                   uint32_t m, float t, int fma_mode, uint8_t *__restrict__ keys,
+                   unsigned int *__restrict__ key_count, unsigned int *__restrict__ cursor,
                    uint32_t run) {
   __shared__ __align__(16) uint32_t sets[kSeedWarps][kSeedWords];
-  __shared__ unsigned int out[kNumRoundClasses];
+  __shared__ unsigned int out[kQueueKeys];
   constexpr uint32_t kPer = 8 / Q;  // tests per code word
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t *set = sets[threadIdx.x >> 5];
-  if (threadIdx.x < kNumRoundClasses) out[threadIdx.x] = 0;
+  for (uint32_t k = threadIdx.x; k < kQueueKeys; k += kSeedWarps * 32) out[k] = 0;
   __syncthreads();
   uint32_t target = kFull;  // whose words the set holds
   for (;;) {
@@ -178,7 +178,7 @@ seed_filter_kernel(const uint32_t *__restrict__ nib, const uint64_t *__restrict_
     if (first >= m) break;
     for (uint32_t base = first; base < min(m, first + run); base += 32) {
       const uint32_t p = base + lane;
-      uint32_t key = p < m ? cls[p] : skip_sort_key();
+      const uint32_t key = p < m ? keys[p] : skip_sort_key();
       uint2 pr = make_uint2(0u, 0u);
       uint32_t lr = 0, lt = 0, need = kFull;
       uint64_t ro = 0, to = 0;
@@ -196,9 +196,10 @@ seed_filter_kernel(const uint32_t *__restrict__ nib, const uint64_t *__restrict_
       // waited for, shared by the pairs of these 32 that have it) and about
       // need words tested, against the columns an unrelated pair takes before
       // its exit times its window (a group of lanes takes twice as long).  The
-      // factor where it measured best: 200,000 nucleotide reads at 95, binning
-      // and align 3.57 ms without the filter, 2.17 / 2.05 / 2.07 at 1.25 / 0.8 /
-      // 0.5; 2 million unordered protein pairs at 90 7.98, 5.6 - 6.9.
+      // factors where they measured best: 200,000 nucleotide reads at 95, whose
+      // targets have 47 pairs each, binning and align 3.57 ms without the
+      // filter, 2.17 / 2.05 / 2.07 at 1.25 / 0.8 / 0.5; 2 million unordered
+      // protein pairs at 90 7.98 ms without, 5.5 / 6.0 at 1.25 / 0.8.
       const uint32_t peers = __match_any_sync(kFull, eligible ? pr.y : kFull - 1u);
       uint32_t ls = 0, rs = 0;
       if (eligible) {
@@ -206,10 +207,11 @@ seed_filter_kernel(const uint32_t *__restrict__ nib, const uint64_t *__restrict_
         ls = b.ls;
         rs = b.rs;
         const uint32_t words = stream_width(b);
-        const float shared = 1.0f / (float)__popc(peers);
+        const uint32_t sharers = __popc(peers);
+        const float shared = 1.0f / (float)sharers;
         const float align = (float)(need + 64) * (float)(words + 3) * (words > 28 ? 0.25f : 0.125f);
         const float test = ((float)lt * 0.25f + 400.0f) * shared + 40.0f + 0.65f * (float)need;
-        eligible = need <= kPer * (lr >> 3) && align > 0.8f * test;
+        eligible = need <= kPer * (lr >> 3) && align > (sharers >= 4 ? 0.8f : 1.25f) * test;
       }
       // The band lets a rep's word meet the target's only within its own reach,
       // so a long target's words are marked a window at a time.
@@ -267,29 +269,31 @@ seed_filter_kernel(const uint32_t *__restrict__ nib, const uint64_t *__restrict_
           todo &= todo - 1;
         }
       }
-      const uint32_t dropped = __match_any_sync(kFull, drop ? key >> 3 : kFull);
+      const uint32_t dropped = __match_any_sync(kFull, drop ? key : kFull);
       if (drop) {
         if ((dropped & ((1u << lane) - 1u)) == 0)
-          atomicAdd(&out[key >> 3], (unsigned int)__popc(dropped));
-        cls[p] = skip_sort_key();
+          atomicAdd(&out[key], (unsigned int)__popc(dropped));
+        keys[p] = (uint8_t)skip_sort_key();
       }
     }
   }
   __syncthreads();
-  if (threadIdx.x < kNumRoundClasses && out[threadIdx.x]) {
-    atomicSub(class_count + threadIdx.x, out[threadIdx.x]);
-    atomicAdd(class_count + kSkipClass, out[threadIdx.x]);
-  }
+  for (uint32_t k = threadIdx.x; k < kQueueKeys; k += kSeedWarps * 32)
+    if (out[k]) atomicSub(key_count + k, out[k]);
 }
 
 int seed_filter(const uint32_t *nib, int K, const uint64_t *offs, const uint32_t *lens,
-                const uint2 *pairs, uint32_t m, uint32_t identity, uint32_t *cls,
-                unsigned int *class_count, unsigned int *cursor, cudaStream_t s) {
+                const uint2 *pairs, uint32_t m, uint32_t identity, uint8_t *keys,
+                unsigned int *key_count, unsigned int *cursor, cudaStream_t s) {
   const uint32_t q = K == 16 ? 4 : 8;
   // every rep of Lr residues has Lr / q blocks, and a pair passes the length
   // filter with at least (1 - t) Lr unmatched to spare: below 1 - 1 / q no
   // pair can be told
   if (m == 0 || identity * q <= 100 * (q - 1)) return NGIA_OK;
+  // few pairs of a large alphabet, mostly relatives, are aligned in less than
+  // the filter's own latency (38,873 protein pairs: align 59 us without, 55
+  // with it, after 24 us of filter)
+  if (q == 4 && m < 65536u) return NGIA_OK;
   const float t = identity_threshold(identity);
   const void *func = q == 4 ? reinterpret_cast<const void *>(seed_filter_kernel<4>)
                             : reinterpret_cast<const void *>(seed_filter_kernel<8>);
@@ -301,10 +305,10 @@ int seed_filter(const uint32_t *nib, int K, const uint64_t *offs, const uint32_t
   run = run < 32u ? 32u : run > 256u ? 256u : run;
   if (q == 4)
     seed_filter_kernel<4><<<grid, kSeedWarps * 32, 0, s>>>(
-        nib, offs, lens, pairs, m, t, round_mode(), cls, class_count, cursor, run);
+        nib, offs, lens, pairs, m, t, round_mode(), keys, key_count, cursor, run);
   else
     seed_filter_kernel<8><<<grid, kSeedWarps * 32, 0, s>>>(
-        nib, offs, lens, pairs, m, t, round_mode(), cls, class_count, cursor, run);
+        nib, offs, lens, pairs, m, t, round_mode(), keys, key_count, cursor, run);
   NGIA_LAUNCHED();
   return NGIA_OK;
 }

@@ -29,20 +29,22 @@ int main() {
   for (uint32_t id = 5; id <= 95; id += 5)
     for (uint32_t lr = 1; lr < 4000; lr += 1 + lr / 37)
       for (uint32_t lt = 1; lt <= 4000; lt += 1 + lt / 29)
-        for (int K = 8; K <= 16; K += 8) {
+        for (uint32_t widest = 16; widest <= kWidestWindow; widest += 12) {
           const Band b = make_band(lr, lt, identity_threshold(id), NGIA_ROUND_FMA);
           const uint32_t ws = stream_width(b);
-          const int c = round_class(b, default_plan(), widest_window(K));
+          const int c = round_class(b, default_plan(), widest);
           const int base = width_class(b, default_plan());
           bool ok = c >= 0 && c < kNumRoundClasses && (class_sort_key(c, b) >> 3) == (uint32_t)c;
-          if (c >= kFirstFixedClass) ok = ok && (int)b.nr <= fixed_width(c - kFirstFixedClass);
+          if (c >= kFirstFixedClass)
+            ok = ok && (int)b.nr <= fixed_width(c - kFirstFixedClass) &&
+                 (widest > 16 || fixed_width(c - kFirstFixedClass) <= 16);
           else if (c >= kFirstWideClass)
             ok = ok && (int)ws <= wide_width(c - kFirstWideClass) &&
-                 wide_width(c - kFirstWideClass) <= (int)widest_window(K);
+                 wide_width(c - kFirstWideClass) <= (int)widest;
           else ok = ok && c == base;
           ok = ok && (c == kSkipClass) == !b.pass;
-          ok = ok && round_class(b, narrow, widest_window(K)) == width_class(b, narrow);
-          if (!ok && bad++ < 5) printf("lr %u lt %u id %u K %d class %d\n", lr, lt, id, K, c);
+          ok = ok && round_class(b, narrow, widest) == width_class(b, narrow);
+          if (!ok && bad++ < 5) printf("lr %u lt %u id %u widest %u class %d\n", lr, lt, id, widest, c);
           ++seen[c];
         }
   for (int c = kFirstWideClass; c < kNumRoundClasses; ++c) bad += seen[c] == 0;
