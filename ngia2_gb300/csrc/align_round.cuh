@@ -87,11 +87,15 @@ align_group_kernel(const __grid_constant__ RoundArgs a) {
   count_work(done, a.work);
 }
 
-// The one-pair-per-lane classes in three kernels by width (tier 0: windows of
-// 4-8 words, 1: 9-16, 2: 18-28), one warp per block, a table of
-// window_slots(K, tier) slots each.
+// The one-pair-per-lane classes in kernels by width, one warp per block, a
+// table of window_slots(K, tier) slots each: tier 0 windows of 4-8 words, 1 of
+// 9-16 (rounds of few pairs), 2 of 18-28, and for other rounds 9-12 and 14-16 by
+// themselves (3 and 4), whose tables leave room for eight and six warps per
+// multiprocessor with 16 entries (1,000,003 proteins at
+// identity 50, align: 9.28 ms as one tier of six, 8.96 so).
 __host__ __device__ constexpr int window_slots(int K, int tier) {
-  return K == 16 ? (tier == 0 ? 12 : tier == 1 ? 18 : 27) : (tier == 0 ? 16 : tier == 1 ? 24 : 36);
+  return K == 16 ? (tier == 0 ? 12 : tier == 2 ? 27 : tier == 3 ? 14 : 18)
+                 : (tier == 0 ? 16 : tier == 2 ? 36 : tier == 3 ? 18 : 24);
 }
 
 // The classes of a tier, widest first.
@@ -100,7 +104,7 @@ struct WindowClass {
   bool slide;
 };
 __host__ __device__ constexpr int window_classes(int K, int T) {
-  return T == 1 ? 10 : T == 0 ? 6 : widest_window(K) == 28 ? 6 : 5;
+  return T == 0 ? 6 : T == 1 ? 10 : T == 3 ? 6 : T == 4 ? 4 : widest_window(K) == 28 ? 6 : 5;
 }
 __host__ __device__ constexpr WindowClass window_class(int T, int k) {
   constexpr int w = kFirstWideClass, f = kFirstFixedClass;
@@ -112,7 +116,7 @@ __host__ __device__ constexpr WindowClass window_class(int T, int k) {
                                 {9, 5, true}};
   constexpr WindowClass t2[] = {{24, w + 2, true},  {24, f + 6, false}, {20, w + 1, true},
                                 {20, f + 5, false}, {18, w, true},      {28, w + 3, true}};
-  return T == 0 ? t0[k] : T == 1 ? t1[k] : t2[k];
+  return T == 0 ? t0[k] : T == 2 ? t2[k] : T == 3 ? t1[4 + k] : t1[k];
 }
 
 // The classes from `first` on (kFrom) or those before it, one after another.
@@ -191,12 +195,14 @@ int launch_align_k(int kernel, const RoundArgs &a, uint32_t m, cudaStream_t s) {
   switch (kernel) {
     case 0:
       return launch_round(align_wide_kernel<KC>, 32, (size_t)KC * 16 * 32 * 4, m, a, s);
-    case 1:
+    case 2:
       return launch_round(align_group_kernel<KC>, kGroupThreads, group_smem_bytes(6, KC), warps,
                           a, s);
-    case 2: return launch_round(align_window_kernel<K, 2>, 32, slots(2), lanes, a, s);
-    case 3: return launch_round(align_window_kernel<K, 1>, 32, slots(1), lanes, a, s);
-    case 4: return launch_round(align_window_kernel<K, 0>, 32, slots(0), lanes, a, s);
+    case 1: return launch_round(align_window_kernel<K, 2>, 32, slots(2), lanes, a, s);
+    case 3: return launch_round(align_window_kernel<K, 4>, 32, slots(4), lanes, a, s);
+    case 4: return launch_round(align_window_kernel<K, 3>, 32, slots(3), lanes, a, s);
+    case 5: return launch_round(align_window_kernel<K, 1>, 32, slots(1), lanes, a, s);
+    case 6: return launch_round(align_window_kernel<K, 0>, 32, slots(0), lanes, a, s);
     default: return NGIA_ERR_ARG;
   }
 }

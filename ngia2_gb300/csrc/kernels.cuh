@@ -88,10 +88,10 @@ int persistent_grid(const void *func, int threads, size_t smem, uint32_t want, u
 // of 0 .. kAlignKernels - 1 (independent of one another; each takes the pairs
 // of its classes through their cursors, zero before the launch).  m: the
 // round's pairs, an upper bound of any class's.
-constexpr int kAlignKernels = 5;
+constexpr int kAlignKernels = 7;
 // Whether a round of windows of at most `widest` words can have pairs for it.
 constexpr bool align_kernel_used(int kernel, uint32_t widest) {
-  return kernel != 2 || widest > 16;
+  return widest > 16 ? kernel != 5 : kernel != 1 && kernel != 3 && kernel != 4;
 }
 int launch_align(int kernel, const RoundArgs &a, int K, uint32_t m, cudaStream_t s);
 // All layouts of records offs[0..n) in one pass under an assumed code map

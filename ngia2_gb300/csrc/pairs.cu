@@ -278,8 +278,8 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 // ---- width classes ------------------------------------------------------------------
 // A pair's queue key (class_sort_key: its class, then its columns in octaves)
 // in a byte, the keys' histogram, and each pair's place in the queue by its
-// key's run.  The order inside a run is free, so two passes of atomics place
-// the pairs where a radix sort took three launches and moved the keys too.
+// key's run.  The order inside a run is free, so one pass of atomics places the
+// pairs where a radix sort took three launches and moved the keys too.
 constexpr uint32_t kClassifyUnroll = 4;
 
 __global__ void __launch_bounds__(256)
@@ -360,41 +360,56 @@ class_bounds_kernel(unsigned int *__restrict__ key_count, uint32_t *__restrict__
 }
 
 // Places the pairs by their keys: a block takes its keys' shares of their runs
-// with one atomic per key, its threads their places in those.
+// with one atomic per key.  Within a block the pairs keep their order, so that
+// the pairs a warp of the aligner takes together share targets, and reps near
+// each other, as they come from the candidates.
 constexpr uint32_t kPlacePairs = 16;  // per thread
+constexpr uint32_t kPlaceWarps = 8;
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kPlaceWarps * 32)
 place_kernel(const uint8_t *__restrict__ keys, uint32_t count,
              unsigned int *__restrict__ key_next, uint32_t *__restrict__ order) {
-  __shared__ unsigned int at[kQueueKeys];
-  at[threadIdx.x] = 0;
-  __syncthreads();
-  const uint32_t base = blockIdx.x * (256u * kPlacePairs);
-  const uint32_t lt_mask = (1u << (threadIdx.x & 31u)) - 1u;
-  uint32_t key[kPlacePairs];
+  static_assert(kPlaceWarps * 32 == kQueueKeys, "a thread per key");
+  __shared__ uint32_t at[kPlaceWarps][kQueueKeys];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  for (uint32_t k = lane; k < kQueueKeys; k += 32) at[warp][k] = 0;
+  __syncwarp();
+  const uint32_t base = (blockIdx.x * kPlaceWarps + warp) * (32u * kPlacePairs) + lane;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  uint32_t key[kPlacePairs], place[kPlacePairs];  // place: within the warp's share
 #pragma unroll
   for (uint32_t j = 0; j < kPlacePairs; ++j) {
-    const uint32_t p = base + j * 256u + threadIdx.x;
+    const uint32_t p = base + 32u * j;
     key[j] = p < count ? keys[p] : skip_sort_key();
   }
-  uint32_t place[kPlacePairs];  // within the block's share of the key
 #pragma unroll
   for (uint32_t j = 0; j < kPlacePairs; ++j) {
     const uint32_t peers = __match_any_sync(kFull, key[j]);
-    const uint32_t leader = __ffs(peers) - 1;
-    uint32_t first = 0;
-    if ((threadIdx.x & 31u) == leader) first = atomicAdd(&at[key[j]], (unsigned)__popc(peers));
-    place[j] = __shfl_sync(kFull, first, leader) + __popc(peers & lt_mask);
+    const uint32_t seen = at[warp][key[j]];
+    __syncwarp();
+    if ((peers & lt_mask) == 0) at[warp][key[j]] = seen + __popc(peers);
+    __syncwarp();
+    place[j] = seen + __popc(peers & lt_mask);
   }
   __syncthreads();
-  const unsigned int mine = at[threadIdx.x];
-  if (mine && threadIdx.x >> 3 != (uint32_t)kSkipClass)
-    at[threadIdx.x] = atomicAdd(&key_next[threadIdx.x], mine);
+  const uint32_t k = threadIdx.x;
+  if (k >> 3 != (uint32_t)kSkipClass) {
+    uint32_t mine = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kPlaceWarps; ++w) mine += at[w][k];
+    uint32_t next = mine ? atomicAdd(&key_next[k], mine) : 0u;
+#pragma unroll
+    for (uint32_t w = 0; w < kPlaceWarps; ++w) {
+      const uint32_t c = at[w][k];
+      at[w][k] = next;
+      next += c;
+    }
+  }
   __syncthreads();
 #pragma unroll
   for (uint32_t j = 0; j < kPlacePairs; ++j)
     if (key[j] >> 3 != (uint32_t)kSkipClass)
-      order[at[key[j]] + place[j]] = base + j * 256u + threadIdx.x;
+      order[at[warp][key[j]] + place[j]] = base + 32u * j;
 }
 
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
@@ -417,7 +432,7 @@ int place_pairs(const uint8_t *keys, uint32_t count, unsigned int *key_count, ui
   class_bounds_kernel<<<1, kQueueKeys, 0, s>>>(key_count, bounds);
   NGIA_LAUNCHED();
   if (count == 0) return NGIA_OK;
-  place_kernel<<<ceil_div(count, 256u * kPlacePairs), 256, 0, s>>>(keys, count, key_count, order);
+  place_kernel<<<ceil_div(count, kQueueKeys * kPlacePairs), kQueueKeys, 0, s>>>(keys, count, key_count, order);
   NGIA_LAUNCHED();
   return NGIA_OK;
 }
