@@ -278,12 +278,20 @@ int ctx_fast_cluster(ngia_ctx *c, uint32_t identity, uint32_t bands, uint32_t *h
   // a run per band costs 64 rounds (20,000 proteins, families of ten close
   // relatives, identity 90: 16.3 ms one band at a time through the
   // one-thread-per-pair kernel, 0.6 ms so).
-  const uint32_t most = (1u << 30) / n ? (1u << 30) / n : 1u;
+  // Where the device has no room for a run's pairs (8 bytes a slot, 9 more a
+  // pair) the run is halved, down to a band at a time.
+  uint32_t most = (1u << 30) / n ? (1u << 30) / n : 1u;
   for (uint32_t b0 = 0, b1; b0 < bands; b0 = b1) {
     const uint32_t end = b0 < 4 ? 4u : b0 < 16 ? 16u : (uint32_t)kBands;
     b1 = std::min(std::min(end, bands), b0 + most);
     NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
-    NGIA_TRY(c->pairs.reserve((size_t)(b1 - b0) * n * 8));
+    int room = c->pairs.reserve((size_t)(b1 - b0) * n * 8);
+    if (room == NGIA_ERR_NOMEM && b1 - b0 > 1) {
+      most = (b1 - b0) / 2;
+      b1 = b0;
+      continue;
+    }
+    NGIA_TRY(room);
     uint2 *pairs = c->pairs.as<uint2>();
     NGIA_TRY(collect_scan(rep + (size_t)b0 * n, c->lens.as<uint32_t>(), parent, n, b1 - b0,
                           identity, &dc->collect_ticket,
@@ -295,9 +303,16 @@ int ctx_fast_cluster(ngia_ctx *c, uint32_t identity, uint32_t bands, uint32_t *h
     if (hc.collect_error) return NGIA_ERR_CUDA;
     const uint32_t m = (uint32_t)hc.unique_total;
     if (m == 0) continue;
-    NGIA_TRY(c->scores.reserve((size_t)m * 4));
+    room = c->scores.reserve((size_t)m * 4);
+    if (room == NGIA_OK) room = c->round.reserve(m);
+    if (room == NGIA_ERR_NOMEM && b1 - b0 > 1) {
+      c->pairs.release();  // (a shorter run reserves less)
+      most = (b1 - b0) / 2;
+      b1 = b0;
+      continue;
+    }
+    NGIA_TRY(room);
     uint32_t *scores = c->scores.as<uint32_t>();
-    NGIA_TRY(c->round.reserve(m));
     NGIA_TRY(c->round.enqueue(db_view(c), pairs, m, identity, scores, nullptr));
     NGIA_TRY(fast_first_band(rep, n, b0, b1, pairs, scores, m, parent, s));
   }
