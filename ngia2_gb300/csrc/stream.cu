@@ -13,13 +13,14 @@
 // rows, candidates (distinct pairs grouped by target, the reference's length
 // filter).
 // Pass 2, align: pairs are keyed by (chunk of rep, chunk of target) -- rep
-// precedes target, so rep's chunk <= target's -- and sorted by that key.  For
-// each outer chunk a (resident in slot 0), the inner chunks b = a, a+1, ... are
-// streamed through slots 1 and 2 (b+1 is copied while the block (a, b) is
-// aligned); a block's pairs are renumbered into a two-chunk index space
-// (a's records, then b's) and aligned by one batched round.  Scores go back to
-// the pairs' own positions, so the emission (sorted unique edges) is the
-// resident path's.
+// precedes target, so rep's chunk <= target's -- and sorted by that key.  The
+// blocks of an outer chunk a follow one another, (a, a), (a, last), ... down to
+// (a, a + 1), whose chunk a + 1 is the next outer one and stays in its slot;
+// three slots hold chunks, so the next block's chunk is copied and laid out
+// while a block is aligned.  A block's pairs are renumbered into the slots'
+// record tables and aligned by one batched round.  Scores go back to the
+// pairs' own positions, so the emission (sorted unique edges) is the resident
+// path's.
 #include <chrono>
 #include <cstring>
 #include <thread>
@@ -63,26 +64,32 @@ block_key_kernel(const uint2 *__restrict__ pairs, uint32_t m,
   keys[p] = chunk_of(pr.x) * chunks + chunk_of(pr.y);
 }
 
-// A block's pairs in the region's numbering: records of chunk a are
-// 0..na-1, those of chunk b follow (for a == b, b's are a's).
+// A block's pairs in the region's numbering: the records of the rep's chunk a
+// from base_a on, those of the target's chunk b from base_b on (a == b: the
+// same).
 __global__ void __launch_bounds__(256)
 block_pairs_kernel(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ order,
-                   uint32_t begin, uint32_t cnt, uint32_t first_a, uint32_t na,
-                   uint32_t first_b, int same, uint2 *__restrict__ out) {
+                   uint32_t begin, uint32_t cnt, uint32_t first_a, uint32_t base_a,
+                   uint32_t first_b, uint32_t base_b, uint2 *__restrict__ out) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cnt) return;
   const uint2 pr = pairs[order[begin + k]];
-  const uint32_t x = pr.x - first_a;  // the rep is in chunk a
-  const uint32_t y = same ? pr.y - first_a : na + (pr.y - first_b);
-  out[k] = make_uint2(x, y);
+  out[k] = make_uint2(base_a + (pr.x - first_a), base_b + (pr.y - first_b));
 }
 
+// A block's scores to its pairs' places; its computed blocks and band cells
+// added to the running totals (rounds follow one another on the stream).
 __global__ void __launch_bounds__(256)
 scatter_block_scores_kernel(const uint32_t *__restrict__ order, uint32_t begin, uint32_t cnt,
                             const uint32_t *__restrict__ block_scores,
-                            uint32_t *__restrict__ scores) {
+                            uint32_t *__restrict__ scores, const Counters *__restrict__ rc,
+                            unsigned long long *__restrict__ acc) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < cnt) scores[order[begin + k]] = block_scores[k];
+  if (k == 0) {
+    acc[0] += rc->work;
+    acc[1] += rc->cells;
+  }
 }
 
 using SClock = std::chrono::steady_clock;
@@ -200,13 +207,6 @@ struct Stager {
   }
 };
 
-// Adds one round's computed blocks and band cells to running totals.
-__global__ void accumulate_kernel(const Counters *__restrict__ rc,
-                                  unsigned long long *__restrict__ acc) {
-  acc[0] += rc->work;
-  acc[1] += rc->cells;
-}
-
 struct StreamState {
   DevBuf region_packed, region_nib, region_dplanes, r_offs, r_lens;
   DevBuf offs, lens, sigs, rep, scratch, ucount, uoff, counters, pairs, scores,
@@ -214,17 +214,22 @@ struct StreamState {
       edges;
   Round round;
   Stager stager;
-  cudaStream_t s = nullptr;
+  cudaStream_t s = nullptr, lay = nullptr;  // rounds; the chunks' layouts
+  cudaEvent_t laid[Stager::kSlots] = {};    // a slot's layouts are written
   void destroy() {
     DevBuf *bufs[] = {&region_packed, &region_nib, &region_dplanes, &r_offs, &r_lens,
                       &offs,          &lens,       &sigs,         &rep,
                       &scratch,       &ucount,     &uoff,         &counters, &pairs,
                       &scores,        &keys,       &keys_sorted,  &order,   &block_pairs,
                       &block_scores,  &chunk_first, &presence,    &emit_tmp, &edges};
+    if (lay) cudaStreamSynchronize(lay);
     if (s) cudaStreamSynchronize(s);
     stager.destroy();
     round.destroy();
     for (DevBuf *b : bufs) b->release();
+    for (cudaEvent_t e : laid)
+      if (e) cudaEventDestroy(e);
+    if (lay) cudaStreamDestroy(lay);
     if (s) cudaStreamDestroy(s);
   }
 };
@@ -260,18 +265,21 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
 
   NGIA_CUDA(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
   cudaStream_t s = S.s;
+  NGIA_CUDA(cudaStreamCreateWithFlags(&S.lay, cudaStreamNonBlocking));
+  for (cudaEvent_t &e : S.laid) NGIA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   NGIA_TRY(S.round.init(s));
   NGIA_TRY(S.stager.init(h_packed, words, chunk_words));
   NGIA_TRY(S.region_packed.reserve(3 * chunk_words * 4));
   NGIA_TRY(S.region_nib.reserve(3 * chunk_words * 4));
-  NGIA_TRY(S.r_offs.reserve(2ull * max_recs * 8));
-  NGIA_TRY(S.r_lens.reserve(2ull * max_recs * 4));
+  NGIA_TRY(S.r_offs.reserve(3ull * max_recs * 8));
+  NGIA_TRY(S.r_lens.reserve(3ull * max_recs * 4));
   NGIA_TRY(S.offs.reserve((size_t)n * 8));
   NGIA_TRY(S.lens.reserve((size_t)n * 4));
   NGIA_TRY(S.sigs.reserve((size_t)bands * n * 4));
   NGIA_TRY(S.presence.reserve((size_t)C * 4 + 32));  // one word per chunk, then totals
   unsigned long long *acc =
       reinterpret_cast<unsigned long long *>(S.presence.as<uint32_t>() + ((C + 1) & ~1u));
+  NGIA_CUDA(cudaMemsetAsync(S.presence.p, 0, (size_t)C * 4 + 32, s));
   NGIA_TRY(S.counters.reserve(sizeof(Counters)));
   NGIA_CUDA(cudaMemcpyAsync(S.offs.p, h_offs, (size_t)n * 8, cudaMemcpyHostToDevice, s));
   NGIA_CUDA(cudaMemcpyAsync(S.lens.p, h_lens, (size_t)n * 4, cudaMemcpyHostToDevice, s));
@@ -287,26 +295,36 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
 
   // Loads chunk k into region slot `slot` (planes, and the nibble codes; once
   // the alphabet is known to be dense (pass 2) the recoded codes in their place
-  // and the code planes) with its record table at entries [at, at + count);
-  // the work is ordered on s.
+  // and the code planes) with its record table at entries [slot * max_recs, +
+  // count).  The layouts have a stream of their own, so that they run beside
+  // the kernels of the chunk before on s, which then waits for them; the copy
+  // waits until s has let the slot go.  What bounds the align pass: a slot's
+  // copy (42 us of 7.3 MB), its layouts and its block's round in turn, over two
+  // slots.  400,009 proteins, ten chunks: sketch pass 0.74 and align pass 3.5
+  // ms so; 0.87 and 5.0 ms with the layouts on s and the outer chunk loaded anew
+  // for each row of blocks.
   uint64_t map = 0;
   bool dense = false;
-  auto load_chunk = [&](uint32_t k, int slot, uint32_t at, uint32_t *presence) -> int {
+  auto load_chunk = [&](uint32_t k, int slot, uint32_t *presence) -> int {
     const Chunk &c = chunks[k];
     const uint64_t base = (uint64_t)slot * chunk_words;
+    const uint64_t at = (uint64_t)slot * max_recs;
     cudaEvent_t copied;
     NGIA_TRY(S.stager.stage(c, slot, rp + base, &copied));
-    NGIA_CUDA(cudaStreamWaitEvent(s, copied, 0));
-    region_table_kernel<<<ceil_div(c.count, 256u), 256, 0, s>>>(
-        S.offs.as<uint64_t>(), S.lens.as<uint32_t>(), c.first, c.count, c.word_first, base, at,
-        roffs, rlens);
+    NGIA_CUDA(cudaStreamWaitEvent(S.lay, S.stager.slot_done[slot], 0));
+    region_table_kernel<<<ceil_div(c.count, 256u), 256, 0, S.lay>>>(  // beside the copy
+        S.offs.as<uint64_t>(), S.lens.as<uint32_t>(), c.first, c.count, c.word_first, base,
+        (uint32_t)at, roffs, rlens);
     NGIA_LAUNCHED();
+    NGIA_CUDA(cudaStreamWaitEvent(S.lay, copied, 0));
     if (dense)
       NGIA_TRY(launch_dense_layouts(rp, roffs + at, c.count, map, rn,
-                                    S.region_dplanes.as<uint32_t>(), s));
+                                    S.region_dplanes.as<uint32_t>(), S.lay));
     else
       NGIA_TRY(launch_nibbles(rp, roffs + at, rlens + at, c.count, base + chunk_words, rn,
-                              presence, s));
+                              presence, S.lay, /*accumulate=*/true));
+    NGIA_CUDA(cudaEventRecord(S.laid[slot], S.lay));
+    NGIA_CUDA(cudaStreamWaitEvent(s, S.laid[slot], 0));
     return NGIA_OK;
   };
 
@@ -315,8 +333,8 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
   uint32_t present = 0;
   for (uint32_t k = 0; k < C; ++k) {
     const int slot = (int)(k & 1u);
-    NGIA_TRY(load_chunk(k, slot, 0, S.presence.as<uint32_t>() + k));
-    NGIA_TRY(launch_sketch_nibbles(rn, roffs, chunks[k].count,
+    NGIA_TRY(load_chunk(k, slot, S.presence.as<uint32_t>() + k));
+    NGIA_TRY(launch_sketch_nibbles(rn, roffs + (uint64_t)slot * max_recs, chunks[k].count,
                                    S.sigs.as<uint32_t>() + chunks[k].first, n, bands, s));
     NGIA_TRY(S.stager.slot_free(slot, s));
   }
@@ -413,39 +431,48 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
   const DbView view{rp, rn, ab, roffs, rlens};
   NGIA_CUDA(cudaMemsetAsync(acc, 0, 16, s));
   uint64_t loads = 0;
-  int inner = 1;  // slot of the current inner chunk (1 and 2 alternate)
+  // The slots hold three chunks.  A row of blocks (one outer chunk a) runs from
+  // its own block over the last chunk down to a + 1, which is then the next
+  // row's outer chunk and stays where it is.
+  uint32_t held[Stager::kSlots], used[Stager::kSlots] = {}, turn = 0;
+  for (uint32_t &h : held) h = kFull;
+  auto slot_of = [&](uint32_t k, int keep, int *slot) -> int {
+    int at = -1;
+    for (int q = 0; q < Stager::kSlots; ++q)
+      if (held[q] == k) at = q;
+    if (at < 0) {  // into the slot that was read longest ago
+      for (int q = 0; q < Stager::kSlots; ++q)
+        if (q != keep && (at < 0 || used[q] < used[at])) at = q;
+      NGIA_TRY(load_chunk(k, at, S.presence.as<uint32_t>()));
+      held[at] = k;
+      ++loads;
+    }
+    used[at] = ++turn;
+    *slot = at;
+    return NGIA_OK;
+  };
   for (uint32_t a = 0; a < C; ++a) {
-    bool a_loaded = false;
-    for (uint32_t b = a; b < C; ++b) {
+    for (uint32_t j = 0; j < C - a; ++j) {
+      const uint32_t b = j == 0 ? a : C - j;
       const size_t blk = (size_t)a * C + b;
       const uint32_t beg = block_begin[blk], cnt = block_begin[blk + 1] - beg;
       if (cnt == 0) continue;
-      if (!a_loaded) {
-        NGIA_TRY(load_chunk(a, 0, 0, S.presence.as<uint32_t>()));
-        a_loaded = true;
-        ++loads;
-      }
-      const bool same = a == b;
-      if (!same) {
-        // the other inner slot: its copy overlaps the block still using this one
-        inner = inner == 1 ? 2 : 1;
-        NGIA_TRY(load_chunk(b, inner, chunks[a].count, S.presence.as<uint32_t>()));
-        ++loads;
-      }
+      int sa, sb;
+      NGIA_TRY(slot_of(a, -1, &sa));
+      NGIA_TRY(slot_of(b, sa, &sb));
       block_pairs_kernel<<<ceil_div(cnt, 256u), 256, 0, s>>>(
           S.pairs.as<uint2>(), S.order.as<uint32_t>(), beg, cnt, chunks[a].first,
-          chunks[a].count, chunks[b].first, same ? 1 : 0, S.block_pairs.as<uint2>());
+          (uint32_t)sa * max_recs, chunks[b].first, (uint32_t)sb * max_recs,
+          S.block_pairs.as<uint2>());
       NGIA_LAUNCHED();
       NGIA_TRY(S.round.enqueue(view, S.block_pairs.as<uint2>(), cnt, identity,
                                S.block_scores.as<uint32_t>(), nullptr));
       scatter_block_scores_kernel<<<ceil_div(cnt, 256u), 256, 0, s>>>(
           S.order.as<uint32_t>(), beg, cnt, S.block_scores.as<uint32_t>(),
-          S.scores.as<uint32_t>());
+          S.scores.as<uint32_t>(), S.round.counters(), acc);
       NGIA_LAUNCHED();
-      accumulate_kernel<<<1, 1, 0, s>>>(S.round.counters(), acc);  // before the next round
-      NGIA_LAUNCHED();
-      NGIA_TRY(S.stager.slot_free(0, s));
-      if (!same) NGIA_TRY(S.stager.slot_free(inner, s));
+      NGIA_TRY(S.stager.slot_free(sa, s));
+      if (sb != sa) NGIA_TRY(S.stager.slot_free(sb, s));
     }
   }
   unsigned long long totals[2] = {0, 0};
