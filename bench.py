@@ -66,7 +66,7 @@ SKETCH_ALU_OPS_PER_HASH = 10
 # to a full launch by the units it processes (both grow in proportion).
 SKETCH_DRAM_BYTES_PER_POSITION = 0.553
 SKETCH_TABLE_DRAM_BYTES_PER_POSITION = 0.537  # sketch_rank_kernel, per signed position
-ALIGN_DRAM_BYTES_PER_CELL = 1.13e-3  # all width classes of one step (profiles/align_*)
+ALIGN_DRAM_BYTES_PER_CELL = 4.83e-3  # the align kernels of one step (profiles/align_phase_*)
 # The reference's host code clusters about 650 families (6,500 sequences) of
 # this generator per second on 16 Grace cores; samples are sized from that.
 CPU_FAMILIES_PER_S = 650
@@ -487,7 +487,7 @@ def run_ours(args, world, rank, local, pg):
                            "signed_positions", SKETCH_DRAM_BYTES_PER_POSITION, sketch_bytes, 1)
     rs = {
         "sketch": sketch_roof,
-        # the align phase: one launch per populated width class, timed as a whole
+        # the align phase: its concurrent launches, timed as a whole
         "align": align_roof(roof, cells, align_ms, int_peak,
                             st["unique_pairs"] * 12 + int(db["lens"].sum()) / 2),
     }
@@ -561,8 +561,8 @@ def align_roof(roof, cells, align_ms, int_peak, algo_bytes) -> dict:
     """The align phase against the integer-logic peak, with both op counts per
     32 cells: 3 (the update's irreducible ops) and 5 (each of AND, add with
     carry in, carry out, AND-NOT, OR counted)."""
-    r = roof("align phase (align_stream_kernel / align_group_kernel / align_general_kernel "
-             "per width class)", cells / 32 * ALIGN_OPS_PER_WORD_STEP, align_ms, cells,
+    r = roof("align phase (align_window_kernel per tier of widths / align_group_kernel / "
+             "align_wide_kernel)", cells / 32 * ALIGN_OPS_PER_WORD_STEP, align_ms, cells,
              "computed_cells", ALIGN_DRAM_BYTES_PER_CELL, algo_bytes, 1)
     ops5 = cells / 32 * ALIGN_OPS_PER_WORD_STEP_5
     r["ops_per_word_step"] = ALIGN_OPS_PER_WORD_STEP
@@ -580,7 +580,7 @@ def hbm_rooflines(stats, st, n, hbm) -> dict:
             ("bucket", "ms_bucket", 8 * BANDS * n,
              "rs_hist/rs_scatter (segmented radix partition) + rep_resolve_kernel / rep_resolve_far_kernel"),
             ("emit", "ms_emit", 12 * st["unique_pairs"] + 12 * st["edges"],
-             "emit_sorted (run counts, ordered compaction, radix sort by rep)")):
+             "emission (few hits: append_hits_kernel / emit_hits_kernel; else emit_sorted)")):
         ms = statistics.mean(s[ms_key] for s in stats)
         achieved = algo / (ms * 1e-3) if ms > 0 else 0.0
         out[name] = {"bound": "hbm", "kernel": kernel, "achieved": achieved / 1e9,

@@ -86,8 +86,9 @@ int ngia_sketch(const uint32_t *d_packed, const uint64_t *d_rec_offsets,
 /* ---- stage (b): bucket --------------------------------------------------------
  * Rep rows from band-major signatures: d_rep[b*n + i] for b < bands.
  * Replaces MakeDB::groupSignatures (src/makedb.hpp:289-364): a stable radix
- * sort of (sig, idx) per band and the predecessor chain.  Scratch: about
- * 16 * bands * n bytes from the stream-ordered allocator. */
+ * sort of (sig, idx) per band and the predecessor chain.  Scratch: none up to
+ * 4,096 records, beyond that about 16 * bands * n bytes from the
+ * stream-ordered allocator. */
 int ngia_bucket(const uint32_t *d_sigs, uint32_t n, uint32_t bands,
                 uint32_t *d_rep, void *stream);
 
@@ -258,11 +259,11 @@ int ngia_ctx_autotune(ngia_ctx *ctx, const uint32_t *d_pairs, uint32_t count,
                       uint32_t identity, int reps, ngia_plan *best, double *best_ms);
 
 /* Whether ngia_ctx_align_pairs captures its round (classification, queue
- * sort and every class launch) as a CUDA graph and replays it while the
+ * order and the class launches) as a CUDA graph and replays it while the
  * pair/score addresses, count, identity, rounding, plan and the loaded
  * database (its buffers and alphabet) stay the same, and whether the
- * bucketing of every graph build is replayed the same way while its buffers,
- * record count and bands stay the same (default on).  Returns the previous
+ * bucketing of every graph build of more than 4,096 records is replayed the
+ * same way while its buffers, record count and bands stay the same (default on).  Returns the previous
  * setting (0/1), or NGIA_ERR_ARG. */
 int ngia_ctx_use_graphs(ngia_ctx *ctx, int on);
 
@@ -379,7 +380,9 @@ void ngia_server_destroy(ngia_server *srv);
 
 /* Fast greedy clustering (src/fastClustering.hpp:249-352): per band, targets
  * not yet assigned are aligned against their rep and assigned on a hit;
- * h_cluster[i] = root index.  Synchronises. */
+ * h_cluster[i] = root index.  Bands are aligned in runs and assigned in band
+ * order; up to 8 bytes per record and band of a run, shorter runs where the
+ * device has not that much.  Synchronises. */
 int ngia_ctx_fast_cluster(ngia_ctx *ctx, uint32_t identity, uint32_t bands,
                           uint32_t *h_cluster, ngia_stats *stats);
 
