@@ -8,16 +8,16 @@
 //   with H Wang's 32-bit integer hash followed by two extra xor-shift-multiply
 //   rounds (the steps below), minimum 0xFFFFFFFF when nothing is signed.
 //
-// Mapping: one warp per record; each lane signs a contiguous run of the
-// positions and keeps all 64 running minima in registers (64 independent
-// hash chains per position), then one redux.sync min per band combines the
-// lanes.  Records are in length-descending index order, so the longest are
-// scheduled first.
+// Mapping: one warp per record, two bands per lane (sketch_kernel); few records
+// or few bands take runs of bands, each lane a run of the positions
+// (sketch_bands_kernel).  Records are in length-descending index order, so the
+// longest are scheduled first.
 //
 // The work is integer-bound: 64 hashes of 13 integer instructions per
 // position against half a byte read.  On this GPU the logic/shift pipe and
 // the integer multiply-add pipe draw on the same integer issue budget, and a
 // multiply-high costs two of its slots, so the shifts stay shifts.
+#include "align_lds.cuh"
 #include "kernels.cuh"
 
 namespace ngia {
@@ -47,6 +47,15 @@ struct PlaneKmers {
     PlaneKmers k;
     k.rec = r;
     return k;
+  }
+  // code word w of a record: residues 8w..8w+7, the first in the high nibble
+  __device__ static __forceinline__ uint32_t word(const uint32_t *r, uint32_t w) {
+    const uint32_t *b = r + 1 + 4 * (w >> 2);
+    uint32_t out = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      out |= spread8((__brev(__ldg(b + e)) >> (24 - 8 * (w & 3u))) & 0xFFu) << e;
+    return out;
   }
   uint32_t block = 0xFFFFFFFFu;
   uint32_t p0 = 0, p1 = 0, p2 = 0, p3 = 0;
@@ -81,6 +90,9 @@ struct PlaneKmers {
 struct NibbleKmers {
   const uint32_t *nib;  // the record's first code word
   __device__ static NibbleKmers make(const uint32_t *r) { return NibbleKmers{r + 1}; }
+  __device__ static __forceinline__ uint32_t word(const uint32_t *r, uint32_t w) {
+    return __ldg(r + 1 + w);
+  }
   __device__ __forceinline__ void start(uint32_t) {}
   __device__ __forceinline__ uint32_t at(uint32_t p) {
     if (p < 7) return __ldg(nib) >> (28 - 4 * p);  // short record: codes 0..p
@@ -90,43 +102,75 @@ struct NibbleKmers {
   }
 };
 
+// All 64 bands of a record by one warp, bands `lane` and `lane + 32` in each
+// lane, every lane over all positions.  A tile of 256 positions at a time: the
+// lanes load (or make) its code words, turn them into the positions' folded
+// k-mers in shared memory, and then all read the same four k-mers per 16-byte
+// load and hash them for their own bands.
+//
+// What bounds it: the logic pipe, ten operations a hash.  The positions are
+// hashed as many times as there are, up to three more at a record's end, and
+// nothing is combined across lanes; with a run of the positions per lane and
+// all 64 minima in its registers a record of 333 positions took 352 (eleven in
+// each lane), 64 reductions, and left room for 16 warps per multiprocessor:
+// 20,000 proteins of 340 residues on average 244 us, so 234 (1.82e12 hashes/s;
+// 1.97e12 without loads and tails).  A block per four records, not a grid that
+// loops: the blocks follow one another as they end, longest first.  1, 2, 4, 8
+// warps a block: 4,800 records 82, 82, 82, 103 us (eight of the longest on one
+// multiprocessor), 20,000 242, 238, 234, 236.
+constexpr uint32_t kSketchWarps = 4;  // per block
+constexpr uint32_t kSketchTile = 256;
+
 template <typename Source>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kSketchWarps * 32)
 sketch_kernel(const uint32_t *__restrict__ words, const uint64_t *__restrict__ offs,
               uint32_t n, uint32_t *__restrict__ sigs) {
+  __shared__ __align__(16) uint32_t kmers[kSketchWarps][kSketchTile];
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+  uint32_t *km = kmers[threadIdx.x >> 5];
+  const uint4 *km4 = reinterpret_cast<const uint4 *>(km);
+  const uint32_t fold0 = band_seed_fold(lane), fold1 = band_seed_fold(lane + 32);
+  const uint32_t i = blockIdx.x * kSketchWarps + (threadIdx.x >> 5);
+  if (i < n) {
     const uint32_t *rec = words + offs[i];
     const uint32_t len = __ldg(rec);
-    const uint32_t first = len >= 8 ? 7u : (len > 0 ? len - 1 : 0u);
-    const uint32_t span = len - first;  // signed positions
-    const uint32_t per = (span + 31u) >> 5;
-    const uint32_t pb = first + lane * per;
-    const uint32_t pe = min(pb + per, len);
-
-    uint32_t mn[kBands];
-#pragma unroll
-    for (int k = 0; k < kBands; ++k) mn[k] = kFull;
-
-    if (pb < pe) {
-      Source src = Source::make(rec);
-      src.start(pb);
-      for (uint32_t p = pb; p < pe; ++p) {
-        const uint32_t kmer = src.at(p);
-        const uint32_t y = kmer ^ (kmer >> 16);
-#pragma unroll
-        for (int k = 0; k < kBands; ++k)
-          mn[k] = min(mn[k], band_hash_tail(y ^ band_seed_fold((uint32_t)k)));
-      }
-    }
+    const uint32_t nw = (len + 7u) >> 3;  // code words
+    const uint32_t span = len >= 8 ? len - 7 : (len ? 1u : 0u);  // signed positions
     uint32_t lo = kFull, hi = kFull;
+    for (uint32_t s0 = 0; s0 < span; s0 += kSketchTile) {
+      const uint32_t cnt = min(span - s0, kSketchTile);
+      const uint32_t w0 = s0 >> 3;
+      const uint32_t mine = w0 + lane < nw ? Source::word(rec, w0 + lane) : 0u;
+      uint32_t after = w0 + 32 < nw ? Source::word(rec, w0 + 32) : 0u;
+      const uint32_t next = __shfl_down_sync(kFull, mine, 1);
+      if (lane < 31) after = next;
+      // the lane's eight windows: the k-mer of window r starts at its residue r
+      // (a record of fewer than eight residues has one, of all of them)
+      __syncwarp();
 #pragma unroll
-    for (int k = 0; k < kBands; ++k) {
-      const uint32_t r = __reduce_min_sync(kFull, mn[k]);
-      if ((uint32_t)(k & 31) == lane) {
-        if (k < 32) lo = r;
-        else hi = r;
+      for (uint32_t r = 0; r < 8; ++r) {
+        uint32_t k = __funnelshift_l(after, mine, 4 * r);
+        if (len < 8) k = mine >> (4 * (8 - len));
+        k ^= k >> 16;
+        const uint32_t q = 8 * lane + r;
+        if (q < cnt) km[q] = k;
+        // the last group of four filled up with the last k-mer
+        if (q == cnt - 1)
+          for (uint32_t f = cnt; f & 3u; ++f) km[f] = k;
+      }
+      __syncwarp();
+      const uint32_t groups = (cnt + 3) >> 2;
+#pragma unroll 2
+      for (uint32_t g = 0; g < groups; ++g) {
+        const uint4 y = km4[g];
+        lo = min(lo, band_hash_tail(y.x ^ fold0));
+        hi = min(hi, band_hash_tail(y.x ^ fold1));
+        lo = min(lo, band_hash_tail(y.y ^ fold0));
+        hi = min(hi, band_hash_tail(y.y ^ fold1));
+        lo = min(lo, band_hash_tail(y.z ^ fold0));
+        hi = min(hi, band_hash_tail(y.z ^ fold1));
+        lo = min(lo, band_hash_tail(y.w ^ fold0));
+        hi = min(hi, band_hash_tail(y.w ^ fold1));
       }
     }
     sigs[(size_t)lane * n + i] = lo;
@@ -199,11 +243,10 @@ static int launch(const uint32_t *words, const uint64_t *offs, uint32_t n, uint3
   // Fewer bands than the file's 64 are hashed as such (400,009 proteins, 3
   // bands: 0.23 ms where 64 take 4.8).  All 64 of few records are split over
   // warps: a warp that hashes 64 bands of a record of 340 takes 8,300
-  // instructions by itself, and fewer records than the device holds warps (16
-  // per multiprocessor with 64 minima each) leave it waiting for that.  64, 16
-  // and 8 bands a warp, proteins: 200 records 35, 13.6, 12.6 us; 600: 35, 20.8,
-  // 20.6; 2,400: 62, 49, 54; 4,800: 82, 87, 92 (every run of bands rolls the
-  // k-mers again).
+  // instructions by itself, and fewer records than keep the device busy leave it
+  // waiting for that.  Proteins, 16 and 8 bands a warp: 200 records 13.6, 12.6
+  // us; 600: 20.8, 20.6; 2,400: 49, 54; 4,800: 87, 92 (every run of bands rolls
+  // the k-mers again); all 64 a warp: 2,433 51 us, 4,800 82.
   if (bands <= 4) return launch_bands<Source, 4>(words, offs, n, sigs, stride, bands, cap, s);
   if (bands <= 8 || n <= (uint32_t)sms * 2u)
     return launch_bands<Source, 8>(words, offs, n, sigs, stride, bands, cap, s);
@@ -211,8 +254,7 @@ static int launch(const uint32_t *words, const uint64_t *offs, uint32_t n, uint3
     return launch_bands<Source, 16>(words, offs, n, sigs, stride, bands, cap, s);
   if (bands < (uint32_t)kBands || stride != n)
     return launch_bands<Source, 32>(words, offs, n, sigs, stride, bands, cap, s);
-  const uint32_t want = ceil_div(n, 8u);  // 8 warps per block
-  sketch_kernel<Source><<<want < cap ? want : cap, 256, 0, s>>>(words, offs, n, sigs);
+  sketch_kernel<Source><<<ceil_div(n, kSketchWarps), kSketchWarps * 32, 0, s>>>(words, offs, n, sigs);
   NGIA_LAUNCHED();
   return NGIA_OK;
 }
