@@ -102,7 +102,7 @@ struct NibbleKmers {
   }
 };
 
-// All 64 bands of a record by one warp, bands `lane` and `lane + 32` in each
+// More than 32 bands of a record by one warp, bands `lane` and `lane + 32` in each
 // lane, every lane over all positions.  A tile of 256 positions at a time: the
 // lanes load (or make) its code words, turn them into the positions' folded
 // k-mers in shared memory, and then all read the same four k-mers per 16-byte
@@ -124,7 +124,7 @@ constexpr uint32_t kSketchTile = 256;
 template <typename Source>
 __global__ void __launch_bounds__(kSketchWarps * 32)
 sketch_kernel(const uint32_t *__restrict__ words, const uint64_t *__restrict__ offs,
-              uint32_t n, uint32_t *__restrict__ sigs) {
+              uint32_t n, uint32_t *__restrict__ sigs, size_t stride, uint32_t bands) {
   __shared__ __align__(16) uint32_t kmers[kSketchWarps][kSketchTile];
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t *km = kmers[threadIdx.x >> 5];
@@ -173,8 +173,8 @@ sketch_kernel(const uint32_t *__restrict__ words, const uint64_t *__restrict__ o
         hi = min(hi, band_hash_tail(y.w ^ fold1));
       }
     }
-    sigs[(size_t)lane * n + i] = lo;
-    sigs[(size_t)(lane + 32) * n + i] = hi;
+    if (lane < bands) sigs[lane * stride + i] = lo;
+    if (lane + 32 < bands) sigs[(lane + 32) * stride + i] = hi;
   }
 }
 
@@ -246,15 +246,16 @@ static int launch(const uint32_t *words, const uint64_t *offs, uint32_t n, uint3
   // instructions by itself, and fewer records than keep the device busy leave it
   // waiting for that.  Proteins, 16 and 8 bands a warp: 200 records 13.6, 12.6
   // us; 600: 20.8, 20.6; 2,400: 49, 54; 4,800: 87, 92 (every run of bands rolls
-  // the k-mers again); all 64 a warp: 2,433 51 us, 4,800 82.
+  // the k-mers again); all 64 a warp: 2,433 51 us, 4,800 82.  More than 32 bands
+  // of many records are hashed as 64 (33 bands of 200,003 streamed proteins,
+  // sketch pass: 2.83 ms in two runs of 32, 2.40 so).
   if (bands <= 4) return launch_bands<Source, 4>(words, offs, n, sigs, stride, bands, cap, s);
   if (bands <= 8 || n <= (uint32_t)sms * 2u)
     return launch_bands<Source, 8>(words, offs, n, sigs, stride, bands, cap, s);
   if (bands <= 32 || n <= (uint32_t)sms * 16u)
     return launch_bands<Source, 16>(words, offs, n, sigs, stride, bands, cap, s);
-  if (bands < (uint32_t)kBands || stride != n)
-    return launch_bands<Source, 32>(words, offs, n, sigs, stride, bands, cap, s);
-  sketch_kernel<Source><<<ceil_div(n, kSketchWarps), kSketchWarps * 32, 0, s>>>(words, offs, n, sigs);
+  sketch_kernel<Source><<<ceil_div(n, kSketchWarps), kSketchWarps * 32, 0, s>>>(
+      words, offs, n, sigs, stride, bands);
   NGIA_LAUNCHED();
   return NGIA_OK;
 }

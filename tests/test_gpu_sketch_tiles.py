@@ -37,3 +37,20 @@ def test_sketch_at_tile_edges_matches_oracle(cuda, built, alphabet):
         ctx.load(packed, offs, lens)
         ctx.sketch_bucket(64)
         assert np.array_equal(ctx.sigs(), want)
+
+
+@pytest.mark.parametrize("bands", [33, 63, 64])
+def test_streamed_chunks_of_many_bands(cuda, built, bands):
+    """More than 32 bands of chunks of more than 2,432 records, whose rows are
+    further apart than the chunk is long."""
+    from gpu_util import build_db
+    s = synth.families(9_000, 900, synth.AMINO, synth.AMINO_FREQ,
+                       synth._lognormal_roots(40, 0.3, 8, 90), 0.0, 0.2, 0.01, 2.0, 91)
+    packed, offs, lens = build_db([s.seq(int(i)) for i in np.argsort(-s.lens, kind="stable")])
+    got, st = ng.stream_graph(packed, offs, lens, 60, bands, 36 * (len(packed) // 3 + 400))
+    with ng.Context() as ctx:
+        ctx.load(packed, offs, lens)
+        m, rst = ctx.group_align(60, bands)
+        want = ctx.edges(m)
+    assert 2 <= st["chunks"] <= 3 and len(want) > 0
+    assert np.array_equal(got, want) and st["unique_pairs"] == rst["unique_pairs"]
