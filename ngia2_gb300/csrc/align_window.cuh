@@ -283,8 +283,10 @@ __device__ __forceinline__ uint32_t align_window(const RoundArgs &a, int cls, ui
       if (mine) {
         sp.lr = len & 0xFFFFu;
         sp.lt = len >> 16;
-        if (sp.lt == 0) {
-          a.scores[p] = identity_score(0u, sp.lr, 0u, a.t);
+        // no columns, or no row to enter the window (a sliding window's words
+        // below row 0 assume one does)
+        if (sp.lt == 0 || sp.lr == 0) {
+          a.scores[p] = identity_score(0u, sp.lr, sp.lt, a.t);
         } else {
           sp.rep = a.rows + ro;
           sp.tar = a.nib + to + 1;
