@@ -135,7 +135,8 @@ int ctx_sketch_bucket(ngia_ctx *c, uint32_t bands, ngia_stats *st, bool sketch_d
 }
 
 int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_n_edges,
-                    ngia_stats *st, uint32_t part, uint32_t parts, uint64_t *h_range) {
+                    ngia_stats *st, uint32_t part, uint32_t parts, uint64_t *h_range,
+                    bool *load_stands) {
   if (c->n == 0 || c->rep_bands == 0) return NGIA_ERR_STATE;
   if (identity < 1 || identity > 99) return NGIA_ERR_ARG;
   if (bands < 1 || bands > c->rep_bands) return NGIA_ERR_ARG;
@@ -164,6 +165,10 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   Counters &hc = c->h_counters->pairs;
   NGIA_CUDA(cudaMemcpyAsync(&hc, dc, sizeof(Counters), cudaMemcpyDeviceToHost, s));
   NGIA_CUDA(cudaStreamSynchronize(s));
+  if (load_stands) {
+    *load_stands = *c->h_flag == 0;
+    if (!*load_stands) return NGIA_OK;
+  }
   if (hc.collect_error) return NGIA_ERR_CUDA;  // a look-back gave up (never seen)
   const uint64_t total = hc.unique_total;
   if (total > 0xFFFFFFFFull) return NGIA_ERR_NOMEM;  // beyond one launch's index range
@@ -501,8 +506,8 @@ int makedb_device(ngia_ctx *c, Makedb &m) {
 // has been seen; the pipeline assumes the previous load's map (its sketch
 // tables are cached) and checks that every residue's code is one of the map's
 // and every record lay inside its piece (offsets in order); the check's
-// result lands in *c->h_flag (nonzero: the caller discards the step and loads
-// as usual) once the stream passes it.  Runs only when that map takes the
+// result lands in *c->h_flag once the stream passes it (nonzero: the step is
+// discarded before anything is aligned, and the caller loads as usual).  Runs only when that map takes the
 // table sketch.  *used = false: nothing was done (the caller loads as usual);
 // else the load and the signatures are in place, subject to the check.
 int ctx_load_sketch(ngia_ctx *c, const uint32_t *h_packed, uint64_t words,
@@ -608,11 +613,14 @@ int ctx_load_sketch(ngia_ctx *c, const uint32_t *h_packed, uint64_t words,
   NGIA_CUDA(cudaStreamWaitEvent(s, c->ev[7], 0));
   NGIA_CUDA(cudaEventRecord(c->ev[9], s));
   // a code outside the map, or a record outside its piece: copied to
-  // *h_flag and read by the caller after the step's next synchronisation,
-  // without a host round trip here.  Until then the step goes on as if the map serves (the
-  // layouts of such records hold in-range codes, so the work on them is
-  // wasted, never out of bounds); if the check fails, the caller starts over
-  // with the plain load.
+  // *h_flag and read after the step's next synchronisation (the graph build's,
+  // for its pair count), without a host round trip here.  Until then the step
+  // goes on as if the map serves, with kernels that stay in bounds whatever
+  // the layouts of such records hold: the sketch, the bucketing and the
+  // candidates.  The aligners do not -- they take lengths from lens[] and index
+  // their tables by the codes, and a record laid out empty has whatever an
+  // earlier database left behind its length word -- so no round is enqueued
+  // before the flag has been read.
   *c->h_flag = 0;
   NGIA_CUDA(cudaMemcpyAsync(c->h_flag, c->presence.p, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                             s));
@@ -980,25 +988,32 @@ int ngia_ctx_run_host(ngia_ctx *c, const uint32_t *h_packed, uint64_t packed_wor
     NGIA_TRY(ngia::ctx_load_sketch(c, h_packed, packed_words, h_rec_offsets, h_lens, n, &piped,
                                    &sketched));
   if (piped) {
-    // no synchronisation until the graph build needs its pair count; the
-    // pieced load's code-map check is read after the build
-    NGIA_TRY(ngia::ctx_sketch_bucket(c, bands, stats, true, true));
+    // no synchronisation until the graph build needs its pair count, where it
+    // also reads the pieced load's check
+    int rc = ngia::ctx_sketch_bucket(c, bands, stats, true, true);
     // the host check of every record, while the device sketches and buckets
     // (nothing launched so far trusts the offsets; the candidates do)
-    if (!ngia::records_inside(h_rec_offsets, h_lens, n, packed_words)) {
+    const bool inside = ngia::records_inside(h_rec_offsets, h_lens, n, packed_words);
+    if (rc == NGIA_OK && !inside) rc = NGIA_ERR_ARG;
+    bool stands = false;  // the map served every record
+    if (rc == NGIA_OK)
+      rc = ngia::ctx_build_graph(c, identity, bands, h_n_edges, stats, 0, 1, nullptr, &stands);
+    if (!stands) {
       cudaStreamSynchronize(c->copy);  // the caller's buffers stay in use until then
       cudaStreamSynchronize(c->layout);
       cudaStreamSynchronize(c->side);
-      NGIA_CUDA(cudaStreamSynchronize(c->stream));
-      c->n = 0;  // the copies overwrote the resident records: no database until a load
-      c->packed_words = 0;
-      c->sigs_valid = false;
-      c->rep_bands = 0;
-      c->n_edges = 0;
-      return NGIA_ERR_ARG;
+      const cudaError_t e = cudaStreamSynchronize(c->stream);
+      if (e != cudaSuccess || !inside || *c->h_flag != 0) {
+        c->n = 0;  // the copies overwrote the resident records: no database until a load
+        c->packed_words = 0;
+        c->sigs_valid = false;
+        c->rep_bands = 0;
+        c->n_edges = 0;
+      }
+      NGIA_CUDA(e);
     }
-    NGIA_TRY(ngia::ctx_build_graph(c, identity, bands, h_n_edges, stats));
-    if (*c->h_flag == 0) {  // the map served every record: the step stands
+    if (rc != NGIA_OK) return rc;
+    if (stands) {
       if (stats) {
         ngia::ctx_stage_stats(c, stats);
         stats->load_pipelined = 1u;

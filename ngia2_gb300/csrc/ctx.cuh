@@ -84,7 +84,9 @@ int ctx_load_text(ngia_ctx *c, const char *h_text, uint64_t text_bytes,
                   uint32_t n, uint64_t words);
 // parts > 1: only the part-th share of the distinct pairs by band cells is
 // aligned and emitted; h_range (optional) receives its [first, end).
+// load_stands (optional): after a pieced load, receives whether its check
+// passed, read once the pair count is there; if not, nothing is aligned.
 int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_n_edges,
                     ngia_stats *st, uint32_t part = 0, uint32_t parts = 1,
-                    uint64_t *h_range = nullptr);
+                    uint64_t *h_range = nullptr, bool *load_stands = nullptr);
 }  // namespace ngia
