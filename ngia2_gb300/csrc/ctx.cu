@@ -592,7 +592,9 @@ int ctx_load_sketch(ngia_ctx *c, const uint32_t *h_packed, uint64_t words,
     const uint32_t r0 = first[k], cnt = first[k + 1] - first[k];
     NGIA_CUDA(cudaStreamWaitEvent(c->layout, c->chunk_ev[k], 0));
     if (cnt) {
-      const uint64_t w0 = bound(k), w1 = bound(k + 1);
+      // (offsets out of order may end a piece before its start: an empty one,
+      // whose records are flagged)
+      const uint64_t w0 = bound(k), w1 = std::max(w0, bound(k + 1));
       NGIA_TRY(launch_load_layouts(packed, offs + r0, c->lens.as<uint32_t>() + r0, cnt, w0, w1,
                                    words, spec.inv, c->nib_dense.as<uint32_t>(),
                                    c->dplanes.as<uint32_t>(), c->presence.as<uint32_t>(),

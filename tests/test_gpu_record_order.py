@@ -48,6 +48,21 @@ def test_offsets_out_of_order(cuda, built):
         assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("name", ["reversed", "rotated", "random"])
+def test_any_order_is_served(cuda, built, name):
+    """Whatever the order: the pieces' bounds are looked up as if the offsets
+    ascended, and may then not ascend themselves (random order)."""
+    db = dna(12_000, 1_200, 64)
+    n = len(db[2])
+    want = resident_edges(db, 90)
+    order = {"reversed": np.arange(n)[::-1], "rotated": np.roll(np.arange(n), n // 3),
+             "random": np.random.default_rng(65).permutation(n)}[name]
+    with ng.Context() as ctx:
+        host_edges(ctx, dna(16_000, 800, 61), 90)
+        got, _ = host_edges(ctx, moved(db, order), 90)
+    assert np.array_equal(got, want)
+
+
 def test_a_refused_step_leaves_the_database(cuda, built):
     """A pieced upload whose records pass its check stays loaded when the graph
     build refuses its arguments."""
