@@ -289,6 +289,43 @@ int persistent_grid(const void *func, int threads, size_t smem, uint32_t want, u
   return NGIA_OK;
 }
 
+// The general class: one pair per thread, grid-stride over the class's range.
+// A launch of its own, without tables: some 20 warps per multiprocessor where
+// the kernel of the 32-lane classes leaves room for seven.  One-warp blocks
+// spread few pairs over the multiprocessors, whose row words (up to 8 KB a
+// thread in local memory) are what binds it.  Rounds of related proteins, ms in
+// that kernel, here in blocks of 128, here: 60,000 pairs of 20,000 residues at
+// identity 50 571, 670, 515; 2,000 116, 129, 113; 1,000
+// of 60,000 at 40 1,175, 1,391, 1,175.
+__global__ void __launch_bounds__(32)
+align_general_kernel(const __grid_constant__ RoundArgs a) {
+  const uint32_t begin = a.bounds[kGeneralClass], end = a.bounds[kGeneralClass + 1];
+  uint32_t done = 0;
+  for (uint32_t k = begin + blockIdx.x * 32u + threadIdx.x; k < end; k += gridDim.x * 32u) {
+    const uint32_t p = a.order[k];
+    const uint2 pr = a.pairs[p];
+    const uint32_t *rep = a.packed + a.offs[pr.x];
+    const uint32_t *tar = a.packed + a.offs[pr.y];
+    const uint32_t lr = __ldg(rep), lt = __ldg(tar);
+    const Band b = make_band(lr, lt, a.t, a.fm);
+    uint32_t lines[kMaxRowBlocks];
+    uint32_t blocks;
+    const uint32_t lcs = lcs_general(rep, tar, b, lines, blocks);
+    done += blocks * ((b.width + 7u) & ~7u);
+    a.scores[p] = identity_score(lcs, lr, lt, a.t);
+  }
+  count_work(done, a.work);
+}
+
+int launch_align_general(const RoundArgs &a, uint32_t m, cudaStream_t s) {
+  uint32_t grid = 0;
+  NGIA_TRY(persistent_grid(reinterpret_cast<const void *>(align_general_kernel), 32, 0,
+                           ceil_div(m, 32u), &grid));
+  align_general_kernel<<<grid, 32, 0, s>>>(a);
+  NGIA_LAUNCHED();
+  return NGIA_OK;
+}
+
 template <int K>
 int launch_align_k(int kernel, const RoundArgs &a, uint32_t m, cudaStream_t s);
 

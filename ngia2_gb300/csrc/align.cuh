@@ -286,6 +286,19 @@ __host__ __device__ inline int round_class(const Band &b, const ClassPlan &plan,
   return slide >= 0 ? slide : c;
 }
 
+// Whether a round over records of at most `longest` residues can have pairs of
+// the general class: a rep of at most G slices goes to a group class of G
+// lanes that the plan uses, whatever its band (16,384 residues with the
+// default plan).
+__host__ __device__ inline bool general_possible(const ClassPlan &plan, uint32_t longest) {
+  uint32_t words = 0;
+  for (int g = 0; g < kNumGroupClasses; ++g) {
+    const GroupShape sh = group_shape(kFirstGroupClass + g);
+    if (plan.group_limit[g] && (uint32_t)(sh.G * sh.K) > words) words = (uint32_t)(sh.G * sh.K);
+  }
+  return (longest + 31) / 32 > words;
+}
+
 // Queue order inside a class: longest targets first.  The sort key of a pair
 // is class-major, then 7 - floor(log2 nc) (column blocks in octaves, capped
 // at 7), in eight bits.

@@ -90,4 +90,13 @@ __device__ __forceinline__ uint4 planes_to_nibbles(const uint4 &pl) {
   return make_uint4(out[0], out[1], out[2], out[3]);
 }
 
+// Adds the warp's computed 32x32 blocks (row words x column blocks) to *work.
+__device__ __forceinline__ void count_work(uint32_t blocks, unsigned long long *work) {
+  // two 16-bit halves, so that a warp's sum cannot overflow
+  const uint32_t lo = __reduce_add_sync(kFull, blocks & 0xFFFFu);
+  const uint32_t hi = __reduce_add_sync(kFull, blocks >> 16);
+  const unsigned long long sum = ((unsigned long long)hi << 16) + lo;
+  if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(work, sum);
+}
+
 }  // namespace ngia

@@ -9,15 +9,6 @@
 
 namespace ngia {
 
-// Adds the warp's computed 32x32 blocks (row words x column blocks) to *work.
-__device__ __forceinline__ void count_work(uint32_t blocks, unsigned long long *work) {
-  // two 16-bit halves, so that a warp's sum cannot overflow
-  const uint32_t lo = __reduce_add_sync(kFull, blocks & 0xFFFFu);
-  const uint32_t hi = __reduce_add_sync(kFull, blocks >> 16);
-  const unsigned long long sum = ((unsigned long long)hi << 16) + lo;
-  if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(work, sum);
-}
-
 // The batched kernels read their classes' ranges of the queue order from
 // device memory (bounds[cls] .. bounds[cls + 1], written by the classifier),
 // so that a round needs no host round trip and can be captured as a graph.
@@ -26,27 +17,6 @@ __device__ __forceinline__ void count_work(uint32_t blocks, unsigned long long *
 // is empty (an empty class costs a load).  One launch per class, 20 a round,
 // cost the small rounds more than their work: 600 proteins at identity 50
 // spent 0.14 ms aligning 1,176 pairs.
-
-// General class: one pair per thread, grid-stride over the class's range.
-__device__ __forceinline__ uint32_t align_general(const RoundArgs &a, int cls) {
-  const uint32_t begin = a.bounds[cls], end = a.bounds[cls + 1];
-  uint32_t done = 0;
-  for (uint32_t k = begin + blockIdx.x * blockDim.x + threadIdx.x; k < end;
-       k += gridDim.x * blockDim.x) {
-    const uint32_t p = a.order[k];
-    const uint2 pr = a.pairs[p];
-    const uint32_t *rep = a.packed + a.offs[pr.x];
-    const uint32_t *tar = a.packed + a.offs[pr.y];
-    const uint32_t lr = __ldg(rep), lt = __ldg(tar);
-    const Band b = make_band(lr, lt, a.t, a.fm);
-    uint32_t lines[kMaxRowBlocks];
-    uint32_t blocks;
-    const uint32_t lcs = lcs_general(rep, tar, b, lines, blocks);
-    done += blocks * ((b.width + 7u) & ~7u);
-    a.scores[p] = identity_score(lcs, lr, lt, a.t);
-  }
-  return done;
-}
 
 // One group class: the block's warps take its pairs (align_group.cuh).
 template <int C, int KC>
@@ -57,8 +27,7 @@ __device__ __forceinline__ uint32_t group_class(const RoundArgs &a, uint32_t *sm
                                      a.bounds[C + 1], a.cursors + C, a.scores, a.t, a.fm, smem);
 }
 
-// The classes of 32 lanes, widest first, and the general class: few and long
-// pairs, at most seven warps of them per multiprocessor, so that a pair of
+// The classes of 32 lanes, widest first: few and long pairs, at most seven warps of them per multiprocessor, so that a pair of
 // 30,000 residues does not share its scheduler with three others and end the
 // round alone (2 million heavy-tailed pairs after the seed filter: 6.3 ms in
 // one kernel with the classes of 8 and 16 lanes at 14 warps, 4.7 ms here).
@@ -66,8 +35,7 @@ template <int KC>
 __global__ void __launch_bounds__(32)
 align_wide_kernel(const __grid_constant__ RoundArgs a) {
   extern __shared__ uint32_t smem[];
-  uint32_t done = align_general(a, kGeneralClass);
-  done += group_class<kFirstGroupClass + 7, KC>(a, smem);
+  uint32_t done = group_class<kFirstGroupClass + 7, KC>(a, smem);
   done += group_class<kFirstGroupClass + 6, KC>(a, smem);
   done += group_class<kFirstGroupClass + 5, KC>(a, smem);
   done += group_class<kFirstGroupClass + 4, KC>(a, smem);

@@ -36,7 +36,7 @@ namespace ngia {
 
 DbView db_view(const ngia_ctx *c) {
   return DbView{c->packed.as<uint32_t>(), c->align_nib, c->ab, c->offs.as<uint64_t>(),
-                c->lens.as<uint32_t>()};
+                c->lens.as<uint32_t>(), c->longest};
 }
 
 // The bucketing on the context's stream, through a cached graph when the
@@ -389,8 +389,9 @@ static int use_alphabet(ngia_ctx *c, const AlphaChoice &a, uint64_t words, uint3
 // Every record inside the region by its offset and read length, and no read
 // longer than the format allows (one pass over the two arrays, before any
 // copy); the device checks each record's length word as it lays it out.
+// *longest: the longest read.
 bool records_inside(const uint64_t *h_offs, const uint32_t *h_lens, uint32_t n,
-                    uint64_t words) {
+                    uint64_t words, uint32_t *longest) {
   // the longest read and the furthest record end, compared once (a max
   // reduction the compiler vectorises; a record's end lies past its offset)
   uint32_t max_len = 0;
@@ -401,6 +402,7 @@ bool records_inside(const uint64_t *h_offs, const uint32_t *h_lens, uint32_t n,
     max_len = len > max_len ? len : max_len;
     max_end = end > max_end ? end : max_end;
   }
+  *longest = max_len;
   return max_len <= NGIA_MAX_READ && max_end <= words;
 }
 
@@ -408,7 +410,8 @@ int ctx_load(ngia_ctx *c, const uint32_t *h_packed, uint64_t words, const uint64
              const uint32_t *h_lens, uint32_t n, const uint32_t *h_rep, uint32_t bands) {
   if (n == 0 || !h_packed || !h_offs || !h_lens) return NGIA_ERR_ARG;
   if (h_rep && (bands < 1 || bands > (uint32_t)kBands)) return NGIA_ERR_ARG;
-  if (!records_inside(h_offs, h_lens, n, words)) return NGIA_ERR_ARG;
+  uint32_t longest = 0;
+  if (!records_inside(h_offs, h_lens, n, words, &longest)) return NGIA_ERR_ARG;
   cudaStream_t s = c->stream;
   NGIA_TRY(c->packed.reserve(words * 4));
   NGIA_TRY(c->offs.reserve((size_t)n * 8));
@@ -433,6 +436,7 @@ int ctx_load(ngia_ctx *c, const uint32_t *h_packed, uint64_t words, const uint64
   NGIA_TRY(use_alphabet(c, choose_alphabet(present), words, n, true));
   c->last_present = present;
   c->n = n;
+  c->longest = longest;
   c->sigs_valid = false;
   c->packed_words = words;
   c->rep_bands = 0;
@@ -477,6 +481,7 @@ int ctx_load_text(ngia_ctx *c, const char *h_text, uint64_t text_bytes,
   NGIA_TRY(use_alphabet(c, choose_alphabet(present), words, n, true));
   c->last_present = present;
   c->n = n;
+  c->longest = *std::max_element(h_lens, h_lens + n);
   c->sigs_valid = false;
   c->packed_words = words;
   c->rep_bands = 0;
@@ -630,6 +635,7 @@ int ctx_load_sketch(ngia_ctx *c, const uint32_t *h_packed, uint64_t words,
   c->nib_stale = true;
   NGIA_TRY(use_alphabet(c, spec, words, n, false));
   c->n = n;
+  c->longest = NGIA_MAX_READ;  // until the host has looked
   c->sigs_valid = false;
   c->packed_words = words;
   c->rep_bands = 0;
@@ -995,7 +1001,8 @@ int ngia_ctx_run_host(ngia_ctx *c, const uint32_t *h_packed, uint64_t packed_wor
     int rc = ngia::ctx_sketch_bucket(c, bands, stats, true, true);
     // the host check of every record, while the device sketches and buckets
     // (nothing launched so far trusts the offsets; the candidates do)
-    const bool inside = ngia::records_inside(h_rec_offsets, h_lens, n, packed_words);
+    const bool inside =
+        ngia::records_inside(h_rec_offsets, h_lens, n, packed_words, &c->longest);
     if (rc == NGIA_OK && !inside) rc = NGIA_ERR_ARG;
     bool stands = false;  // the map served every record
     if (rc == NGIA_OK)

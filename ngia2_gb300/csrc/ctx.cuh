@@ -47,6 +47,7 @@ struct ngia_ctx {
   bool table_ok = false, table_built = false, use_table = true;
   uint64_t table_inv = 0;  // the aligner-code map the sketch tables were built for
   ngia::DevBuf sketch_table;
+  uint32_t longest = 0;  // no read of the database is longer
   // graph build work
   ngia::DevBuf ucount, uoff, counters, pairs, scores, emit_tmp, edges, scan_tmp,
       sort_tmp;

@@ -94,6 +94,8 @@ constexpr bool align_kernel_used(int kernel, uint32_t widest) {
   return widest > 16 ? kernel != 5 : kernel != 1 && kernel != 3 && kernel != 4;
 }
 int launch_align(int kernel, const RoundArgs &a, int K, uint32_t m, cudaStream_t s);
+// The general class of the round (none of the kernels above takes its pairs).
+int launch_align_general(const RoundArgs &a, uint32_t m, cudaStream_t s);
 // All layouts of records offs[0..n) in one pass under an assumed code map
 // (inv: nibble d = residue code of aligner code d, pipelined loads): nibbles,
 // recoded nibbles and code planes.  *bad = 1 if a residue has a code outside

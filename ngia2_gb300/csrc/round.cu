@@ -60,6 +60,7 @@ bool Round::Key::operator==(const Key &o) const {
   return pairs == o.pairs && scores == o.scores && nib == o.nib && packed == o.packed &&
          dplanes == o.dplanes && offs == o.offs && lens == o.lens && m == o.m &&
          identity == o.identity && round_mode == o.round_mode && ab_k == o.ab_k &&
+         general == o.general &&
          ab_inv == o.ab_inv && alloc_gen == o.alloc_gen && plan_gen == o.plan_gen;
 }
 
@@ -169,10 +170,15 @@ int Round::enqueue(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t id
   // so, 5.7 with the groups ahead, 5.6 with the narrow windows ahead; 2 million
   // pairs: 5.8, 6.1, 6.0).
   NGIA_CUDA(cudaEventRecord(fork_, s));
+  const bool general = general_possible(plan, db.longest);
   for (int k = 0; k < kAlignKernels; ++k) {
     if (!align_kernel_used(k, widest)) continue;
     NGIA_CUDA(cudaStreamWaitEvent(side_[k], fork_, 0));
     NGIA_TRY(launch_align(k, args, db.ab.K, m, side_[k]));
+    // The general class behind the narrowest windows, not on a branch of its
+    // own: an eighth one, empty, cost 2 million heavy-tailed pairs 5.65 -> 6.35
+    // ms, and a pair of the class takes tens of milliseconds anyway.
+    if (general && k == kAlignKernels - 1) NGIA_TRY(launch_align_general(args, m, side_[k]));
     NGIA_CUDA(cudaEventRecord(join_[k], side_[k]));
   }
   for (int k = 0; k < kAlignKernels; ++k)
@@ -188,8 +194,8 @@ int Round::launch(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t ide
   // buffers and alphabet (a new load may reuse the buffers with another
   // alphabet, whose classes are other kernels), the pairs, the plan
   const Key key{pairs,   scores, db.nib,   db.packed,    db.ab.dplanes, db.offs,
-                db.lens, m,      identity, round_mode(), db.ab.K,       db.ab.inv,
-                g_alloc_gen.load(), plan_gen};
+                db.lens, m,      identity, round_mode(), db.ab.K,       general_possible(plan, db.longest),
+                db.ab.inv, g_alloc_gen.load(), plan_gen};
   if (!exec_ || !(key == key_)) {
     if (exec_) cudaGraphExecDestroy(exec_);
     exec_ = nullptr;

@@ -48,6 +48,7 @@ struct DbView {
   Alphabet ab;
   const uint64_t *offs;
   const uint32_t *lens;
+  uint32_t longest;  // no read is longer
 };
 
 double ev_ms(cudaEvent_t a, cudaEvent_t b);
@@ -102,6 +103,7 @@ class Round {
     const void *pairs, *scores, *nib, *packed, *dplanes, *offs, *lens;
     uint32_t m, identity;
     int round_mode, ab_k;
+    bool general;
     uint64_t ab_inv, alloc_gen, plan_gen;
     bool operator==(const Key &o) const;
   } key_{};

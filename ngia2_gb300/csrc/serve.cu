@@ -16,6 +16,7 @@
 // keeps it, the others are marked empty and skipped by the classifier --,
 // the batched round, selection of the first band with a hit, copy out, and a
 // host callback that completes the request.
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
@@ -166,9 +167,11 @@ struct Server {
   bool stop = false;
   std::thread dispatcher;
 
-  DbView view() const {
+  uint32_t longest = 0;       // no read of the database is longer
+  DbView view(uint32_t longest_query) const {
     return DbView{packed.as<uint32_t>(), recode_map ? dense.as<uint32_t>() : nib.as<uint32_t>(),
-                  ab, offs.as<uint64_t>(), lens.as<uint32_t>()};
+                  ab, offs.as<uint64_t>(), lens.as<uint32_t>(),
+                  longest_query > longest ? longest_query : longest};
   }
 };
 
@@ -222,8 +225,9 @@ static int run_request(Server *s, Slot *sl, Request *r) {
   NGIA_LAUNCHED();
   uint32_t *scores = sl->scores.as<uint32_t>();
   if (!s->cfg.plain) {
-    NGIA_TRY(sl->round.enqueue(s->view(), sl->pairs.as<uint2>(), slots, s->cfg.identity, scores,
-                               nullptr));
+    const uint32_t longest = *std::max_element(r->lens.begin(), r->lens.end());
+    NGIA_TRY(sl->round.enqueue(s->view(longest), sl->pairs.as<uint2>(), slots,
+                               s->cfg.identity, scores, nullptr));
   } else {
     // the plain form: compact the pairs, one launch of the drop-in kernel
     NGIA_CUDA(cudaMemsetAsync(sl->count.p, 0, 4, st));
@@ -376,6 +380,7 @@ static int server_init(ngia_server *s, ngia_ctx *db, const uint32_t *h_cluster,
   const uint64_t W = s->cfg.max_words;
   s->n = n;
   s->db_words = db->packed_words;
+  s->longest = db->longest;
   s->ab = db->ab;
   s->recode_map = db->recode_map;
   const uint64_t total_words = db->packed_words + (uint64_t)S * W;

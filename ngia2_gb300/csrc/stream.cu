@@ -21,6 +21,7 @@
 // record tables and aligned by one batched round.  Scores go back to the
 // pairs' own positions, so the emission (sorted unique edges) is the resident
 // path's.
+#include <algorithm>
 #include <chrono>
 #include <cstring>
 #include <thread>
@@ -258,6 +259,7 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
     c.count += 1;
     c.words = h_offs[i] + w - c.word_first;
   }
+  const uint32_t longest = *std::max_element(h_lens, h_lens + n);
   const uint32_t C = (uint32_t)chunks.size();
   if ((uint64_t)C * C > 0xFFFFFFFFull) return NGIA_ERR_ARG;
   uint32_t max_recs = 0;
@@ -428,7 +430,7 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
   NGIA_TRY(S.block_scores.reserve(mb * 4));
   NGIA_TRY(S.round.reserve(max_block));
   NGIA_CUDA(cudaMemsetAsync(S.scores.p, 0, mm * 4, s));
-  const DbView view{rp, rn, ab, roffs, rlens};
+  const DbView view{rp, rn, ab, roffs, rlens, longest};
   NGIA_CUDA(cudaMemsetAsync(acc, 0, 16, s));
   uint64_t loads = 0;
   // The slots hold three chunks.  A row of blocks (one outer chunk a) runs from
