@@ -5,7 +5,7 @@
 // A warp takes 32 jobs in job order, one pair per lane, in the windows of the
 // batched aligner (align_window.cuh): the lanes whose pairs fit 4, 8, 12, 16
 // and 24 words (the whole rep, or the sliding band) run together, the rest
-// through the general form.  Match masks come from tables in shared memory, as
+// through the general form (in a launch of their own where there are many jobs).  Match masks come from tables in shared memory, as
 // there; the target's codes are made from its bit planes, block by block.
 //
 // What bounds it at the reference's launch sizes (a band's few thousand jobs):
@@ -18,7 +18,8 @@
 
 namespace ngia {
 
-constexpr int kJobSlots = 27;  // table slots: 24 words and room to slide
+constexpr uint32_t kJobWords = 24;  // the widest window
+constexpr int kJobSlots = 27;       // table slots: room for it to slide
 
 // The lanes of the warp with `run` align their pairs; returns the score.
 template <int W, bool kSlide>
@@ -59,6 +60,40 @@ __device__ __forceinline__ void job_window(bool run, const uint32_t *rep, const 
   }
 }
 
+// A job, and how it is aligned.
+struct Job {
+  const uint32_t *rep, *tar;
+  Band b;
+  bool mine, empty;  // to be scored; no columns
+  bool fixed;        // the whole rep is narrower than the sliding window
+  uint32_t words;    // of the narrower of the two (0: nothing to align)
+};
+
+__device__ __forceinline__ Job load_job(const uint32_t *packed, const uint64_t *offs,
+                                        const uint32_t *jobs, uint32_t j, uint32_t count,
+                                        float t, int fma_mode) {
+  Job w{packed, packed, {}, false, true, false, 0u};
+  if (j >= count) return w;
+  w.rep = packed + offs[jobs[3 * (size_t)j]];
+  w.tar = packed + offs[jobs[3 * (size_t)j + 1]];
+  w.b = make_band(__ldg(w.rep), __ldg(w.tar), t, fma_mode);
+  w.mine = w.b.pass;  // else the reference leaves the score word as it was
+  w.empty = w.b.nc == 0;
+  const uint32_t ws = stream_width(w.b);
+  w.fixed = w.b.nr < ws;
+  w.words = w.mine && !w.empty ? (w.fixed ? w.b.nr : ws) : 0u;
+  return w;
+}
+
+// In the general form, for any width.
+__device__ __forceinline__ uint32_t job_general(const Job &w, float t) {
+  uint32_t lines[kMaxRowBlocks];
+  uint32_t blocks;
+  return identity_score(lcs_general(w.rep, w.tar, w.b, lines, blocks), w.b.lr, w.b.lt, t);
+}
+
+// The jobs of up to kJobWords words, and with kWide the others too.
+template <bool kWide>
 __global__ void __launch_bounds__(32)
 align_jobs_kernel(const uint32_t *__restrict__ packed, const uint64_t *__restrict__ offs,
                   uint32_t *__restrict__ jobs, uint32_t count, float t, int fma_mode) {
@@ -67,19 +102,10 @@ align_jobs_kernel(const uint32_t *__restrict__ packed, const uint64_t *__restric
 #pragma unroll 1
   for (int s = 0; s < kJobSlots; ++s) col[s * 32] = 0u;  // code 0 matches nothing
   const uint32_t j = blockIdx.x * 32u + threadIdx.x;
-  const uint32_t *rep = packed, *tar = packed;
-  Band b{};
-  if (j < count) {
-    rep = packed + offs[jobs[3 * (size_t)j]];
-    tar = packed + offs[jobs[3 * (size_t)j + 1]];
-    b = make_band(__ldg(rep), __ldg(tar), t, fma_mode);
-  }
-  const bool mine = j < count && b.pass;  // else the reference leaves the score word as it was
-  const bool empty = b.nc == 0;
-  // the narrower of the sliding window and the whole rep
-  const uint32_t ws = stream_width(b);
-  const bool fixed = b.nr < ws;
-  const uint32_t words = mine && !empty ? (fixed ? b.nr : ws) : 0u;
+  const Job w = load_job(packed, offs, jobs, j, count, t, fma_mode);
+  const uint32_t *rep = w.rep, *tar = w.tar, words = w.words;
+  const Band &b = w.b;
+  const bool fixed = w.fixed;
   uint32_t score = 0;
   job_window<4, true>(!fixed && words - 1u < 4u, rep, tar, b, col, score);
   job_window<8, true>(!fixed && words - 5u < 4u, rep, tar, b, col, score);
@@ -89,25 +115,49 @@ align_jobs_kernel(const uint32_t *__restrict__ packed, const uint64_t *__restric
   job_window<8, false>(fixed && words - 1u < 8u, rep, tar, b, col, score);
   job_window<16, false>(fixed && words - 9u < 8u, rep, tar, b, col, score);
   job_window<24, false>(fixed && words - 17u < 8u, rep, tar, b, col, score);
-  if (mine && !empty && words > 24) {
-    uint32_t lines[kMaxRowBlocks];
-    uint32_t blocks;
-    score = identity_score(lcs_general(rep, tar, b, lines, blocks), b.lr, b.lt, t);
-  } else if (mine && empty) {
-    score = identity_score(0u, b.lr, b.lt, t);
+  if constexpr (kWide) {
+    if (words > kJobWords) score = job_general(w, t);
   }
-  if (mine) jobs[3 * (size_t)j + 2] = score;
+  if (w.mine && (kWide || words <= kJobWords))
+    jobs[3 * (size_t)j + 2] = w.empty ? identity_score(0u, b.lr, b.lt, t) : score;
+}
+
+// The wider jobs alone, without tables.
+__global__ void __launch_bounds__(32)
+align_jobs_wide_kernel(const uint32_t *__restrict__ packed, const uint64_t *__restrict__ offs,
+                       uint32_t *__restrict__ jobs, uint32_t count, float t, int fma_mode) {
+  const uint32_t j = blockIdx.x * 32u + threadIdx.x;
+  const Job w = load_job(packed, offs, jobs, j, count, t, fma_mode);
+  if (w.words > kJobWords) jobs[3 * (size_t)j + 2] = job_general(w, t);
 }
 
 int launch_align_jobs(const uint32_t *packed, const uint64_t *offs, uint32_t *jobs,
                       uint32_t count, uint32_t identity, cudaStream_t s) {
   if (count == 0) return NGIA_OK;
   constexpr size_t smem = (size_t)kJobSlots * 16 * 32 * 4;
-  const void *func = reinterpret_cast<const void *>(align_jobs_kernel);
-  uint32_t grid = 0;  // (sets the kernel's shared memory)
-  NGIA_TRY(persistent_grid(func, 32, smem, kFull, &grid));
-  align_jobs_kernel<<<ceil_div(count, 32u), 32, smem, s>>>(
-      packed, offs, jobs, count, identity_threshold(identity), round_mode());
+  const void *func = reinterpret_cast<const void *>(align_jobs_kernel<true>);
+  const uint32_t warps = ceil_div(count, 32u);
+  const float t = identity_threshold(identity);
+  uint32_t grid = 0;
+  NGIA_TRY(persistent_grid(func, 32, smem, warps, &grid));
+  if (grid == warps) {
+    align_jobs_kernel<true><<<grid, 32, smem, s>>>(packed, offs, jobs, count, t, round_mode());
+    NGIA_LAUNCHED();
+    return NGIA_OK;
+  }
+  // More jobs than fit on the device at once: the tables leave a multiprocessor
+  // four warps, which pairs over kJobWords words, with no use for tables, would
+  // share.  Their own launch has twenty (100,000 pairs of 1,500 residues at
+  // identity 50: 3.58 ms in one launch, 2.68 in two; 2 million heavy-tailed pairs
+  // at 90 in 64 calls: 3,655 and 3,545 ms), and costs a call without such pairs
+  // a pass over its jobs (200,000 of 300 residues at 90: 66 and 71 us).
+  // Overlapping the two as dependent launches: 3,780 ms with the narrow one
+  // first, 3,498 with the wide one first.
+  const void *narrow = reinterpret_cast<const void *>(align_jobs_kernel<false>);
+  NGIA_TRY(persistent_grid(narrow, 32, smem, warps, &grid));  // (sets its shared memory)
+  align_jobs_kernel<false><<<warps, 32, smem, s>>>(packed, offs, jobs, count, t, round_mode());
+  NGIA_LAUNCHED();
+  align_jobs_wide_kernel<<<warps, 32, 0, s>>>(packed, offs, jobs, count, t, round_mode());
   NGIA_LAUNCHED();
   return NGIA_OK;
 }
