@@ -199,14 +199,14 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   // follows where there turn out to be more
   Counters &rc = c->h_counters->round;
   if (m > 0) {
-    uint64_t *d_m = &dc->unique_total;  // read above, free now
+    uint64_t *d_m = &dc->unique_total;  // (the candidates' counters are read, and free now)
     if (m <= kSmallEmit) {
       NGIA_TRY(emit_small(pairs, scores, m, c->edges.as<ngia_edge>(), d_m, s));
     } else {
       NGIA_TRY(c->emit_tmp.reserve(kSmallEmit * sizeof(uint32_t)));
-      NGIA_CUDA(cudaMemsetAsync(d_m, 0, sizeof(uint64_t), s));
+      NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
       NGIA_TRY(emit_few(pairs, scores, m, c->edges.as<ngia_edge>(), c->emit_tmp.as<uint32_t>(),
-                        d_m, s));
+                        reinterpret_cast<uint64_t *>(&dc->cand_total), d_m, s));
     }
     NGIA_CUDA(cudaEventRecord(c->ev[3], s));
     NGIA_CUDA(cudaMemcpyAsync(&c->h_counters->edges, d_m, sizeof(uint64_t),
@@ -221,7 +221,8 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   if (m > 0) ne = c->h_counters->edges;
   if (ne > kSmallEmit) {
     NGIA_TRY(c->emit_tmp.reserve(emit_scratch_bytes(m, n)));
-    NGIA_TRY(emit_sorted(pairs, scores, m, n, c->edges.as<ngia_edge>(), &ne, c->emit_tmp.p, s));
+    NGIA_TRY(emit_sorted(pairs, scores, m, n, c->edges.as<ngia_edge>(), &ne, c->emit_tmp.p, s,
+                         ne));
     NGIA_CUDA(cudaEventRecord(c->ev[3], s));
     NGIA_CUDA(cudaEventSynchronize(c->ev[3]));
   }

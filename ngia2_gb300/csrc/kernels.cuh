@@ -179,20 +179,23 @@ size_t share_scratch_bytes(uint32_t count);
 int share_range(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
                 uint32_t part, uint32_t parts, void *scratch, uint32_t h_cut[2],
                 cudaStream_t s);
+// known: the number of pairs that scored, where the caller has it (else the
+// call waits for it).
+constexpr uint64_t kUnknownHits = ~0ull;
 size_t emit_scratch_bytes(uint32_t count, uint32_t n_nodes);
 int emit_sorted(const uint2 *pairs, const uint32_t *scores, uint32_t count,
                 uint32_t n_nodes, ngia_edge *out, uint64_t *h_m, void *scratch,
-                cudaStream_t s);
+                cudaStream_t s, uint64_t known = kUnknownHits);
 // The same for at most kSmallEmit pairs in one launch and without a wait: the
 // edge count lands in *d_m.
 constexpr uint32_t kSmallEmit = 4096;
 int emit_small(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
                uint64_t *d_m, cudaStream_t s);
 // The same for any number of pairs as long as at most kSmallEmit of them scored
-// (more: *d_m is some larger number and nothing was written).  hits: kSmallEmit words; *d_m zero
-// before the call.
+// (more: *d_m is their number and nothing was written).  hits: kSmallEmit words;
+// *taken and *d_m zero before the call.
 int emit_few(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
-             uint32_t *hits, uint64_t *d_m, cudaStream_t s);
+             uint32_t *hits, uint64_t *taken, uint64_t *d_m, cudaStream_t s);
 // Fast mode's bands [b0, b1): first_band[target] = min of itself and the first
 // of those bands that names the rep of a pair scoring > 0.
 int fast_first_band(const uint32_t *rep, uint32_t n, uint32_t b0, uint32_t b1,

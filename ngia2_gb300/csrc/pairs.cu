@@ -740,7 +740,7 @@ size_t emit_scratch_bytes(uint32_t count, uint32_t n_nodes) {
 // target-ordered list stably by rep gives (rep, tar) order.  *h_m = edges.
 int emit_sorted(const uint2 *pairs, const uint32_t *scores, uint32_t count,
                 uint32_t n_nodes, ngia_edge *out, uint64_t *h_m, void *scratch,
-                cudaStream_t s) {
+                cudaStream_t s, uint64_t known) {
   *h_m = 0;
   if (count == 0) return NGIA_OK;
   char *w = static_cast<char *>(scratch);
@@ -767,9 +767,11 @@ int emit_sorted(const uint2 *pairs, const uint32_t *scores, uint32_t count,
   NGIA_LAUNCHED();
   compact_hits_kernel<<<runs, 256, 0, s>>>(pairs, scores, count, bcount, erep, etar, escore);
   NGIA_LAUNCHED();
-  uint64_t m = 0;
-  NGIA_CUDA(cudaMemcpyAsync(&m, d_total, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  NGIA_CUDA(cudaStreamSynchronize(s));
+  uint64_t m = known;
+  if (m == kUnknownHits) {
+    NGIA_CUDA(cudaMemcpyAsync(&m, d_total, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    NGIA_CUDA(cudaStreamSynchronize(s));
+  }
   *h_m = m;
   if (m == 0) return NGIA_OK;
   const int bits = bits_for(n_nodes ? n_nodes - 1 : 0);
@@ -811,23 +813,34 @@ emit_small_kernel(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ 
 
 // Any number of pairs, few of which scored: their indices are appended (warp by
 // warp, until there are too many) to a list of kSmallEmit, which one block sorts
-// as above.
+// as above.  taken: places of the list; d_m: all hits, counted to the end, so
+// that the general path need not wait for its own count.
 __global__ void __launch_bounds__(256)
 append_hits_kernel(const uint32_t *__restrict__ scores, uint32_t count,
-                   uint32_t *__restrict__ hits, unsigned long long *__restrict__ d_m) {
+                   uint32_t *__restrict__ hits, unsigned long long *__restrict__ taken,
+                   unsigned long long *__restrict__ d_m) {
+  __shared__ uint32_t found;
+  if (threadIdx.x == 0) found = 0;
+  __syncthreads();
   const uint32_t lane = threadIdx.x & 31u;
+  uint32_t mine = 0;  // the warp's hits
+  bool room = true;
   for (uint32_t p0 = blockIdx.x * 256u; p0 < count; p0 += gridDim.x * 256u) {  // block-uniform
     const uint32_t p = p0 + threadIdx.x;
     const bool hit = p < count && scores[p] > 0;
     const uint32_t all = __ballot_sync(kFull, hit);
-    if (all == 0) continue;
+    mine += __popc(all);
+    if (all == 0 || !room) continue;
     unsigned long long first = 0;
-    if (lane == 0) first = atomicAdd(d_m, (unsigned long long)__popc(all));
+    if (lane == 0) first = atomicAdd(taken, (unsigned long long)__popc(all));
     first = __shfl_sync(kFull, first, 0);
-    if (first > kSmallEmit) return;  // too many: the general path takes over
+    room = first < kSmallEmit;  // too many: the general path takes over
     first += __popc(all & ((1u << lane) - 1u));
     if (hit && first < kSmallEmit) hits[first] = p;
   }
+  if (lane == 0 && mine) atomicAdd(&found, mine);
+  __syncthreads();
+  if (threadIdx.x == 0 && found) atomicAdd(d_m, (unsigned long long)found);
 }
 
 __global__ void __launch_bounds__(1024)
@@ -853,10 +866,11 @@ emit_hits_kernel(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ s
 }
 
 int emit_few(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
-             uint32_t *hits, uint64_t *d_m, cudaStream_t s) {
+             uint32_t *hits, uint64_t *taken, uint64_t *d_m, cudaStream_t s) {
   const uint32_t want = ceil_div(count, 256u * 8u), cap = 152u * 8u;
   append_hits_kernel<<<want < cap ? want : cap, 256, 0, s>>>(
-      scores, count, hits, reinterpret_cast<unsigned long long *>(d_m));
+      scores, count, hits, reinterpret_cast<unsigned long long *>(taken),
+      reinterpret_cast<unsigned long long *>(d_m));
   NGIA_LAUNCHED();
   emit_hits_kernel<<<1, 1024, 0, s>>>(pairs, scores, hits, out, d_m);
   NGIA_LAUNCHED();
