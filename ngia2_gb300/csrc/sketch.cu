@@ -17,6 +17,8 @@
 // position against half a byte read.  On this GPU the logic/shift pipe and
 // the integer multiply-add pipe draw on the same integer issue budget, and a
 // multiply-high costs two of its slots, so the shifts stay shifts.
+#include <algorithm>
+
 #include "align_lds.cuh"
 #include "kernels.cuh"
 
@@ -543,28 +545,6 @@ int build_sketch_table(uint64_t inv, void *table, cudaStream_t s) {
   return rc;
 }
 
-static int rank_blocks_per_sm() {
-  static int cached = 0;
-  if (!cached) {
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, sketch_rank_kernel,
-                                                      kRankWarps * 32, 0) != cudaSuccess ||
-        b < 1)
-      b = 1;
-    // A multiprocessor's split between L1 and shared memory changes only while
-    // it is empty: without a wish of its own the short records' kernel, which
-    // uses no shared memory, keeps the rank walk's blocks out until it ends
-    // (200,000 nucleotide reads: 1.55 ms one after the other, 1.24 beside each
-    // other).
-    (void)cudaFuncSetAttribute(sketch_table_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    (void)cudaFuncSetAttribute(sketch_rank_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    cached = b;
-  }
-  return cached;
-}
-
 int launch_sketch_table(const uint32_t *packed, const uint32_t *dense, const uint64_t *offs,
                         uint32_t n, uint64_t words, uint64_t inv, const void *table,
                         uint32_t *sigs, uint32_t stride, cudaStream_t s, cudaStream_t side,
@@ -574,18 +554,26 @@ int launch_sketch_table(const uint32_t *packed, const uint32_t *dense, const uin
   NGIA_CUDA(cudaGetDevice(&dev));
   NGIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const uint8_t *base = static_cast<const uint8_t *>(table);
-  const uint32_t rank_cap = (uint32_t)(sms * rank_blocks_per_sm());
+  // Both kernels' grids by the one lookup that, per device, also asks for the
+  // most shared memory: a multiprocessor's split between L1 and shared memory
+  // changes only while it is empty, and without that wish the short records'
+  // kernel, which uses no shared memory, keeps the rank walk's blocks out until
+  // it ends (200,000 nucleotide reads: 1.55 ms one after the other, 1.24 beside
+  // each other).
+  uint32_t rank_grid = 0, table_grid = 0;
+  NGIA_TRY(persistent_grid(reinterpret_cast<const void *>(sketch_rank_kernel), kRankWarps * 32, 0,
+                           ceil_div(n, (uint32_t)kRankWarps), &rank_grid));
+  NGIA_TRY(persistent_grid(reinterpret_cast<const void *>(sketch_table_kernel), 256, 0,
+                           std::min(ceil_div(n, 8u), (uint32_t)sms), &table_grid));
   // The rank walk's residency is bound by its bit sets (shared memory), which
   // leaves each SM room in threads and registers for one block of the short
   // records' kernel (no shared memory): one block per SM, beside it.
   NGIA_CUDA(cudaEventRecord(fork, s));
   NGIA_CUDA(cudaStreamWaitEvent(side, fork, 0));
-  const uint32_t want = ceil_div(n, 8u), cap = (uint32_t)sms;
-  sketch_table_kernel<<<want < cap ? want : cap, 256, 0, side>>>(
+  sketch_table_kernel<<<table_grid, 256, 0, side>>>(
       packed, dense, offs, n, words, reinterpret_cast<const uint4 *>(base), sigs, stride);
   NGIA_LAUNCHED();
-  const uint32_t rank_want = ceil_div(n, kRankWarps);
-  sketch_rank_kernel<<<rank_want < rank_cap ? rank_want : rank_cap, kRankWarps * 32, 0, s>>>(
+  sketch_rank_kernel<<<rank_grid, kRankWarps * 32, 0, s>>>(
       dense, offs, n, words, inv, reinterpret_cast<const uint16_t *>(base + kRowTableBytes),
       sigs, stride);
   NGIA_LAUNCHED();
