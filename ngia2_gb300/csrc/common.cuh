@@ -183,9 +183,10 @@ __host__ __device__ inline bool may_reach_threshold(uint32_t lcs_so_far, uint32_
   return stream_may_reach(lcs_so_far, cols_done, b.lr, b.lt, b.t);
 }
 
+// (a build may hold up to 2^32 - 1 pairs: a + b - 1 would wrap)
 template <typename T>
-__host__ __device__ inline T ceil_div(T a, T b) {
-  return (a + b - 1) / b;
+__host__ __device__ constexpr T ceil_div(T a, T b) {
+  return a / b + (a % b != 0 ? 1 : 0);
 }
 
 }  // namespace ngia

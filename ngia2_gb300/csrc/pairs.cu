@@ -374,12 +374,13 @@ place_kernel(const uint8_t *__restrict__ keys, uint32_t count,
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   for (uint32_t k = lane; k < kQueueKeys; k += 32) at[warp][k] = 0;
   __syncwarp();
-  const uint32_t base = (blockIdx.x * kPlaceWarps + warp) * (32u * kPlacePairs) + lane;
+  // (in 64 bits: the last block's places may lie past 2^32)
+  const uint64_t base = ((uint64_t)blockIdx.x * kPlaceWarps + warp) * (32u * kPlacePairs) + lane;
   const uint32_t lt_mask = (1u << lane) - 1u;
   uint32_t key[kPlacePairs], place[kPlacePairs];  // place: within the warp's share
 #pragma unroll
   for (uint32_t j = 0; j < kPlacePairs; ++j) {
-    const uint32_t p = base + 32u * j;
+    const uint64_t p = base + 32u * j;
     key[j] = p < count ? keys[p] : skip_sort_key();
   }
 #pragma unroll
@@ -409,7 +410,7 @@ place_kernel(const uint8_t *__restrict__ keys, uint32_t count,
 #pragma unroll
   for (uint32_t j = 0; j < kPlacePairs; ++j)
     if (key[j] >> 3 != (uint32_t)kSkipClass)
-      order[at[warp][key[j]] + place[j]] = base + 32u * j;
+      order[at[warp][key[j]] + place[j]] = (uint32_t)base + 32u * j;
 }
 
 int classify(const uint32_t *lens, const uint2 *pairs, uint32_t count, uint32_t identity,
@@ -825,8 +826,9 @@ append_hits_kernel(const uint32_t *__restrict__ scores, uint32_t count,
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t mine = 0;  // the warp's hits
   bool room = true;
-  for (uint32_t p0 = blockIdx.x * 256u; p0 < count; p0 += gridDim.x * 256u) {  // block-uniform
-    const uint32_t p = p0 + threadIdx.x;
+  const uint64_t stride = gridDim.x * 256u;  // (the last step may pass 2^32)
+  for (uint64_t p0 = blockIdx.x * 256u; p0 < count; p0 += stride) {  // block-uniform
+    const uint64_t p = p0 + threadIdx.x;
     const bool hit = p < count && scores[p] > 0;
     const uint32_t all = __ballot_sync(kFull, hit);
     mine += __popc(all);
@@ -836,7 +838,7 @@ append_hits_kernel(const uint32_t *__restrict__ scores, uint32_t count,
     first = __shfl_sync(kFull, first, 0);
     room = first < kSmallEmit;  // too many: the general path takes over
     first += __popc(all & ((1u << lane) - 1u));
-    if (hit && first < kSmallEmit) hits[first] = p;
+    if (hit && first < kSmallEmit) hits[first] = (uint32_t)p;
   }
   if (lane == 0 && mine) atomicAdd(&found, mine);
   __syncthreads();

@@ -37,7 +37,7 @@ struct Counters {  // device-side counters of one graph build or round
   unsigned long long work;  // 32x32 blocks the aligners computed
   unsigned int cursor[kNumRoundClasses];  // pairs taken from each class's queue
   uint32_t bounds[kNumRoundClasses + 1];  // class ranges of the queue order
-  unsigned int seed_cursor;  // pairs taken by the seed filter
+  unsigned int seed_cursor;  // runs of pairs taken by the seed filter
   unsigned int collect_ticket, collect_error;  // the one-pass candidate collection
 };
 

@@ -172,13 +172,15 @@ seed_filter_kernel(const uint32_t *__restrict__ nib, const uint64_t *__restrict_
   __syncthreads();
   uint32_t target = kFull;  // whose words the set holds
   for (;;) {
-    uint32_t first = 0;
-    if (lane == 0) first = atomicAdd(cursor, run);
-    first = __shfl_sync(kFull, first, 0);
-    if (first >= m) break;
-    for (uint32_t base = first; base < min(m, first + run); base += 32) {
-      const uint32_t p = base + lane;
-      const uint32_t key = p < m ? keys[p] : skip_sort_key();
+    // runs are counted, not pairs: a sum past m could wrap at 2^32
+    uint32_t claim = 0;
+    if (lane == 0) claim = atomicAdd(cursor, 1u);
+    const uint64_t at = (uint64_t)__shfl_sync(kFull, claim, 0) * run;
+    if (at >= m) break;
+    const uint32_t first = (uint32_t)at, size = min(run, m - first);
+    for (uint32_t base = 0; base < size; base += 32) {
+      const uint32_t p = first + base + lane;
+      const uint32_t key = base + lane < size ? keys[p] : skip_sort_key();
       uint2 pr = make_uint2(0u, 0u);
       uint32_t lr = 0, lt = 0, need = kFull;
       uint64_t ro = 0, to = 0;
