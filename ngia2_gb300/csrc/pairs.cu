@@ -869,7 +869,10 @@ emit_hits_kernel(const uint2 *__restrict__ pairs, const uint32_t *__restrict__ s
 
 int emit_few(const uint2 *pairs, const uint32_t *scores, uint32_t count, ngia_edge *out,
              uint32_t *hits, uint64_t *taken, uint64_t *d_m, cudaStream_t s) {
-  const uint32_t want = ceil_div(count, 256u * 8u), cap = 152u * 8u;
+  int dev = 0, sms = 0;
+  NGIA_CUDA(cudaGetDevice(&dev));
+  NGIA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const uint32_t want = ceil_div(count, 256u * 8u), cap = (uint32_t)sms * 8u;
   append_hits_kernel<<<want < cap ? want : cap, 256, 0, s>>>(
       scores, count, hits, reinterpret_cast<unsigned long long *>(taken),
       reinterpret_cast<unsigned long long *>(d_m));
