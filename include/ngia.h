@@ -215,6 +215,12 @@ int ngia_ctx_group_align(ngia_ctx *ctx, uint32_t identity, uint32_t bands,
 int ngia_ctx_test_lookback_timeout(ngia_ctx *ctx, uint32_t identity, uint32_t bands,
                                    uint32_t spin_limit);
 
+/* Fast mode's fallback without filling the device: where a run's pair slots, or
+ * these and 9 bytes a pair, come to more than `bytes`, the reservation is taken
+ * as refused, and the run is halved (NGIA_ERR_NOMEM when a single band does not
+ * fit).  0, the default: no such limit.  Testing aid, no counterpart in the reference. */
+int ngia_ctx_test_fast_room(ngia_ctx *ctx, uint64_t bytes);
+
 /* Copy the last graph's edges to the host (cap entries at most). */
 int ngia_ctx_edges(ngia_ctx *ctx, ngia_edge *h_edges, uint64_t cap);
 
@@ -381,8 +387,8 @@ void ngia_server_destroy(ngia_server *srv);
 /* Fast greedy clustering (src/fastClustering.hpp:249-352): per band, targets
  * not yet assigned are aligned against their rep and assigned on a hit;
  * h_cluster[i] = root index.  Bands are aligned in runs and assigned in band
- * order; up to 8 bytes per record and band of a run, shorter runs where the
- * device has not that much.  Synchronises. */
+ * order; 8 bytes per record and band of a run, at most 512 MiB unless one band
+ * takes more, shorter runs where the device has not that much.  Synchronises. */
 int ngia_ctx_fast_cluster(ngia_ctx *ctx, uint32_t identity, uint32_t bands,
                           uint32_t *h_cluster, ngia_stats *stats);
 

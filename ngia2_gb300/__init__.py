@@ -144,6 +144,7 @@ _SIGNATURES = {
     "ngia_ctx_build_graph_part": (C.c_int, [C.c_void_p, C.c_uint32, C.c_uint32, C.c_uint32,
                                             C.c_uint32, C.c_void_p, C.POINTER(C.c_uint64),
                                             C.POINTER(Stats)]),
+    "ngia_ctx_test_fast_room": (C.c_int, [C.c_void_p, C.c_uint64]),
     "ngia_ctx_test_lookback_timeout": (C.c_int, [C.c_void_p, C.c_uint32, C.c_uint32,
                                                  C.c_uint32]),
     "ngia_ctx_align_pairs": (C.c_int, [C.c_void_p, C.c_void_p, C.c_uint32, C.c_uint32,

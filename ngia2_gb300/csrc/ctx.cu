@@ -263,6 +263,11 @@ int ctx_align_pairs(ngia_ctx *c, const uint2 *d_pairs, uint32_t m, uint32_t iden
   return NGIA_OK;
 }
 
+// Pair slots of a run of bands: half a gigabyte, which the context keeps (a
+// graph build's 64 x n slots share the buffer).  A run of 48 bands fits up to
+// 1.4 million records; beyond that a shorter run's round is large anyway.
+constexpr uint32_t kFastSlots = 1u << 26;
+
 int ctx_fast_cluster(ngia_ctx *c, uint32_t identity, uint32_t bands, uint32_t *h_cluster,
                      ngia_stats *st) {
   if (c->n == 0 || c->rep_bands == 0) return NGIA_ERR_STATE;
@@ -279,19 +284,21 @@ int ctx_fast_cluster(ngia_ctx *c, uint32_t identity, uint32_t bands, uint32_t *h
   NGIA_CUDA(cudaMemsetAsync(parent, 0xFF, (size_t)n * 4, s));
   NGIA_CUDA(cudaEventRecord(c->ev[0], s));
   // Runs of bands 0-3, 4-15 and the rest, shorter where bands x n would pass
-  // 2^30 pair slots.  One run would align, for a target with many close
+  // kFastSlots.  One run would align, for a target with many close
   // relatives, every distinct rep of 64 bands where the first usually scores;
   // a run per band costs 64 rounds (20,000 proteins, families of ten close
   // relatives, identity 90: 16.3 ms one band at a time through the
   // one-thread-per-pair kernel, 0.6 ms so).
   // Where the device has no room for a run's pairs (8 bytes a slot, 9 more a
   // pair) the run is halved, down to a band at a time.
-  uint32_t most = (1u << 30) / n ? (1u << 30) / n : 1u;
+  uint32_t most = std::max(kFastSlots / n, 1u);
+  auto over = [&](size_t bytes) { return c->fast_room && bytes > c->fast_room; };
   for (uint32_t b0 = 0, b1; b0 < bands; b0 = b1) {
     const uint32_t end = b0 < 4 ? 4u : b0 < 16 ? 16u : (uint32_t)kBands;
     b1 = std::min(std::min(end, bands), b0 + most);
     NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
-    int room = c->pairs.reserve((size_t)(b1 - b0) * n * 8);
+    const size_t slots = (size_t)(b1 - b0) * n * 8;
+    int room = over(slots) ? NGIA_ERR_NOMEM : c->pairs.reserve(slots);
     if (room == NGIA_ERR_NOMEM && b1 - b0 > 1) {
       most = (b1 - b0) / 2;
       b1 = b0;
@@ -309,7 +316,7 @@ int ctx_fast_cluster(ngia_ctx *c, uint32_t identity, uint32_t bands, uint32_t *h
     if (hc.collect_error) return NGIA_ERR_CUDA;
     const uint32_t m = (uint32_t)hc.unique_total;
     if (m == 0) continue;
-    room = c->scores.reserve((size_t)m * 4);
+    room = over(slots + (size_t)m * 9) ? NGIA_ERR_NOMEM : c->scores.reserve((size_t)m * 4);
     if (room == NGIA_OK) room = c->round.reserve(m);
     if (room == NGIA_ERR_NOMEM && b1 - b0 > 1) {
       c->pairs.release();  // (a shorter run reserves less)
@@ -791,6 +798,12 @@ int ngia_ctx_group_align(ngia_ctx *c, uint32_t identity, uint32_t bands,
   NGIA_TRY(ngia::ctx_sketch_bucket(c, bands, stats, false, true));
   NGIA_TRY(ngia::ctx_build_graph(c, identity, bands, h_n_edges, stats));
   if (stats) ngia::ctx_stage_stats(c, stats);
+  return NGIA_OK;
+}
+
+int ngia_ctx_test_fast_room(ngia_ctx *c, uint64_t bytes) {
+  if (!c) return NGIA_ERR_ARG;
+  c->fast_room = bytes;
   return NGIA_OK;
 }
 

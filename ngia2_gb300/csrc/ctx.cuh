@@ -52,6 +52,7 @@ struct ngia_ctx {
   ngia::DevBuf ucount, uoff, counters, pairs, scores, emit_tmp, edges, scan_tmp,
       sort_tmp;
   uint64_t n_edges = 0;
+  uint64_t fast_room = 0;  // testing aid: bytes a run of fast mode may hold (0: any)
   // the batched aligner (scratch, side streams, plan, cached graph) on `stream`
   ngia::Round round;
   // the bucketing's launches (partition passes, resolve) captured as one graph
