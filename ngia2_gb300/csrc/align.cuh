@@ -303,16 +303,14 @@ __host__ __device__ inline bool general_possible(const ClassPlan &plan, uint32_t
 // is class-major, then 7 - floor(log2 nc) (column blocks in octaves, capped
 // at 7), in eight bits.
 __host__ __device__ inline uint32_t class_sort_key(int cls, const Band &b) {
-  uint32_t h = 0;
+  uint32_t h = 0;  // floor(log2 nc)
   if (b.nc > 1) {
 #ifdef __CUDA_ARCH__
-    const uint32_t lg = 31u - (uint32_t)__clz(b.nc);  // floor(log2 nc)
+    h = 31u - (uint32_t)__clz(b.nc);
 #else
-    const uint32_t lg = 31u - (uint32_t)__builtin_clz(b.nc);
+    h = 31u - (uint32_t)__builtin_clz(b.nc);
 #endif
-    h = 2 * lg + ((uint64_t)b.nc * b.nc >= (2ull << (2 * lg)) ? 1u : 0u);
   }
-  h >>= 1;
   return ((uint32_t)cls << 3) | (7u - (h < 7u ? h : 7u));
 }
 constexpr uint32_t kQueueKeys = 256;

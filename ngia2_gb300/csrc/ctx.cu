@@ -145,7 +145,6 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   const uint32_t *rep = c->rep.as<uint32_t>();
   const uint32_t *lens = c->lens.as<uint32_t>();
   NGIA_TRY(c->counters.reserve(sizeof(Counters)));
-  NGIA_TRY(c->ucount.reserve((size_t)n * 4));
   NGIA_TRY(c->uoff.reserve((size_t)n * 8));
   Counters *dc = c->counters.as<Counters>();
   NGIA_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), s));
@@ -722,7 +721,7 @@ void ngia_ctx_destroy(ngia_ctx *c) {
                           &c->offs,     &c->lens,  &c->rep,       &c->sigs,     &c->ucount,
                           &c->uoff,
                           &c->counters, &c->pairs, &c->scores,    &c->sort_tmp, &c->emit_tmp,
-                          &c->edges,    &c->scan_tmp, &c->sketch_table};
+                          &c->edges,    &c->sketch_table};
   for (ngia::DevBuf *b : bufs) b->release();
   c->round.destroy();  // shares c->stream, which it leaves alone
   for (int k = 0; k < ngia_ctx::kEvents; ++k)

@@ -49,8 +49,7 @@ struct ngia_ctx {
   ngia::DevBuf sketch_table;
   uint32_t longest = 0;  // no read of the database is longer
   // graph build work
-  ngia::DevBuf ucount, uoff, counters, pairs, scores, emit_tmp, edges, scan_tmp,
-      sort_tmp;
+  ngia::DevBuf ucount, uoff, counters, pairs, scores, emit_tmp, edges, sort_tmp;
   uint64_t n_edges = 0;
   uint64_t fast_room = 0;  // testing aid: bytes a run of fast mode may hold (0: any)
   // the batched aligner (scratch, side streams, plan, cached graph) on `stream`
