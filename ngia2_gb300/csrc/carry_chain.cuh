@@ -1,14 +1,13 @@
 // carry_chain.cuh -- multi-word add-with-carry chains in inline PTX
 // (internal header).
 //
-// add_chainN_XY(s, a, b[, cin][, cout]) computes the N-word sum
-//   s[0..N) = a[0..N) + b[0..N) + carry_in
-// with the carry rippling from word 0 upward through the hardware carry flag
-// (add.cc / addc.cc), one instruction per word.
-//   X = z : carry_in = 0
-//   X = c : carry_in = (cin != 0) (cin + 0xFFFFFFFF sets the flag)
-//   Y = n : no carry out
-//   Y = c : cout = carry out of word N-1 (0 or 1)
+// All compute the N-word sum s[0..N) = a[0..N) + b[0..N) + carry in, the carry
+// rippling from word 0 upward through the hardware carry flag (add.cc /
+// addc.cc), one instruction per word.
+//   add_chain8_cc(s, a, b, cin, cout) : carry in if cin != 0 (cin + 0xFFFFFFFF
+//     sets the flag), cout = carry out of word 7 (0 or 1)
+//   add_chainN_pp and its halves : carries popped from and pushed to words
+//   add_runN : no carry in or out
 #pragma once
 #include <cstdint>
 
@@ -40,25 +39,6 @@ __device__ __forceinline__ void add_chain8_cc(uint32_t *s, const uint32_t *a, co
 //   add_chainN_pp : pop in, push out
 //   add_chain8_pc : pop in, carry out as 0/1 in c (first half of 16 words)
 //   add_chain8_cp : carry in from c != 0, push out (second half)
-__device__ __forceinline__ void add_chain1_pp(uint32_t *s, const uint32_t *a, const uint32_t *b,
-                                              uint32_t &cin, uint32_t &cout) {
-  asm("add.cc.u32 %1, %1, %1;\n\t"
-      "addc.cc.u32 %0, %3, %4;\n\t"
-      "addc.u32 %2, %2, %2;\n\t"
-      : "=r"(s[0]), "+r"(cin), "+r"(cout)
-      : "r"(a[0]), "r"(b[0]));
-}
-
-__device__ __forceinline__ void add_chain2_pp(uint32_t *s, const uint32_t *a, const uint32_t *b,
-                                              uint32_t &cin, uint32_t &cout) {
-  asm("add.cc.u32 %2, %2, %2;\n\t"
-      "addc.cc.u32 %0, %4, %6;\n\t"
-      "addc.cc.u32 %1, %5, %7;\n\t"
-      "addc.u32 %3, %3, %3;\n\t"
-      : "=r"(s[0]), "=r"(s[1]), "+r"(cin), "+r"(cout)
-      : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]));
-}
-
 __device__ __forceinline__ void add_chain3_pp(uint32_t *s, const uint32_t *a, const uint32_t *b,
                                               uint32_t &cin, uint32_t &cout) {
   asm("add.cc.u32 %3, %3, %3;\n\t"
@@ -151,14 +131,12 @@ __device__ __forceinline__ void add_chain8_cp(uint32_t *s, const uint32_t *a, co
 template <int K>
 __device__ __forceinline__ void add_words_pp(uint32_t *s, const uint32_t *a, const uint32_t *b,
                                              uint32_t &cin, uint32_t &cout) {
-  if constexpr (K == 1) add_chain1_pp(s, a, b, cin, cout);
-  else if constexpr (K == 2) add_chain2_pp(s, a, b, cin, cout);
-  else if constexpr (K == 3) add_chain3_pp(s, a, b, cin, cout);
+  if constexpr (K == 3) add_chain3_pp(s, a, b, cin, cout);
   else if constexpr (K == 4) add_chain4_pp(s, a, b, cin, cout);
   else if constexpr (K == 6) add_chain6_pp(s, a, b, cin, cout);
   else if constexpr (K == 8) add_chain8_pp(s, a, b, cin, cout);
   else {
-    static_assert(K == 16, "carry-word chains of 1, 2, 3, 4, 6, 8 or 16 words");
+    static_assert(K == 16, "carry-word chains of 3, 4, 6, 8 or 16 words");
     uint32_t c;
     add_chain8_pc(s, a, b, cin, c);
     add_chain8_cp(s + 8, a + 8, b + 8, c, cout);
