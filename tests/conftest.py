@@ -22,6 +22,20 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU and the built libngia.so")
 
 
+def pytest_collection_modifyitems(items):
+    """The command-line comparison with the reference's own GPU build needs that
+    build; without the reference's sources (oracle/build.sh) there is none, and
+    it is skipped, as the comparison with the reference's kernel skips itself.
+    With the sources there a missing build still fails it."""
+    import oracle
+    if oracle.ref_gpu_cli().exists() or (oracle.REF / "src" / "buildGraph.hpp").exists():
+        return
+    skip = pytest.mark.skip(reason="reference sources not available (oracle/build.sh)")
+    for item in items:
+        if item.path.name == "test_gpu_reference_cli.py":
+            item.add_marker(skip)
+
+
 @pytest.fixture(scope="session")
 def built():
     """Builds (or reuses) libngia.so and the oracle libraries."""
