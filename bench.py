@@ -467,8 +467,10 @@ def run_ours(args, world, rank, local, pg):
     sketch_bytes = int(db["lens"].sum()) / 2 + 4 * BANDS * n  # codes read + signatures
     if table_active:
         achieved = sketch_bytes / (sketch_ms * 1e-3)
+        # bound by random shared-memory bits, which no measured peak of this
+        # line covers: the figures are of HBM for the input read once
         sketch_roof = {
-            "bound": "hbm", "kernel": "sketch_rank_kernel (+ sketch_table_kernel for records "
+            "bound": "shared_memory", "kernel": "sketch_rank_kernel (+ sketch_table_kernel for records "
             "under the rank walk's minimum span)",
             "achieved": achieved / 1e9, "peak": hbm, "unit": "GB/s",
             "frac": achieved / (hbm * 1e9) if hbm else None,
@@ -476,8 +478,9 @@ def run_ours(args, world, rank, local, pg):
             "units": {"signed_positions": positions}, "launches": 2, "ms": sketch_ms,
             "traffic": SKETCH_TABLE_DRAM_BYTES_PER_POSITION * positions,
             "algorithmic_bytes": sketch_bytes,
-            "note": "input read once; the walk is bound by shared-memory bit tests and "
-                    "issue, not by HBM",
+            "note": "frac is of HBM, for the input read once; the walk is bound by "
+                    "shared-memory bit tests (78 % of its wavefronts' rate, "
+                    "profiles/sketch_rank_kernel_dna100k.txt) and issue",
             "hash_equivalent_tops": positions * BANDS * SKETCH_ALU_OPS_PER_HASH
             / (sketch_ms * 1e-3) / 1e12,
             "table_bands": ng.lib().ngia_sketch_table_bands()}
@@ -957,6 +960,7 @@ def run_pairs(args) -> dict:
                 "19% uniform 1k-5k, 1% uniform 5k-35k; members 1-50% subs, 1% indels), "
                 "half the pairs within a family, half unrelated neighbours in length order",
         "metric": "aligned cells/s", "unit": "cells/s",
+        "note": "band cells of all the pairs, settled early or by the seed filter included",
         "band_cells": cells, "computed_cells": st["computed_cells"],
         "batched": {"value": cells / (ms_b * 1e-3), "ms": ms_b, "steps": steps,
                     "computed_cells_per_s": st["computed_cells"] / (ms_b * 1e-3),

@@ -142,8 +142,10 @@ typedef struct ngia_ctx ngia_ctx;
 typedef struct ngia_stats {
   uint64_t candidate_pairs; /* pairs over all bands, duplicates included (the
                                reference's "compare pairs", buildGraph.hpp:353) */
-  uint64_t unique_pairs;    /* distinct (rep, tar) pairs aligned */
-  uint64_t aligned_cells;   /* 1024 x 32x32 blocks visited over unique pairs */
+  uint64_t unique_pairs;    /* distinct (rep, tar) pairs scored */
+  uint64_t aligned_cells;   /* band cells of the unique pairs: 1024 x the 32x32
+                               blocks the reference visits for them, whether
+                               or not they had to be computed */
   uint64_t edges;           /* emitted edges (sorted, unique) */
   double ms_sketch, ms_bucket, ms_pairs, ms_align, ms_emit; /* device time */
   uint64_t computed_cells;  /* cells the aligners updated: window words (a

@@ -185,8 +185,8 @@ int ctx_build_graph(ngia_ctx *c, uint32_t identity, uint32_t bands, uint64_t *h_
   const uint32_t m = cut[1] - cut[0];
   NGIA_TRY(c->scores.reserve((size_t)(m ? m : 1) * 4));
   uint32_t *scores = c->scores.as<uint32_t>();
-  // 2-3. width classes, then one persistent launch per class (the round is
-  // on the context's stream)
+  // 2-3. width classes, then their persistent launches (the round is on the
+  // context's stream)
   NGIA_TRY(c->round.reserve(m));
   NGIA_TRY(c->round.enqueue(db_view(c), pairs, m, identity, scores, c->ev[1]));
   NGIA_CUDA(cudaEventRecord(c->ev[2], s));

@@ -438,8 +438,8 @@ int place_pairs(const uint8_t *keys, uint32_t count, unsigned int *key_count, ui
   return NGIA_OK;
 }
 
-// Small rounds: one block bins the pairs.  The general path is eight launches
-// (counters and scores cleared, keys, one radix pass, bounds), each a few
+// Small rounds: one block bins the pairs.  The general path is four or five
+// launches (counters cleared, keys, the seed filter, bounds, places), each a few
 // microseconds whatever the count; here the keys stay in shared memory, their
 // histogram and its scan give every class and octave its run of the queue, and
 // pairs take their places in it by atomics (the order inside a key is free).

@@ -23,7 +23,7 @@
 // What bounds it: the shared-memory pipe (random bits, 3.4 wavefronts a test or
 // mark; 70 % of its rate) and issue slots (60 %), some 80 warp instructions a
 // pair.  200,000 nucleotide reads at identity 95, 9.4 million pairs: 1.2 ms,
-// after which 0.44 ms of alignment are left of 3.12.  A set of 8,192 bytes,
+// after which 0.53 ms of alignment are left of 3.12.  A set of 8,192 bytes,
 // marked without atomics, was no faster and told fewer pairs; four-byte loads
 // took 1.4 times as long.
 #include "align.cuh"
