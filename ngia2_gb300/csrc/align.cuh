@@ -287,16 +287,24 @@ __host__ __device__ inline int round_class(const Band &b, const ClassPlan &plan,
 }
 
 // Whether a round over records of at most `longest` residues can have pairs of
-// the general class: a rep of at most G slices goes to a group class of G
-// lanes that the plan uses, whatever its band (16,384 residues with the
-// default plan).
-__host__ __device__ inline bool general_possible(const ClassPlan &plan, uint32_t longest) {
-  uint32_t words = 0;
+// the general class.  A rep of at most G slices goes to a group class of G
+// lanes that the plan uses, whatever its band (16,384 residues with the default
+// plan), and so does a band within the class's limit: ls + rs is about
+// (lr + lt (1 - 2t)) / 32 words, most at the shortest target the length filter
+// lets through (t lr) for t > 1/2 and at the longest for less, and up to four
+// words more by its roundings.  (An empty launch of the class at identity 90
+// cost a round of 2 million pairs of up to 35,000 residues 60 us of 5.88 ms.)
+__host__ __device__ inline bool general_possible(const ClassPlan &plan, uint32_t longest,
+                                                 float t) {
+  const float spread = t > 0.5f ? 1.0f + t - 2.0f * t * t : 2.0f - 2.0f * t;
+  const uint32_t rep = (longest + 31) / 32;
+  const uint32_t band = (uint32_t)((float)longest * spread / 32.0f) + 5;
   for (int g = 0; g < kNumGroupClasses; ++g) {
     const GroupShape sh = group_shape(kFirstGroupClass + g);
-    if (plan.group_limit[g] && (uint32_t)(sh.G * sh.K) > words) words = (uint32_t)(sh.G * sh.K);
+    const uint32_t lim = plan.group_limit[g];
+    if (lim && (rep <= (uint32_t)(sh.G * sh.K) || band <= lim)) return false;
   }
-  return (longest + 31) / 32 > words;
+  return true;
 }
 
 // Queue order inside a class: longest targets first.  The sort key of a pair

@@ -170,7 +170,7 @@ int Round::enqueue(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t id
   // so, 5.7 with the groups ahead, 5.6 with the narrow windows ahead; 2 million
   // pairs: 5.8, 6.1, 6.0).
   NGIA_CUDA(cudaEventRecord(fork_, s));
-  const bool general = general_possible(plan, db.longest);
+  const bool general = general_possible(plan, db.longest, args.t);
   for (int k = 0; k < kAlignKernels; ++k) {
     if (!align_kernel_used(k, widest)) continue;
     NGIA_CUDA(cudaStreamWaitEvent(side_[k], fork_, 0));
@@ -193,8 +193,9 @@ int Round::launch(const DbView &db, const uint2 *pairs, uint32_t m, uint32_t ide
   // everything the captured launches take by value or pointer: the database's
   // buffers and alphabet (a new load may reuse the buffers with another
   // alphabet, whose classes are other kernels), the pairs, the plan
+  const bool general = general_possible(plan, db.longest, identity_threshold(identity));
   const Key key{pairs,   scores, db.nib,   db.packed,    db.ab.dplanes, db.offs,
-                db.lens, m,      identity, round_mode(), db.ab.K,       general_possible(plan, db.longest),
+                db.lens, m,      identity, round_mode(), db.ab.K,       general,
                 db.ab.inv, g_alloc_gen.load(), plan_gen};
   if (!exec_ || !(key == key_)) {
     if (exec_) cudaGraphExecDestroy(exec_);

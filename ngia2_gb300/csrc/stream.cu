@@ -21,7 +21,6 @@
 // record tables and aligned by one batched round.  Scores go back to the
 // pairs' own positions, so the emission (sorted unique edges) is the resident
 // path's.
-#include <algorithm>
 #include <chrono>
 #include <cstring>
 #include <thread>
@@ -246,7 +245,9 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
   // and code planes in the budget)
   const uint64_t chunk_words = chunk_bytes / (3ull * 4 * 3);
   std::vector<Chunk> chunks;
+  uint32_t longest = 0;
   for (uint32_t i = 0; i < n; ++i) {
+    longest = h_lens[i] > longest ? h_lens[i] : longest;
     const uint64_t w = 1 + 4ull * ((h_lens[i] + 31) / 32);
     if (h_lens[i] > NGIA_MAX_READ || h_offs[i] + w > words) return NGIA_ERR_ARG;
     if (i > 0 && h_offs[i] < h_offs[i - 1] + 1 + 4ull * ((h_lens[i - 1] + 31) / 32))
@@ -259,7 +260,6 @@ static int stream_graph(StreamState &S, const uint32_t *h_packed, uint64_t words
     c.count += 1;
     c.words = h_offs[i] + w - c.word_first;
   }
-  const uint32_t longest = *std::max_element(h_lens, h_lens + n);
   const uint32_t C = (uint32_t)chunks.size();
   if ((uint64_t)C * C > 0xFFFFFFFFull) return NGIA_ERR_ARG;
   uint32_t max_recs = 0;

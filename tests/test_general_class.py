@@ -29,13 +29,14 @@ int main() {
   for (int g = 1; g < kNumGroupClasses; ++g) plans[4].group_limit[g] = 0;
   long bad = 0, out = 0, seen = 0;
   const uint32_t steps[] = {31, 32, 33, 767, 768, 769, 8191, 8192, 8193, 16383, 16384, 16385,
-                            16416, 30000, 65534};
+                            16416, 17000, 20000, 25000, 30000, 35000, 40000, 47000, 55000, 60000,
+                            65000, 65533, 65534};
   for (const ClassPlan &p : plans)
     for (uint32_t lr : steps)
       for (uint32_t lt : steps)
-        for (uint32_t id = 1; id <= 99; id += 7) {
+        for (uint32_t id = 1; id <= 99; ++id) {
           const Band b = make_band(lr, lt, identity_threshold(id), NGIA_ROUND_FMA);
-          const bool may = general_possible(p, lr > lt ? lr : lt);
+          const bool may = general_possible(p, lr > lt ? lr : lt, identity_threshold(id));
           out += !may;
           for (uint32_t widest = 16; widest <= kWidestWindow; widest += 12) {
             const int c = round_class(b, p, widest);
@@ -43,9 +44,10 @@ int main() {
             bad += c == kGeneralClass && !may;
           }
         }
-  // the default plan leaves it out up to 16,384 residues, and no further
-  bad += general_possible(plans[0], 16384) || !general_possible(plans[0], 16385);
-  bad += !general_possible(plans[3], 1) || general_possible(plans[4], 768);
+  // the default plan leaves it out up to 16,384 residues, beyond that by the band
+  bad += general_possible(plans[0], 16384, 0.3f) || !general_possible(plans[0], 16385, 0.3f);
+  bad += general_possible(plans[0], 35000, 0.9f) || !general_possible(plans[0], 65534, 0.5f);
+  bad += !general_possible(plans[3], 1, 0.9f) || general_possible(plans[4], 768, 0.3f);
   printf("bad %ld out %ld seen %ld\n", bad, out, seen);
   return bad != 0 || !out || !seen;
 }
