@@ -306,6 +306,8 @@ class Context:
         lens = np.ascontiguousarray(lens, np.uint32)
         if rep is not None:
             rep = np.ascontiguousarray(rep, np.uint32)
+            if rep.size < bands * lens.size:  # the copy would run past the array
+                raise ValueError(f"{rep.size} rep entries for {bands} bands of {lens.size} records")
         _check(lib().ngia_ctx_load(self._h, _ptr(packed), packed.size, _ptr(offsets), _ptr(lens),
                                    lens.size, _ptr(rep), bands), "ngia_ctx_load")
         self.n = int(lens.size)

@@ -32,3 +32,13 @@ def test_edges_at_the_limit(cuda, built, hits):
             want = np.flatnonzero(same)
             assert np.array_equal(edges["rep"], want - 2) and np.array_equal(edges["tar"], want)
             assert (edges["weight"] == 1.0).all()
+
+
+def test_load_refuses_missing_rep_rows(cuda, built):
+    """Fewer rep rows than bands: refused before the copy reads past them."""
+    from gpu_util import build_db
+    packed, offs, lens = build_db([b"ACDEFGHIKL"] * 3)
+    with ng.Context() as ctx:
+        with pytest.raises(ValueError):
+            ctx.load(packed, offs, lens, np.zeros((1, 3), np.uint32))
+        ctx.load(packed, offs, lens, np.zeros((1, 3), np.uint32), bands=1)
