@@ -115,7 +115,8 @@ int ngia_bucket_noalloc(const uint32_t *d_sigs, uint32_t n, uint32_t bands,
  * at :323; same kernel at src/fastClustering.hpp:183-244, launch at :313):
  * for every job, jobs[3j+2] = identity score of (rep = jobs[3j], tar =
  * jobs[3j+1]); pairs failing the length filter keep their score word.
- * identity in 1..99.  One launch.  No scratch memory. */
+ * identity in 1..99.  One launch, or three where there are more jobs than
+ * fit on the device at once.  No scratch memory. */
 int ngia_align_pairs(const uint32_t *d_packed, const uint64_t *d_rec_offsets,
                      uint32_t *d_jobs, uint32_t count, uint32_t identity,
                      void *stream);

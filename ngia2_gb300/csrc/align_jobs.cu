@@ -5,8 +5,9 @@
 // A warp takes 32 jobs in job order, one pair per lane, in the windows of the
 // batched aligner (align_window.cuh): the lanes whose pairs fit 4, 8, 12, 16
 // and 24 words (the whole rep, or the sliding band) run together, the rest
-// through the general form (in a launch of their own where there are many jobs).  Match masks come from tables in shared memory, as
-// there; the target's codes are made from its bit planes, block by block.
+// through the general form.  Many jobs take a launch each for narrow, medium and
+// wide pairs.  Match masks come from tables in shared memory, as there; the
+// target's codes are made from its bit planes, block by block.
 //
 // What bounds it at the reference's launch sizes (a band's few thousand jobs):
 // the longest pair of a warp, a serial chain of 32 columns a block.  With the
@@ -20,13 +21,14 @@ namespace ngia {
 
 constexpr uint32_t kJobWords = 24;  // the widest window
 constexpr int kJobSlots = 27;       // table slots: room for it to slide
+constexpr int kNarrowSlots = 9;     // the same for 8 words
 
 // The lanes of the warp with `run` align their pairs; returns the score.
-template <int W, bool kSlide>
+template <int NS, int W, bool kSlide>
 __device__ __forceinline__ void job_window(bool run, const uint32_t *rep, const uint32_t *tar,
                                            const Band &b, uint32_t *col, uint32_t &score) {
   if (!__any_sync(kFull, run)) return;
-  const LdsTable<kJobSlots, 16> tab{col};
+  const LdsTable<NS, 16> tab{col};
   uint32_t V[W];
 #pragma unroll
   for (int m = 0; m < W; ++m) V[m] = kFull;
@@ -49,7 +51,7 @@ __device__ __forceinline__ void job_window(bool run, const uint32_t *rep, const 
   while (__any_sync(kFull, sp.active)) {
     if constexpr (kSlide) window_advance<W>(tab, base);
     int32_t total = 0, ub = 0;
-    window_block<W, kJobSlots, 16, kSlide, true>(V, sp, tab, base, total, ub);
+    window_block<W, NS, 16, kSlide, true>(V, sp, tab, base, total, ub);
     if (sp.active) {
       const bool last = sp.i >= sp.nc;
       if (last || !lcs_may_reach((uint32_t)ub, sp.lr, sp.lt, b.t)) {
@@ -92,72 +94,85 @@ __device__ __forceinline__ uint32_t job_general(const Job &w, float t) {
   return identity_score(lcs_general(w.rep, w.tar, w.b, lines, blocks), w.b.lr, w.b.lt, t);
 }
 
-// The jobs of up to kJobWords words, and with kWide the others too.
-template <bool kWide>
+// Jobs by the width of their windows: up to 8 words, 9-24, more (general form).
+constexpr int kNarrow = 1, kMid = 2, kWide = 4;
+
+// The jobs of the widths in kSet.
+template <int NS, int kSet>
 __global__ void __launch_bounds__(32)
 align_jobs_kernel(const uint32_t *__restrict__ packed, const uint64_t *__restrict__ offs,
                   uint32_t *__restrict__ jobs, uint32_t count, float t, int fma_mode) {
   extern __shared__ uint32_t smem[];
-  uint32_t *col = smem + threadIdx.x;
-#pragma unroll 1
-  for (int s = 0; s < kJobSlots; ++s) col[s * 32] = 0u;  // code 0 matches nothing
   const uint32_t j = blockIdx.x * 32u + threadIdx.x;
   const Job w = load_job(packed, offs, jobs, j, count, t, fma_mode);
   const uint32_t *rep = w.rep, *tar = w.tar, words = w.words;
   const Band &b = w.b;
   const bool fixed = w.fixed;
+  const int kind = words <= 8 ? kNarrow : words <= kJobWords ? kMid : kWide;
+  const bool mine = w.mine && (kind & kSet);
+  if (!__any_sync(kFull, mine)) return;
+  [[maybe_unused]] uint32_t *col = smem + threadIdx.x;
+  if constexpr (NS > 0) {
+#pragma unroll 1
+    for (int s = 0; s < NS; ++s) col[s * 32] = 0u;  // code 0 matches nothing
+  }
   uint32_t score = 0;
-  job_window<4, true>(!fixed && words - 1u < 4u, rep, tar, b, col, score);
-  job_window<8, true>(!fixed && words - 5u < 4u, rep, tar, b, col, score);
-  job_window<12, true>(!fixed && words - 9u < 4u, rep, tar, b, col, score);
-  job_window<16, true>(!fixed && words - 13u < 4u, rep, tar, b, col, score);
-  job_window<24, true>(!fixed && words - 17u < 8u, rep, tar, b, col, score);
-  job_window<8, false>(fixed && words - 1u < 8u, rep, tar, b, col, score);
-  job_window<16, false>(fixed && words - 9u < 8u, rep, tar, b, col, score);
-  job_window<24, false>(fixed && words - 17u < 8u, rep, tar, b, col, score);
-  if constexpr (kWide) {
+  if constexpr (kSet & kNarrow) {
+    job_window<NS, 4, true>(!fixed && words - 1u < 4u, rep, tar, b, col, score);
+    job_window<NS, 8, true>(!fixed && words - 5u < 4u, rep, tar, b, col, score);
+    job_window<NS, 8, false>(fixed && words - 1u < 8u, rep, tar, b, col, score);
+  }
+  if constexpr (kSet & kMid) {
+    job_window<NS, 12, true>(!fixed && words - 9u < 4u, rep, tar, b, col, score);
+    job_window<NS, 16, true>(!fixed && words - 13u < 4u, rep, tar, b, col, score);
+    job_window<NS, 24, true>(!fixed && words - 17u < 8u, rep, tar, b, col, score);
+    job_window<NS, 16, false>(fixed && words - 9u < 8u, rep, tar, b, col, score);
+    job_window<NS, 24, false>(fixed && words - 17u < 8u, rep, tar, b, col, score);
+  }
+  if constexpr (kSet & kWide) {
     if (words > kJobWords) score = job_general(w, t);
   }
-  if (w.mine && (kWide || words <= kJobWords))
-    jobs[3 * (size_t)j + 2] = w.empty ? identity_score(0u, b.lr, b.lt, t) : score;
+  if (mine) jobs[3 * (size_t)j + 2] = w.empty ? identity_score(0u, b.lr, b.lt, t) : score;
 }
 
-// The wider jobs alone, without tables.
-__global__ void __launch_bounds__(32)
-align_jobs_wide_kernel(const uint32_t *__restrict__ packed, const uint64_t *__restrict__ offs,
-                       uint32_t *__restrict__ jobs, uint32_t count, float t, int fma_mode) {
-  const uint32_t j = blockIdx.x * 32u + threadIdx.x;
-  const Job w = load_job(packed, offs, jobs, j, count, t, fma_mode);
-  if (w.words > kJobWords) jobs[3 * (size_t)j + 2] = job_general(w, t);
-}
+constexpr size_t job_smem(int slots) { return (size_t)slots * 16 * 32 * 4; }
 
 int launch_align_jobs(const uint32_t *packed, const uint64_t *offs, uint32_t *jobs,
                       uint32_t count, uint32_t identity, cudaStream_t s) {
   if (count == 0) return NGIA_OK;
-  constexpr size_t smem = (size_t)kJobSlots * 16 * 32 * 4;
-  const void *func = reinterpret_cast<const void *>(align_jobs_kernel<true>);
-  const uint32_t warps = ceil_div(count, 32u);
   const float t = identity_threshold(identity);
+  const uint32_t warps = ceil_div(count, 32u);
+  constexpr auto all = align_jobs_kernel<kJobSlots, kNarrow | kMid | kWide>;
+  constexpr auto mid = align_jobs_kernel<kJobSlots, kMid>;
+  constexpr auto narrow = align_jobs_kernel<kNarrowSlots, kNarrow>;
   uint32_t grid = 0;
-  NGIA_TRY(persistent_grid(func, 32, smem, warps, &grid));
+  NGIA_TRY(persistent_grid(reinterpret_cast<const void *>(all), 32, job_smem(kJobSlots), warps,
+                           &grid));
   if (grid == warps) {
-    align_jobs_kernel<true><<<grid, 32, smem, s>>>(packed, offs, jobs, count, t, round_mode());
+    all<<<warps, 32, job_smem(kJobSlots), s>>>(packed, offs, jobs, count, t, round_mode());
     NGIA_LAUNCHED();
     return NGIA_OK;
   }
-  // More jobs than fit on the device at once: the tables leave a multiprocessor
-  // four warps, which pairs over kJobWords words, with no use for tables, would
-  // share.  Their own launch has twenty (100,000 pairs of 1,500 residues at
-  // identity 50: 3.58 ms in one launch, 2.68 in two; 2 million heavy-tailed pairs
-  // at 90 in 64 calls: 3,655 and 3,545 ms), and costs a call without such pairs
-  // a pass over its jobs (200,000 of 300 residues at 90: 66 and 71 us).
-  // Overlapping the two as dependent launches: 3,780 ms with the narrow one
-  // first, 3,498 with the wide one first.
-  const void *narrow = reinterpret_cast<const void *>(align_jobs_kernel<false>);
-  NGIA_TRY(persistent_grid(narrow, 32, smem, warps, &grid));  // (sets its shared memory)
-  align_jobs_kernel<false><<<warps, 32, smem, s>>>(packed, offs, jobs, count, t, round_mode());
+  // More jobs than fit on the device at once: the widest windows' tables leave a
+  // multiprocessor four warps, so the pairs that do with less have launches with
+  // smaller tables (eleven warps) and with none (twenty), which cost the others a
+  // pass over their jobs.  In one launch, in two (the pairs over kJobWords words
+  // apart), in three, and with masks from the bit planes throughout:
+  // 1,000,000 of 300 residues at identity 90 244, 258, 201, 205 us; 200,000 65, 71,
+  // 66, 60; 200,000 of 400 at 50 253, 271, 281, 439; 100,000 of 3,000 at 90 533, 549,
+  // 555, 1,076; 100,000 of 1,500 at 50 3.56, 2.69, 2.64, 2.54 ms; 2 million
+  // heavy-tailed pairs at 90 in 64 calls 3,655, 3,545, 3,498, 3,416.
+  NGIA_TRY(persistent_grid(reinterpret_cast<const void *>(narrow), 32, job_smem(kNarrowSlots),
+                           warps, &grid));  // (sets its shared memory)
+  narrow<<<warps, 32, job_smem(kNarrowSlots), s>>>(packed, offs, jobs, count, t, round_mode());
   NGIA_LAUNCHED();
-  align_jobs_wide_kernel<<<warps, 32, 0, s>>>(packed, offs, jobs, count, t, round_mode());
+  NGIA_TRY(persistent_grid(reinterpret_cast<const void *>(mid), 32, job_smem(kJobSlots), warps,
+                           &grid));
+  mid<<<warps, 32, job_smem(kJobSlots), s>>>(packed, offs, jobs, count, t, round_mode());
+  NGIA_LAUNCHED();
+  // (no wish for shared memory: the row words of the general form live in L1;
+  // with it 100,000 of 1,500 residues take 3.66 ms)
+  align_jobs_kernel<0, kWide><<<warps, 32, 0, s>>>(packed, offs, jobs, count, t, round_mode());
   NGIA_LAUNCHED();
   return NGIA_OK;
 }
