@@ -413,6 +413,14 @@ bool records_inside(const uint64_t *h_offs, const uint32_t *h_lens, uint32_t n,
   return max_len <= NGIA_MAX_READ && max_end <= words;
 }
 
+static void no_database(ngia_ctx *c) {
+  c->n = 0;
+  c->packed_words = 0;
+  c->sigs_valid = false;
+  c->rep_bands = 0;
+  c->n_edges = 0;
+}
+
 int ctx_load(ngia_ctx *c, const uint32_t *h_packed, uint64_t words, const uint64_t *h_offs,
              const uint32_t *h_lens, uint32_t n, const uint32_t *h_rep, uint32_t bands) {
   if (n == 0 || !h_packed || !h_offs || !h_lens) return NGIA_ERR_ARG;
@@ -420,6 +428,7 @@ int ctx_load(ngia_ctx *c, const uint32_t *h_packed, uint64_t words, const uint64
   uint32_t longest = 0;
   if (!records_inside(h_offs, h_lens, n, words, &longest)) return NGIA_ERR_ARG;
   cudaStream_t s = c->stream;
+  no_database(c);  // until this load is through (a reservation may fail half way)
   NGIA_TRY(c->packed.reserve(words * 4));
   NGIA_TRY(c->offs.reserve((size_t)n * 8));
   NGIA_TRY(c->lens.reserve((size_t)n * 4));
@@ -436,10 +445,7 @@ int ctx_load(ngia_ctx *c, const uint32_t *h_packed, uint64_t words, const uint64
   NGIA_CUDA(cudaMemcpyAsync(&present, c->presence.p, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                             s));
   NGIA_CUDA(cudaStreamSynchronize(s));
-  if (present & kBadRecord) {  // a length word that is not the record's read length
-    c->n = 0;
-    return NGIA_ERR_FORMAT;
-  }
+  if (present & kBadRecord) return NGIA_ERR_FORMAT;  // a length word not the read length
   NGIA_TRY(use_alphabet(c, choose_alphabet(present), words, n, true));
   c->last_present = present;
   c->n = n;
@@ -462,6 +468,7 @@ int ctx_load_text(ngia_ctx *c, const char *h_text, uint64_t text_bytes,
                   uint32_t n, uint64_t words) {
   if (n == 0 || !h_text || !h_starts || !h_lens || !h_offs) return NGIA_ERR_ARG;
   cudaStream_t s = c->stream;
+  no_database(c);  // as in ctx_load
   NGIA_TRY(c->packed.reserve(words * 4));
   NGIA_TRY(c->nib.reserve(words * 4));
   NGIA_TRY(c->offs.reserve((size_t)n * 8));
@@ -541,6 +548,7 @@ int ctx_load_sketch(ngia_ctx *c, const uint32_t *h_packed, uint64_t words,
     return NGIA_OK;
   *used = true;
   cudaStream_t s = c->stream;
+  no_database(c);  // as in ctx_load
   NGIA_TRY(c->packed.reserve(words * 4));
   NGIA_TRY(c->offs.reserve((size_t)n * 8));
   NGIA_TRY(c->lens.reserve((size_t)n * 4));
@@ -1025,13 +1033,8 @@ int ngia_ctx_run_host(ngia_ctx *c, const uint32_t *h_packed, uint64_t packed_wor
       cudaStreamSynchronize(c->layout);
       cudaStreamSynchronize(c->side);
       const cudaError_t e = cudaStreamSynchronize(c->stream);
-      if (e != cudaSuccess || !inside || *c->h_flag != 0) {
-        c->n = 0;  // the copies overwrote the resident records: no database until a load
-        c->packed_words = 0;
-        c->sigs_valid = false;
-        c->rep_bands = 0;
-        c->n_edges = 0;
-      }
+      if (e != cudaSuccess || !inside || *c->h_flag != 0)
+        ngia::no_database(c);  // the copies overwrote the resident records
       NGIA_CUDA(e);
     }
     if (rc != NGIA_OK) return rc;
