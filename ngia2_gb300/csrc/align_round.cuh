@@ -27,12 +27,16 @@ __device__ __forceinline__ uint32_t group_class(const RoundArgs &a, uint32_t *sm
                                      a.bounds[C + 1], a.cursors + C, a.scores, a.t, a.fm, smem);
 }
 
-// The classes of 32 lanes, widest first: few and long pairs, at most seven warps of them per multiprocessor, so that a pair of
-// 30,000 residues does not share its scheduler with three others and end the
-// round alone (2 million heavy-tailed pairs after the seed filter: 6.3 ms in
-// one kernel with the classes of 8 and 16 lanes at 14 warps, 4.7 ms here).
+// The classes of 32 lanes, widest first: few and long pairs, at most seven warps
+// of them per multiprocessor, so that a pair of 30,000 residues does not share
+// its scheduler with three others and end the round alone (2 million heavy-tailed
+// pairs after the seed filter: 6.3 ms in one kernel with the classes of 8 and 16
+// lanes at 14 warps, 4.7 ms here).  Twenty blocks are asked of the registers (96
+// a thread): the windows' and groups' warps share the multiprocessor (at 108 and
+// 115 registers 2 million pairs lose 2 and 6 %), and as many without the ask gave
+// 2,425 pairs at identity 88, one chain of 32 lanes, 823 us instead of 812.
 template <int KC>
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(32, 20)
 align_wide_kernel(const __grid_constant__ RoundArgs a) {
   extern __shared__ uint32_t smem[];
   uint32_t done = group_class<kFirstGroupClass + 7, KC>(a, smem);
